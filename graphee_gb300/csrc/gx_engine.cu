@@ -83,13 +83,16 @@ DevicePool* device_pool(int dev) {
 namespace {
 
 // Work units of one shard: heavy-vertex chunks first, then tiles of up to 32
-// consecutive light vertices with at most tile_edges edges.
+// consecutive light vertices, cut by unit_caps.
 void build_units(gx_engine* e) {
   const int32_t P = e->P;
   const int64_t* off = e->off.data();
   // Exact-order mode never chunks a vertex: each list is folded in order.
-  const int32_t heavy_deg = e->cfg.exact_order ? INT32_MAX : std::max(e->cfg.heavy_degree, 32);
-  const int64_t cap = std::max<int64_t>(e->cfg.tile_edges, 32);
+  e->caps = unit_caps(e->E, static_cast<int64_t>(e->n_sm) * GX_PULL_MIN_BLOCKS * kWarps, e->cfg.tile_edges,
+                      e->cfg.heavy_degree);
+  if (e->cfg.exact_order) e->caps.heavy = INT32_MAX;
+  const int32_t heavy_deg = e->caps.heavy;
+  const int64_t cap = e->caps.tile, chunk = e->caps.chunk;
   std::vector<std::vector<int2>> su(P);
   std::vector<std::vector<int32_t>> sh(P);
 #pragma omp parallel for schedule(dynamic, 1)
@@ -132,7 +135,7 @@ void build_units(gx_engine* e) {
       return da > db || (da == db && a < b);
     });
     int64_t chunks = 0;
-    for (int32_t v : hv) chunks += (off[v + 1] - off[v] + kHeavyChunk - 1) / kHeavyChunk;
+    for (int32_t v : hv) chunks += (off[v + 1] - off[v] + chunk - 1) / chunk;
     n_units[p + 1] = chunks + static_cast<int64_t>(su[p].size());
     n_heavy[p + 1] = static_cast<int64_t>(hv.size());
     n_part[p + 1] = chunks;
@@ -154,7 +157,7 @@ void build_units(gx_engine* e) {
     e->unit_begin[p] = static_cast<int32_t>(u);
     for (int32_t v : sh[p]) {
       const int64_t d = off[v + 1] - off[v];
-      const int32_t nch = static_cast<int32_t>((d + kHeavyChunk - 1) / kHeavyChunk);
+      const int32_t nch = static_cast<int32_t>((d + chunk - 1) / chunk);
       e->heavy[h] = make_int4(v, nch, static_cast<int32_t>(part), p);
       for (int32_t c = 0; c < nch; ++c) {
         e->units[u] = make_int2(-(static_cast<int32_t>(h) + 1), c);
@@ -838,7 +841,7 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
                                                        use_init, e->relabeled ? e->d_inv : nullptr);
   GX_CUDA(cudaGetLastError());
   GX_CUDA(cudaMemsetAsync(e->d_bm, 0, sizeof(uint32_t) * e->n_words, e->s_comp));
-  GX_CUDA(cudaMemsetAsync(e->d_work, 0, sizeof(unsigned int) * e->n_work, e->s_comp));
+  GX_CUDA(cudaMemsetAsync(e->d_work, 0, sizeof(unsigned int) * kQueueStride * e->n_work, e->s_comp));
   GX_CUDA(cudaMemsetAsync(e->d_hticket, 0, sizeof(unsigned int) * std::max<size_t>(e->heavy.size(), 1), e->s_comp));
 
   PullArgs pa;
@@ -860,7 +863,8 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
   pa.partial = e->d_partial;
   pa.hticket = e->d_hticket;
   pa.ctr = e->d_work;
-  pa.heavy_deg = e->cfg.exact_order ? INT32_MAX : std::max(e->cfg.heavy_degree, 32);
+  pa.heavy_deg = e->caps.heavy;
+  pa.chunk = e->caps.chunk;
   pa.bm = e->d_bm;
   PushArgs qa;
   memset(&qa, 0, sizeof(qa));
@@ -872,7 +876,7 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
   qa.val[1] = e->d_val[1];
   qa.outdeg = e->d_outdeg;
   qa.frontier = e->d_frontier;
-  qa.ctr = e->d_work + kQueues;
+  qa.ctr = e->d_work + kQueues * kQueueStride;
   qa.bm = e->d_bm;
   FinArgs fa;
   memset(&fa, 0, sizeof(fa));
@@ -886,7 +890,7 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
   fa.frontier = e->d_frontier;
   fa.frontier_cap = e->frontier_cap;
   fa.work_ctr = e->d_work;
-  fa.n_work_ctr = e->n_work;
+  fa.n_work_ctr = e->all_resident ? kQueues + 1 : e->n_work;  // the cursors this run's launches use
 
   void (*pull)(PullArgs) = e->cfg.exact_order ? pull_kernel<APP, true> : pull_kernel<APP, false>;
   if constexpr (APP == K_SSSP_UNIT || APP == K_SSSP_W || APP == K_CC) {
@@ -922,6 +926,12 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
         pa.hot_n = static_cast<int32_t>(n);
       }
     }
+  }
+  const int grid_pull_max = grid_pull;
+  {
+    const PullShape shape = pull_shape(pa.u_end, grid_pull_max, threads_pull);
+    grid_pull = shape.grid;
+    pa.grab = shape.grab;
   }
   const int grid_push = occupancy_grid<APP>(e, reinterpret_cast<const void*>(push_kernel<APP>));
   const int grid_fin = std::max(1, std::min(e->n_sm * 4, (e->n_words + kThreads - 1) / kThreads));
@@ -1132,7 +1142,7 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
         PullArgs sp = pa;
         sp.u_begin = e->unit_begin[p];
         sp.u_end = e->unit_begin[p + 1];
-        sp.ctr = e->d_work + 2 * kQueues + kQueues * p;
+        sp.ctr = e->d_work + static_cast<int64_t>(kQueueStride) * kQueues * (2 + p);
         if (sp.u_end == sp.u_begin) continue;
         const bool active = shard_on[p] != 0;
         const bool use_comp = e->comp && !e->resident[p] && active && e->cb_bytes[p] > 0;
@@ -1179,10 +1189,10 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
           if (weighted) sp.w = e->slot_w[slot] - lo;
           ++streamed;
         }
-        const int units = sp.u_end - sp.u_begin;
-        const int grid = std::max(1, std::min(grid_pull, (units + kWarps - 1) / kWarps));
-        if (use_comp) pull_comp<<<grid, kThreads, 0, e->s_comp>>>(sp);
-        else pull<<<grid, kThreads, 0, e->s_comp>>>(sp);
+        const PullShape shape = pull_shape(sp.u_end - sp.u_begin, grid_pull_max, kThreads);
+        sp.grab = shape.grab;
+        if (use_comp) pull_comp<<<shape.grid, kThreads, 0, e->s_comp>>>(sp);
+        else pull<<<shape.grid, kThreads, 0, e->s_comp>>>(sp);
         GX_CUDA(cudaGetLastError());
         ++launches;
         ++pull_launches;
@@ -1498,7 +1508,7 @@ gx_status gx_load_csc(gx_engine* e, int32_t V, int32_t P, const int32_t* bounds,
   e->n_words = (V + 31) / 32 + 2;
   GX_TRY(dev_alloc(&e->d_bm, static_cast<size_t>(e->n_words)));
   e->n_work = kQueues * (P + 2);
-  GX_TRY(dev_alloc(&e->d_work, static_cast<size_t>(e->n_work)));
+  GX_TRY(dev_alloc(&e->d_work, static_cast<size_t>(kQueueStride) * e->n_work));
   phase("vertex arrays");
   if (direct) {
     unsigned int h = 0;

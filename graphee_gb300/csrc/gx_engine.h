@@ -163,6 +163,7 @@ struct gx_engine {
   gx::hvec<int64_t> off;
   gx::hvec<int32_t> outdeg;
   int64_t n_dangling = 0;            // vertices of out-degree 0
+  gx::UnitCaps caps{};               // tile and chunk sizes, heavy threshold (build_units)
   gx::hvec<int2> units;
   gx::hvec<int32_t> unit_shard;
   std::vector<int32_t> unit_begin;  // P+1

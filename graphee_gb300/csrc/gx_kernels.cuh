@@ -101,6 +101,8 @@ struct PullArgs {
   unsigned int* hticket;    // per heavy vertex: chunks finished this step
   unsigned int* ctr;        // kQueues work-unit cursors of this launch (reset by finalize)
   int32_t heavy_deg;        // lists longer than this are swept by their own units
+  int32_t chunk;            // edges of one heavy chunk
+  int32_t grab;             // units a warp claims at once; 0: warp i takes unit i, none has two (pull_shape)
   uint32_t* bm;             // next-frontier bitmap
   // Compressed shard (COMP launches): chunk headers indexed by global chunk
   // id (edge >> 5), payload words, and byte weights indexed by global edge id.
@@ -138,7 +140,7 @@ struct FinArgs {
   const int32_t* outdeg;
   int4* frontier;
   unsigned long long frontier_cap;  // entries; |frontier| + E / kPushChunk + 1 fit by construction
-  unsigned int* work_ctr;
+  unsigned int* work_ctr;   // n_work_ctr cursors, kQueueStride words apart
   int32_t n_work_ctr;
 };
 
@@ -289,27 +291,74 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long x) {
 //    with up to GX_MID_MAX edges are then swept four lists at a time by
 //    groups of 8 lanes, and longer lists by the whole warp one by one
 //    (coalesced index loads, fixed-shape tree sums);
-//  * a heavy vertex (in-degree > heavy) is split into chunks of kHeavyChunk
+//  * a heavy vertex (in-degree > heavy) is split into chunks of `chunk`
 //    edges; each chunk is reduced by one warp, and the warp that finishes a
-//    vertex's last chunk folds the partials in chunk order and applies it.
+//    vertex's last chunk folds the partials (lane i those of chunks i, i + 32,
+//    ..., then a fixed xor tree) and applies it.
 // In exact-order mode (EXACT) every vertex is folded sequentially in edge
 // order: tiles with a longer list stage their edge range through shared
 // memory and each lane folds its own slice; no vertex is chunked.
 // Results are deterministic run to run in both modes.
 // ---------------------------------------------------------------------------
-constexpr int kHeavyChunk = 2048;
+constexpr int kHeavyChunk = 2048;  // longest heavy chunk
+constexpr int kMinChunk = 256;     // shortest: one round of warp_reduce_range
 #ifndef GX_LANE_MAX
 #define GX_LANE_MAX 16
 #endif
-#ifndef GX_GRAB
-#define GX_GRAB 4
-#endif
-#ifndef GX_TILE_PREFETCH
-#define GX_TILE_PREFETCH 0
-#endif
 constexpr int kLaneMaxDegree = GX_LANE_MAX;  // longest list a lane walks alone
-constexpr int kGrab = GX_GRAB;               // units a warp claims per atomic
+// Units a warp claims per atomic.  The next claim is issued before this one's
+// units are swept, so only its count matters: at 7 M vertices a superstep
+// takes 0.467 ms with 2, 0.477 with 3, 0.479 with 1.
+constexpr int kGrab = 2;
+// PageRank loads a tile's offsets, old values and out-degrees a unit ahead
+// (0.467 -> 0.457 ms at 7 M vertices); the min apps, a register short of
+// holding them, lose by it (weighted SSSP at scale 24: 6.45 -> 6.54 ms).
+template <int APP> constexpr bool tile_prefetch() { return is_pr<APP>(); }
 constexpr int kQueues = 64;          // work-unit cursors per launch
+// A cursor to a 128-byte line: atomics on one line are served one after the
+// other.  With the 64 cursors in two lines single-unit claims set the time of
+// a launch: 16 M edges, 0.139 -> 0.099 ms a superstep.
+constexpr int kQueueStride = 32;
+
+// How a graph of E edges is cut for a GPU that holds `warps` pull warps.  A
+// unit is a serial chain of loads, and a launch is never shorter than its
+// longest unit: the caps shrink until every warp has about four units, down
+// to one round of a warp's loads, and reach their full size (2048-edge tiles
+// and chunks, 4096-edge lists whole) at 40 M edges.  Measured per superstep
+// (two claimed at once): 16 M edges 0.099 ms with 4 units a warp, 0.111 with
+// 2, 0.104 with 6 and 8; 0.128 with the full-size caps and four claimed at
+// once.  A graph of 1000 vertices: 34 -> 14 us.
+struct UnitCaps {
+  int32_t tile, chunk, heavy;
+};
+inline UnitCaps unit_caps(int64_t E, int64_t warps, int32_t tile_edges, int32_t heavy_degree) {
+  const int64_t even = E / (4 * (warps > 0 ? warps : 1));
+  const int64_t most = tile_edges > 32 ? tile_edges : 32;
+  UnitCaps c;
+  c.tile = static_cast<int32_t>(even < 64 ? (most < 64 ? most : 64) : even < most ? even : most);
+  const int64_t ch = (static_cast<int64_t>(c.tile) + kMinChunk - 1) / kMinChunk * kMinChunk;
+  c.chunk = static_cast<int32_t>(ch < kHeavyChunk ? ch : kHeavyChunk);
+  const int32_t own = heavy_degree > 32 ? heavy_degree : 32;
+  c.heavy = own < 2 * c.chunk ? own : 2 * c.chunk;
+  return c;
+}
+
+// Launch shape of a pull over U units with room for `grid` CTAs.  With no
+// more units than warps each warp takes the unit of its own index, and CTAs
+// without one are not launched: no claim stands before the first load, and
+// the work spreads over the SMs.  Beyond, warps claim kGrab units at a time.
+struct PullShape {
+  int grid, grab;
+};
+inline PullShape pull_shape(int64_t U, int grid, int threads) {
+  const int64_t nw = threads / 32, warps = static_cast<int64_t>(grid) * nw;
+  PullShape s{grid, kGrab};
+  if (U <= warps) {
+    s.grid = static_cast<int>(U <= nw ? 1 : (U + nw - 1) / nw);
+    s.grab = 0;
+  }
+  return s;
+}
 
 // Queue q of nq splits U units evenly; its cursor counts units handed out.
 // Returns the first queue after q (cyclically) whose cursor is below its
@@ -318,12 +367,12 @@ __device__ __forceinline__ int next_queue(const unsigned int* ctr, int q, int nq
   bool ok0 = false, ok1 = false;
   if (lane < nq) {
     const int64_t size = (U * (lane + 1)) / nq - (U * lane) / nq;
-    ok0 = static_cast<int64_t>(*reinterpret_cast<const volatile unsigned int*>(ctr + lane)) < size;
+    ok0 = static_cast<int64_t>(*reinterpret_cast<const volatile unsigned int*>(ctr + lane * kQueueStride)) < size;
   }
   if (lane + 32 < nq) {
     const int j = lane + 32;
     const int64_t size = (U * (j + 1)) / nq - (U * j) / nq;
-    ok1 = static_cast<int64_t>(*reinterpret_cast<const volatile unsigned int*>(ctr + j)) < size;
+    ok1 = static_cast<int64_t>(*reinterpret_cast<const volatile unsigned int*>(ctr + j * kQueueStride)) < size;
   }
   const unsigned long long left = static_cast<unsigned long long>(__ballot_sync(0xffffffffu, ok0)) |
                                   (static_cast<unsigned long long>(__ballot_sync(0xffffffffu, ok1)) << 32);
@@ -573,19 +622,31 @@ __global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLO
   const int U = a.u_end - a.u_begin;
   const int nq = U / 256 < 1 ? 1 : (U / 256 < kQueues ? U / 256 : kQueues);
   const int gw = blockIdx.x * NW + wid;
-  int q = gw % nq;
+  int q = a.grab ? gw % nq : gw;
+  int qb = a.u_begin, qe = a.u_end, claim = gw;
+  if (a.grab) {
+    qb = a.u_begin + static_cast<int>((static_cast<int64_t>(U) * q) / nq);
+    qe = a.u_begin + static_cast<int>((static_cast<int64_t>(U) * (q + 1)) / nq);
+    if (lane == 0) claim = static_cast<int>(atomicAdd(a.ctr + q * kQueueStride, static_cast<unsigned>(a.grab)));
+  }
   for (;;) {
-    const int qb = a.u_begin + static_cast<int>((static_cast<int64_t>(U) * q) / nq);
-    const int qe = a.u_begin + static_cast<int>((static_cast<int64_t>(U) * (q + 1)) / nq);
-    int u0 = 0;
-    if (lane == 0) u0 = qb + static_cast<int>(atomicAdd(a.ctr + q, static_cast<unsigned>(kGrab)));
-    u0 = __shfl_sync(0xffffffffu, u0, 0);
-    if (u0 >= qe) {
-      q = next_queue(a.ctr, q, nq, U, lane);
-      if (q < 0) break;
-      continue;
+    const int u0 = qb + __shfl_sync(0xffffffffu, claim, 0);
+    int cnt = 1;
+    if (a.grab == 0) {  // at most as many units as warps
+      if (u0 >= qe) break;
+      claim = U;
+    } else {
+      if (u0 >= qe) {
+        q = next_queue(a.ctr, q, nq, U, lane);
+        if (q < 0) break;
+        qb = a.u_begin + static_cast<int>((static_cast<int64_t>(U) * q) / nq);
+        qe = a.u_begin + static_cast<int>((static_cast<int64_t>(U) * (q + 1)) / nq);
+        if (lane == 0) claim = static_cast<int>(atomicAdd(a.ctr + q * kQueueStride, static_cast<unsigned>(a.grab)));
+        continue;
+      }
+      cnt = qe - u0 < a.grab ? qe - u0 : a.grab;
+      if (lane == 0) claim = static_cast<int>(atomicAdd(a.ctr + q * kQueueStride, static_cast<unsigned>(a.grab)));
     }
-    const int cnt = qe - u0 < kGrab ? qe - u0 : kGrab;
     // One coalesced load for the batch's descriptors.
     int2 myu = make_int2(0, 0);
     int mysh = 0;
@@ -593,8 +654,8 @@ __global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLO
       myu = a.units[u0 + lane];
       if (selective) mysh = a.unit_shard[u0 + lane];
     }
-    // A tile's per-lane offsets, old value and out-degree are loaded one
-    // unit ahead, so those loads overlap the previous unit's gathers.
+    // A tile's per-lane offsets, old value and out-degree, a unit ahead
+    // (tile_prefetch): those loads overlap the previous unit's gathers.
     int64_t pbeg = 0, pend = 0;
     T pold = T(0);
     int32_t pod = 0;
@@ -608,7 +669,7 @@ __global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLO
         if constexpr (is_pr<APP>()) pod = __ldcs(a.outdeg + pv);
       }
     };
-    if (GX_TILE_PREFETCH) prefetch_tile(0);
+    if (tile_prefetch<APP>()) prefetch_tile(0);
     for (int j = 0; j < cnt; ++j) {
       const int2 wu = make_int2(__shfl_sync(0xffffffffu, myu.x, j), __shfl_sync(0xffffffffu, myu.y, j));
       const int jsh = __shfl_sync(0xffffffffu, mysh, j);
@@ -616,7 +677,7 @@ __global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLO
       const int64_t cbeg = pbeg, cend = pend;
       const T cold = pold;
       const int32_t cod = pod;
-      if (GX_TILE_PREFETCH && j + 1 < cnt) prefetch_tile(j + 1);
+      if (tile_prefetch<APP>() && j + 1 < cnt) prefetch_tile(j + 1);
       if (wu.x < 0) {
         // ---- heavy chunk ----
         const int h = -wu.x - 1;
@@ -630,28 +691,32 @@ __global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLO
           continue;
         }
         const int64_t vb = a.off[v], ve = a.off[v + 1];
-        const int64_t b = vb + static_cast<int64_t>(wu.y) * kHeavyChunk;
-        const int64_t e = ve < b + kHeavyChunk ? ve : b + kHeavyChunk;
+        const int64_t b = vb + static_cast<int64_t>(wu.y) * a.chunk;
+        const int64_t e = ve < b + a.chunk ? ve : b + a.chunk;
         T acc = identity<APP>();
         if constexpr (APP != K_INDEG) acc = warp_reduce_range<APP, ASYNC, COMP, HOT>(a, src_val, src_con, b, e, lane, hot);
+        T* part = static_cast<T*>(a.partial) + H.z;
+        bool last = H.y == 1;
         if (lane == 0) {
           la.edges += e - b;
-          T* part = static_cast<T*>(a.partial);
-          bool last = H.y == 1;
           if (!last) {
-            part[H.z + wu.y] = acc;
+            part[wu.y] = acc;
             __threadfence();
             last = atomicAdd(a.hticket + h, 1u) == static_cast<unsigned>(H.y) - 1;
           }
-          if (last) {
+        }
+        last = __shfl_sync(0xffffffffu, last, 0);
+        if (last) {
+          T tot = acc;
+          if (H.y > 1) {
             __threadfence();
-            const volatile T* vp = part;
-            T tot = acc;
-            if (H.y > 1) {
-              tot = identity<APP>();
-              for (int i = 0; i < H.y; ++i) tot = combine<APP>(tot, vp[H.z + i]);
-              a.hticket[h] = 0;
-            }
+            tot = identity<APP>();
+            for (int i = lane; i < H.y; i += 32) tot = combine<APP>(tot, __ldcg(part + i));
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) tot = combine<APP>(tot, __shfl_xor_sync(0xffffffffu, tot, o));
+          }
+          if (lane == 0) {
+            if (H.y > 1) a.hticket[h] = 0;
             const T old = static_cast<const T*>(src_val)[v];
             const int32_t od = is_pr<APP>() ? a.outdeg[v] : 0;
             T fin;
@@ -669,7 +734,7 @@ __global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLO
       int64_t beg = 0, end = 0;
       T old = T(0);
       int32_t od = 0;
-      if (GX_TILE_PREFETCH) {
+      if (tile_prefetch<APP>()) {
         if (lane < n) {
           beg = cbeg;
           end = cend;
@@ -1084,7 +1149,7 @@ __global__ void __launch_bounds__(kThreads) finalize_kernel(FinArgs a) {
     __threadfence();
     ctl->done = done;
   }
-  for (int i = threadIdx.x; i < a.n_work_ctr; i += kThreads) a.work_ctr[i] = 0;
+  for (int i = threadIdx.x; i < a.n_work_ctr; i += kThreads) a.work_ctr[static_cast<int64_t>(i) * kQueueStride] = 0;
   // The bitmap the next finalize marks into starts empty.
   if (c.mark_mode == MARK_OUT && mark) {
     uint32_t* old_bm = c.shard_bm + static_cast<int64_t>(c.shard_cur) * c.shard_words;

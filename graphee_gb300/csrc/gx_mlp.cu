@@ -729,10 +729,10 @@ gx_status engine_features(gx_engine* e, double damping, float* feat, double* uni
                           FeatScratch& fs) {
   const int32_t V = e->V;
   const double dangling0 = static_cast<double>(e->n_dangling) / V;
-  // The engine's heavy-vertex table (in-degree above heavy_degree) marks
+  // The engine's heavy-vertex table (in-degree above caps.heavy) marks
   // the lists the tile kernel leaves to a CTA each.
   const int32_t n_heavy = static_cast<int32_t>(e->heavy.size());
-  const int64_t heavy_deg = e->cfg.exact_order ? INT64_MAX : std::max(e->cfg.heavy_degree, 32);
+  const int64_t heavy_deg = e->cfg.exact_order ? INT64_MAX : e->caps.heavy;
   mlp_nbr_kernel<<<fs.grid, 256, 0, s>>>(e->d_off, e->d_outdeg, V, fs.nb);
   GX_CUDA(cudaMemsetAsync(fs.cursor, 0, sizeof(unsigned int), s));
   GX_CUDA(cudaMemsetAsync(fs.part, 0, sizeof(double) * fs.grid, s));

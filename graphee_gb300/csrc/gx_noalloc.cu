@@ -28,12 +28,12 @@ constexpr int32_t kNoAllocMaxVertices = 1 << 20;
 constexpr int32_t kNoAllocMaxSteps = 1024;
 constexpr int32_t kNoAllocUnits = (kNoAllocMaxVertices + 31) / 32;
 constexpr int32_t kNoAllocWords = kNoAllocMaxVertices / 32 + 2;
-constexpr int32_t kNoAllocWork = kQueues + 64;
+constexpr int32_t kNoAllocWork = kQueues;  // cursors, kQueueStride words apart
 
 struct NoAllocScratch {
   Ctl ctl;
   StepStats stats[kNoAllocMaxSteps];
-  unsigned int work[kNoAllocWork];
+  unsigned int work[kNoAllocWork * kQueueStride];
   unsigned int hticket[4];
   float partial[4];
   int4 heavy[1];
@@ -97,7 +97,7 @@ __global__ void noalloc_setup_kernel(NoAllocScratch* s, int32_t V, int32_t max_i
     s->unit_shard[i] = 0;
   }
   for (int i = tid; i < kNoAllocWords; i += nt) s->bm[i] = 0;
-  for (int i = tid; i < kNoAllocWork; i += nt) s->work[i] = 0;
+  for (int i = tid; i < kNoAllocWork * kQueueStride; i += nt) s->work[i] = 0;
   for (int i = tid; i < 4; i += nt) s->hticket[i] = 0;
 }
 
@@ -152,8 +152,9 @@ extern "C" gx_status gx_pagerank_noalloc(const int64_t* d_off, const int32_t* d_
   cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
   void (*pull)(PullArgs) = pull_kernel<K_PR_REF, false>;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void*>(pull), kThreads, 0);
-  const int grid_pull = (per_sm > 0 ? per_sm : 1) * n_sm;
   const int32_t U = (V + 31) / 32;
+  const PullShape shape = pull_shape(U, (per_sm > 0 ? per_sm : 1) * n_sm, kThreads);
+  const int grid_pull = shape.grid;
   const int n_words = V / 32 + 2;
   const int grid_fin = std::max(1, std::min(n_sm * 4, (n_words + kThreads - 1) / kThreads));
 
@@ -179,6 +180,8 @@ extern "C" gx_status gx_pagerank_noalloc(const int64_t* d_off, const int32_t* d_
   pa.partial = s->partial;
   pa.hticket = s->hticket;
   pa.ctr = s->work;
+  pa.chunk = kHeavyChunk;
+  pa.grab = shape.grab;
   pa.heavy_deg = INT32_MAX;  // no chunked vertices: long lists are swept by the tile's warp
   pa.bm = s->bm;
   FinArgs fa{};

@@ -111,13 +111,13 @@ __global__ void __launch_bounds__(kPprThreads) ppr_kernel(const PprArgs a) {
     const float* rs_in = (it & 1) ? a.rs[1] : a.rs[0];
     float* rs_out = (it & 1) ? a.rs[0] : a.rs[1];
     float* r_out = it + 1 == a.iters ? a.r_out : nullptr;
-    unsigned int* ctr = a.ctr + static_cast<size_t>(kQueues) * it;
+    unsigned int* ctr = a.ctr + static_cast<size_t>(kQueues) * kQueueStride * it;
     int q = (blockIdx.x * kPprWarps + wid) % nq;
     for (;;) {
       const int qb = static_cast<int>((static_cast<int64_t>(U) * q) / nq);
       const int qe = static_cast<int>((static_cast<int64_t>(U) * (q + 1)) / nq);
       int u0 = 0;
-      if (lane == 0) u0 = qb + static_cast<int>(atomicAdd(ctr + q, static_cast<unsigned>(kPprClaim)));
+      if (lane == 0) u0 = qb + static_cast<int>(atomicAdd(ctr + q * kQueueStride, static_cast<unsigned>(kPprClaim)));
       u0 = __shfl_sync(0xffffffffu, u0, 0);
       if (u0 >= qe) {
         q = next_queue(ctr, q, nq, U, lane);
@@ -249,7 +249,7 @@ extern "C" gx_status gx_ppr(gx_engine* e, int32_t k, const int32_t* sources, int
   guard.p.push_back(d_units);
   if ((st = dev_alloc(&d_src, kPprMaxCols)) != GX_OK) return st;
   guard.p.push_back(d_src);
-  if ((st = dev_alloc(&ctr, static_cast<size_t>(kQueues) * steps)) != GX_OK) return st;
+  if ((st = dev_alloc(&ctr, static_cast<size_t>(kQueues) * kQueueStride * steps)) != GX_OK) return st;
   guard.p.push_back(ctr);
   if ((st = dev_alloc(&ticket, static_cast<size_t>(std::max(n_part, 1)))) != GX_OK) return st;
   guard.p.push_back(ticket);
@@ -303,7 +303,7 @@ extern "C" gx_status gx_ppr(gx_engine* e, int32_t k, const int32_t* sources, int
   // The step's resets, R0 = S and the persistent launch, as one graph.
   auto enqueue = [&]() -> cudaError_t {
     cudaError_t err = cudaMemsetAsync(rs0, 0, rows * sizeof(float), s);
-    if (err == cudaSuccess) err = cudaMemsetAsync(ctr, 0, sizeof(unsigned int) * kQueues * steps, s);
+    if (err == cudaSuccess) err = cudaMemsetAsync(ctr, 0, sizeof(unsigned int) * kQueues * kQueueStride * steps, s);
     if (err == cudaSuccess) err = cudaMemsetAsync(arrive, 0, sizeof(unsigned int) * steps, s);
     if (err == cudaSuccess) err = cudaMemsetAsync(abort_flag, 0, sizeof(unsigned int), s);
     if (err != cudaSuccess) return err;
