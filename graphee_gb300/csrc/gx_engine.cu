@@ -711,6 +711,7 @@ gx_status build_out_edges(gx_engine* e, bool weighted) {
   // V + E / kPushChunk + 1 entries hold any frontier.
   e->frontier_cap = static_cast<unsigned long long>(V) + static_cast<unsigned long long>(e->E) / kPushChunk + 1;
   if (!e->d_frontier) GX_TRY(dev_alloc(&e->d_frontier, static_cast<size_t>(e->frontier_cap)));
+  GX_TRY(dev_alloc(&e->d_hubs, static_cast<size_t>(e->E / (kHubEntries * kPushChunk)) + 1));
   GX_TRY(dev_alloc(&e->d_ooff, static_cast<size_t>(V) + 1));
   GX_TRY(dev_alloc(&e->d_ocol, static_cast<size_t>(e->E) + 8));
   if (weighted) GX_TRY(dev_alloc(&e->d_ow, static_cast<size_t>(e->E) + 8));
@@ -866,6 +867,8 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
   pa.heavy_deg = e->caps.heavy;
   pa.chunk = e->caps.chunk;
   pa.bm = e->d_bm;
+  pa.hubs = e->d_hubs;
+  pa.frontier = e->d_frontier;
   PushArgs qa;
   memset(&qa, 0, sizeof(qa));
   qa.ctl = e->d_ctl;
@@ -888,6 +891,7 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
   fa.val[1] = e->d_val[1];
   fa.outdeg = e->d_outdeg;
   fa.frontier = e->d_frontier;
+  fa.hubs = e->d_hubs;
   fa.frontier_cap = e->frontier_cap;
   fa.work_ctr = e->d_work;
   fa.n_work_ctr = e->all_resident ? kQueues + 1 : e->n_work;  // the cursors this run's launches use

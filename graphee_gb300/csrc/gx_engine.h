@@ -223,6 +223,7 @@ struct gx_engine {
   bool out_unbuildable = false;      // vertexout.npy disagrees with the shards: no out-edge CSR
   int4* d_frontier = nullptr;
   unsigned long long frontier_cap = 0;
+  int4* d_hubs = nullptr;            // changed vertices whose frontier entries the next pull launch writes
   int64_t* d_ooff = nullptr;
   int32_t* d_ocol = nullptr;
   uint32_t* d_ow = nullptr;
@@ -311,6 +312,7 @@ struct gx_engine {
     shard_set_words = 0;
     out_unbuildable = false;
     gx::dev_free(&d_frontier);
+    gx::dev_free(&d_hubs);
     gx::dev_free(&d_ooff);
     gx::dev_free(&d_ocol);
     gx::dev_free(&d_ow);

@@ -24,6 +24,7 @@ constexpr int kChunk = 256;             // edges staged per warp per round
 constexpr int kGpsInf = 10000;          // GPS_INF, GraphMP/system/Global.h:50
 constexpr uint32_t kInfW = 0xFFFFFFFFu; // INF of weighted SSSP
 constexpr int kPushChunk = 256;         // out-edges per push frontier entry (longer lists get several)
+constexpr int kHubEntries = 8;          // entries a lane of finalize writes itself; more are expand_hubs'
 
 struct StepStats {
   unsigned long long changed;  // reference _Changed_Vertex
@@ -82,6 +83,7 @@ struct Ctl {
   unsigned long long changed, active, edges, resid_fx, dangl_fx;  // current-step accumulators
   unsigned long long front_edges;      // out-edges of the vertices that changed this step
   unsigned int next_frontier;
+  unsigned int n_hubs;      // vertices whose frontier entries expand_hubs writes
   unsigned int fin_ticket;
 };
 
@@ -117,6 +119,10 @@ struct PullArgs {
   // streamed graphs): every unit only carries its vertices' values over, and
   // no edge is read (col then points nowhere valid).
   int32_t skip;
+  // Push steps (the launch has no pull to do): the hubs the last finalize
+  // listed, as (vertex, value bits, first slot, entries), and the frontier.
+  const int4* hubs;
+  int4* frontier;
 };
 
 struct PushArgs {
@@ -139,6 +145,7 @@ struct FinArgs {
   void* val[2];
   const int32_t* outdeg;
   int4* frontier;
+  int4* hubs;               // out-degree above kHubEntries * kPushChunk: at most E / that + 1
   unsigned long long frontier_cap;  // entries; |frontier| + E / kPushChunk + 1 fit by construction
   unsigned int* work_ctr;   // n_work_ctr cursors, kQueueStride words apart
   int32_t n_work_ctr;
@@ -569,6 +576,16 @@ __device__ __forceinline__ typename AppTraits<APP>::T group_reduce_range(const P
 constexpr int kHotThreads = 1024;
 template <bool HOT> constexpr int pull_threads() { return HOT ? kHotThreads : kThreads; }
 
+// The frontier entries of hubs, a warp per hub; slots were reserved and
+// checked by finalize.
+__device__ __forceinline__ void expand_hubs(const PullArgs& a, int warp, int warps, int lane) {
+  const int n = static_cast<int>(a.ctl->n_hubs);
+  for (int h = warp; h < n; h += warps) {
+    const int4 x = a.hubs[h];
+    for (int k = lane; k < x.w; k += 32) a.frontier[static_cast<unsigned>(x.z) + k] = make_int4(x.x, x.y, k * kPushChunk, 0);
+  }
+}
+
 template <int APP, bool EXACT, bool ASYNC = false, bool COMP = false, bool HOT = false>
 __global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLOCKS) pull_kernel(PullArgs a) {
   typedef typename AppTraits<APP>::T T;
@@ -578,7 +595,10 @@ __global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLO
   extern __shared__ __align__(16) unsigned char s_dyn[];
   Ctl* ctl = a.ctl;
   const int done = ctl->done, mode = ctl->mode;
-  if (done || mode == MODE_PUSH) return;
+  if (done || mode == MODE_PUSH) {
+    if (!done) expand_hubs(a, blockIdx.x * NW + (threadIdx.x >> 5), gridDim.x * NW, threadIdx.x & 31);
+    return;
+  }
   const void* hot = nullptr;
   if constexpr (HOT) {
     // The current step's values of sources [0, hot_n) (PageRank: their
@@ -898,9 +918,13 @@ __global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLO
 // a vertex whose in-neighbours did not change cannot improve, so the values
 // and the per-step change counts are those of a full pull.
 // Frontier entries cover at most kPushChunk out-edges each (a hub is several
-// entries).  A warp claims 32 entries and sweeps their concatenated edge
-// ranges 32 edges at a time; each lane finds the entry that owns its edge by
-// a binary search over the warp's exclusive prefix sums.
+// entries).  A warp takes up to 32 entries and sweeps their concatenated edge
+// ranges 128 edges at a time; each lane finds the entry that owns its edge by
+// a binary search over the warp's exclusive prefix sums.  A sweep is a serial
+// chain of rounds, so a frontier too small to give every warp 32 entries is
+// spread thinner, down to one entry a warp (386 entries of 256 edges: 32 to a
+// warp took 0.527 ms, one to a warp 0.02 ms); the first entries of each warp
+// are those of its own index, later ones are claimed.
 // ---------------------------------------------------------------------------
 template <int APP>
 __global__ void __launch_bounds__(kThreads) push_kernel(PushArgs a) {
@@ -909,15 +933,14 @@ __global__ void __launch_bounds__(kThreads) push_kernel(PushArgs a) {
   const int cur = a.ctl->cur;
   const int lane = threadIdx.x & 31;
   const int nf = a.ctl->n_frontier;
+  if (blockIdx.x == 0 && threadIdx.x == 0) a.ctl->n_hubs = 0;  // written out by the pull launch before this one
   LocalAcc la;
   if constexpr (!is_pr<APP>() && APP != K_INDEG) {
   T* val = static_cast<T*>(cur ? a.val[1] : a.val[0]);
-  for (;;) {
-    int base = 0;
-    if (lane == 0) base = static_cast<int>(atomicAdd(a.ctr, 32u));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (base >= nf) break;
-    const int cnt = nf - base < 32 ? nf - base : 32;
+  const int warps = gridDim.x * kWarps;
+  const int take = nf >= 32 * warps ? 32 : (nf + warps - 1) / warps;
+  for (int64_t base = static_cast<int64_t>(blockIdx.x * kWarps + (threadIdx.x >> 5)) * take; base < nf;) {
+    const int cnt = nf - base < take ? static_cast<int>(nf - base) : take;
     int d = 0;
     uint32_t su = 0;
     long long b = 0;
@@ -987,6 +1010,10 @@ __global__ void __launch_bounds__(kThreads) push_kernel(PushArgs a) {
         }
       }
     }
+    if (static_cast<int64_t>(warps) * take >= nf) break;  // every entry had its warp
+    int next = 0;
+    if (lane == 0) next = static_cast<int>(atomicAdd(a.ctr, static_cast<unsigned>(take)));
+    base = static_cast<int64_t>(warps) * take + __shfl_sync(0xffffffffu, next, 0);
   }
   }
   flush_block(a.ctl, la);
@@ -1031,7 +1058,13 @@ __global__ void __launch_bounds__(kThreads) finalize_kernel(FinArgs a) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   unsigned long long act = 0;
   // Warp-uniform sweep: lane i takes word w0 + i, so the frontier compaction
-  // can reserve its slots with one atomic per warp.
+  // can reserve its slots with one atomic per warp.  A vertex of more than
+  // kHubEntries entries only reserves them: the next pull launch, which has
+  // no step to do, writes them with the whole GPU (expand_hubs).  (Written by
+  // the vertex's lane, R-MAT's hubs made this 0.185 ms of a step at scale 24.
+  // Words spread over a warp's lanes vertex by vertex, with the loads of 4 to
+  // 16 words in flight, swept dense frontiers 1.2 to 4 times slower: the many
+  // lanes walking their own words keep more loads in flight.)
   for (int w0 = blockIdx.x * kThreads + (wid << 5); w0 < a.n_words; w0 += gridDim.x * kThreads) {
     const int w = w0 + lane;
     const uint32_t word = w < a.n_words ? a.bm[w] : 0u;
@@ -1084,10 +1117,15 @@ __global__ void __launch_bounds__(kThreads) finalize_kernel(FinArgs a) {
           const int od = __ldg(a.outdeg + u);
           T vu = newv[u];
           const int bits = *reinterpret_cast<int*>(&vu);
-          for (int k = 0; k < od; k += kPushChunk, ++pos) {
-            if (pos < a.frontier_cap) a.frontier[pos] = make_int4(u, bits, k, 0);
-            else ctl->error = 2;
+          const int n = (od + kPushChunk - 1) / kPushChunk;
+          if (pos + n > a.frontier_cap) {
+            ctl->error = 2;
+          } else if (n > kHubEntries) {
+            a.hubs[atomicAdd(&ctl->n_hubs, 1u)] = make_int4(u, bits, static_cast<int>(pos), n);
+          } else {
+            for (int k = 0; k < n; ++k) a.frontier[pos + k] = make_int4(u, bits, k * kPushChunk, 0);
           }
+          pos += n;
         }
       }
     }

@@ -58,3 +58,32 @@ def test_units(V, lists, fill, relabel):
         e.load(g)
         e.run(gx.APP_PAGERANK_REF, 12)
         assert np.array_equal(e.values().view(np.uint32), ref.view(np.uint32))
+
+
+# Out-degrees around a frontier entry (256 edges), around what a lane of the
+# compaction writes itself (8 entries) and beyond a warp's 32 entries.
+HUBS = [1, 255, 256, 257, 2047, 2048, 2049, 2305, 8192, 8193, 40000]
+
+
+@pytest.mark.parametrize("relabel", [0, 1])
+@pytest.mark.parametrize("copies", [1, 40, 600])
+def test_push_hubs(copies, relabel):
+    """The source reaches `copies` of each hub in step 0, which reach the rest in step 1."""
+    V = 60000
+    rng = np.random.default_rng(copies)
+    lists = np.array(HUBS * copies)[:1 + 2_000_000 // 5000]
+    hub = 1 + np.arange(len(lists))
+    src = np.concatenate([np.zeros(len(lists), np.int64), np.repeat(hub, lists)])
+    dst = np.concatenate([hub] + [rng.permutation(V)[:n] for n in lists])
+    off, col = gx.build_csc(V, src, dst)
+    g = gx.Graph(V, off, col, None, 5)
+    g.weights = gx.edge_weights(9, g)
+    a = (g.V, g.P, g.bounds, g.off, g.col, g.outdeg)
+    with gx.Engine(relabel=relabel, push_edge_fraction=1.0) as e:
+        e.load(g)
+        for weighted in (True, False):
+            st = e.run(gx.APP_SSSP, 1000, source=0, weighted=weighted)
+            ref, changed, _ = O.run(O.SSSP, *a, 1000, weights=g.weights if weighted else None, source=0)
+            assert np.array_equal(e.values(), ref)
+            assert [e.iter_stats(i)["changed"] for i in range(st["iterations"])] == list(changed)
+            assert st["push_iterations"] == st["iterations"]
