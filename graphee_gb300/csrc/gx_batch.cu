@@ -15,9 +15,31 @@
 // triple-buffered change counts per instance, polled with a bounded spin (a
 // timeout raises an abort flag that every CTA honours, and the host reports
 // GX_ERR_TIMEOUT).  The launch holds no more CTAs than fit on the GPU at
-// once, so every member of a claimed team is running.  Inside a CTA, warps
-// sweep 32-vertex tiles: lanes walk lists of up to `lane_max` edges alone
-// (edge order), longer lists are swept by the whole warp.
+// once, so every member of a claimed team is running.
+//
+// Two things bounded the sweep of an instance's lists as they lie in the CSC:
+// the gather of a neighbour's value per edge (from global memory a warp's 32
+// addresses cost the L1 a lookup each, even when all hit), and instructions
+// spent on lanes whose list had ended or not begun.  So each call first
+// rewrites every instance (about 35 supersteps read what it writes once):
+//  * its vertices are renumbered by descending list length, and its edges
+//    hold the new ids;
+//  * the edges are laid out in rounds of 4 per lane, 32 lanes side by side, so
+//    that a warp's load of a round is one contiguous piece: lists of up to
+//    `lane_max` edges 32 to a tile, a lane each, in edge order; longer lists
+//    across the warp, or across half of it when 16 lanes hold them.  Ids are
+//    16-bit where they fit, and unused places hold the id of a slot whose
+//    value does not count (0 in a sum, the largest label in a minimum).
+// A CTA gathers from a table in shared memory, where a gather of 32 costs its
+// bank conflicts, three or four cycles: both buffers of an instance that fits
+// twice, else the values of its first vertices (the hottest on R-MAT),
+// refreshed from global memory after each superstep; other values are gathered
+// from there.  Sums are taken in the order of the lists' plain sweep (a lane
+// per short list, else 4 consecutive edges per lane per round of 128 aligned
+// edges and an xor tree), so results do not depend on the layout.
+// 512 instances of scales 10 to 17 (290 M edges, 35 supersteps): 52.6 ms a
+// call swept as they lie, 26.8 rewritten (the rewriting's share 3.5 ms); long
+// scoreboard stalls on the id loads lead now, at 0.29 of HBM's rate.
 // Threads per CTA, lane_max and CTAs per SM come from the autotuner
 // (gx_batch_autotune), which times candidate schedules on the batch and
 // records the winner in a table file.
@@ -26,8 +48,10 @@
 #include <algorithm>
 #include <chrono>
 #include <cstdio>
+#include <memory>
 #include <numeric>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "gx_engine.h"
@@ -36,6 +60,21 @@
 using namespace gx;
 
 namespace {
+
+constexpr int kBatchSortThreads = 512;
+constexpr int kFillSplit = 8;       // CTAs that share an instance in batch_fill_kernel
+constexpr int kBatchL1 = 64 * 1024;  // shared-memory bytes per SM left to the L1
+constexpr int kCheckSplit = 4;  // CTAs that share an instance in batch_check_kernel
+
+// A unit of an instance's sweep: `cnt` vertices from local (new) id `first`
+// on, its rounds from round `at` of the instance on.
+enum : int { kUnitTile = 0, kUnitHalf = 1, kUnitWarp = 2 };
+struct __align__(16) BatchUnit {
+  int32_t first;
+  int32_t kind_cnt;  // kind << 8 | cnt
+  int32_t at;
+  int32_t rounds;    // kUnitWarp: rounds per vertex, else of the unit
+};
 
 struct BatchArgs {
   const int64_t* off;
@@ -49,77 +88,119 @@ struct BatchArgs {
   unsigned int* team;       // per instance: arrivals, change counts [3]
   unsigned int* abort;      // set when a team barrier times out
   unsigned int spin_limit;
-  float *pr0, *pr1;
+  float *pr0, *pr1;         // working values, indexed vbeg[i] + new local id
   float *con0, *con1;
   int32_t *lab0, *lab1;
-  float* pr_out;
+  float* pr_out;            // results, by the caller's vertex
   int32_t* cc_out;
   int32_t* pr_steps;        // per instance
   int32_t* cc_steps;
   int32_t pr_iters, cc_max;
   int32_t lane_max;
+  int32_t tab;              // 4-byte values of the CTA's table in dynamic shared memory
+  // The rewritten instances.
+  int32_t* inv;             // vertex of new id vbeg[i] + k
+  int32_t* perm;            // new local id of a vertex
+  int32_t* od;              // out-degrees by new id
+  BatchUnit* units;         // instance i's at units[vbeg[i]]
+  int32_t* n_units;
+  unsigned long long* rounds;  // per instance: 256-byte blocks of its rounds
+  const unsigned long long* round_base;  // first block
+  uint2* ids;               // blocks of 32 x 4 16-bit ids; a round of 32-bit ids is two
   double damping;
 };
 
-// Gathers a vertex's in-edge values: PR contributions (sum) or labels (min).
-// Lanes walk lists of up to lane_max edges alone, 8 edges per step from two
-// 128-bit index loads (edge order kept: positions outside the list are
-// masked), so each lane has 8 gathers in flight; longer lists are swept by the
-// whole warp, 4 consecutive edges per lane per round.
+// Ids are 32-bit from this many vertices on (ids run to n, the unused place's).
+constexpr int kBatchWide = 65535;
+
+// Vertices of the instance whose values the table holds (besides the unused
+// place's), and whether both buffers fit.
+__host__ __device__ inline int batch_table(int n, int tab) { return n < tab - 1 ? n : tab - 1; }
+__host__ __device__ inline bool batch_dual(int n, int team, int tab) {
+  return team == 1 && 2 * (static_cast<int64_t>(n) + 1) <= tab;
+}
+
+// The value of id x, as the layout holds it: ids up to tn are table slots (tn
+// is the unused place's), those beyond are vertex x - 1's value in global
+// memory.  Without a branch: the table is read at a clamped index, global
+// memory under a predicate.
+template <bool FULL>
+__device__ __forceinline__ uint32_t batch_gather(const uint32_t* tab, int tn, const uint32_t* g, int32_t x) {
+  if constexpr (FULL) return tab[x];
+  uint32_t r = tab[x < tn ? x : tn];
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.gt.s32 p, %1, %2;\n\t@p ld.global.b32 %0, [%3];\n\t}"
+               : "+r"(r) : "r"(x), "r"(tn), "l"(g + x - 1) : "memory");
+  return r;
+}
+
+// Folds a value into the sum (PR: contributions) or minimum (labels).
 template <bool PR>
-__device__ __forceinline__ void batch_vertex_lists(const BatchArgs& a, const float* con, const int32_t* lab,
-                                                   int64_t beg, int64_t end, bool valid, float& facc, int32_t& iacc,
-                                                   int lane) {
-  const bool longl = valid && end - beg > a.lane_max;
-  if (valid && !longl && end > beg) {
-    for (int64_t k = beg & ~3ll; k < end; k += 8) {
-      const int4 c0 = __ldg(reinterpret_cast<const int4*>(a.col + k));
-      int4 c1 = make_int4(0, 0, 0, 0);
-      if (k + 4 < end) c1 = __ldg(reinterpret_cast<const int4*>(a.col + k + 4));
-      const int32_t cs[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-      float fv[8];
-      int32_t iv[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const bool in = k + j >= beg && k + j < end;
-        if (PR) fv[j] = in ? __ldg(con + cs[j]) : 0.f;
-        else iv[j] = in ? __ldg(lab + cs[j]) : 0x7fffffff;
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        if (PR) {
-          if (k + j >= beg && k + j < end) facc += fv[j];
-        } else {
-          iacc = min(iacc, iv[j]);
-        }
-      }
-    }
+__device__ __forceinline__ void batch_fold(uint32_t x, float& f, int32_t& m) {
+  if (PR) f += __uint_as_float(x);
+  else m = min(m, static_cast<int32_t>(x));
+}
+
+// A lane's four ids of a round.
+template <bool WIDE>
+struct BatchIds {
+  uint4 x;
+};
+template <>
+struct BatchIds<false> {
+  uint2 x;
+};
+template <bool WIDE>
+__device__ __forceinline__ BatchIds<WIDE> batch_load(const void* ids, int64_t round, int lane) {
+  BatchIds<WIDE> r;
+  if constexpr (WIDE) r.x = __ldcs(static_cast<const uint4*>(ids) + round * 32 + lane);
+  else r.x = __ldcs(static_cast<const uint2*>(ids) + round * 32 + lane);
+  return r;
+}
+template <bool PR, bool WIDE, bool FULL>
+__device__ __forceinline__ void batch_fold4(const BatchIds<WIDE>& c, const uint32_t* tab, int tn, const uint32_t* g,
+                                            float& f, int32_t& m) {
+  uint32_t id[4];
+  if constexpr (WIDE) {
+    id[0] = c.x.x, id[1] = c.x.y, id[2] = c.x.z, id[3] = c.x.w;
+  } else {
+    id[0] = c.x.x & 0xffffu, id[1] = c.x.x >> 16, id[2] = c.x.y & 0xffffu, id[3] = c.x.y >> 16;
   }
-  for (unsigned m = __ballot_sync(0xffffffffu, longl); m; m &= m - 1) {
-    const int l = __ffs(m) - 1;
-    const int64_t bl = __shfl_sync(0xffffffffu, beg, l), el = __shfl_sync(0xffffffffu, end, l);
-    float fs = 0.f;
-    int32_t is = 0x7fffffff;
-    for (int64_t q = (bl & ~3ll) + 4 * lane; q < el; q += 128) {
-      const int4 c = __ldg(reinterpret_cast<const int4*>(a.col + q));
-      const int32_t cs[4] = {c.x, c.y, c.z, c.w};
+  uint32_t v[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (q + j >= bl && q + j < el) {
-          if (PR) fs += __ldg(con + cs[j]);
-          else is = min(is, __ldg(lab + cs[j]));
-        }
-      }
-    }
+  for (int j = 0; j < 4; ++j) v[j] = batch_gather<FULL>(tab, tn, g, static_cast<int32_t>(id[j]));
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      if (PR) fs += __shfl_xor_sync(0xffffffffu, fs, o);
-      else is = min(is, __shfl_xor_sync(0xffffffffu, is, o));
-    }
-    if (lane == l) {
-      if (PR) facc += fs;
-      else iacc = min(iacc, is);
-    }
+  for (int j = 0; j < 4; ++j) batch_fold<PR>(v[j], f, m);
+}
+
+// Folds rounds [at, at + n), 32 bytes a lane in flight.
+template <bool PR, bool WIDE, bool FULL>
+__device__ __forceinline__ void batch_rounds(const void* ids, int64_t at, int n, int lane, const uint32_t* tab, int tn,
+                                             const uint32_t* g, float& f, int32_t& m) {
+  constexpr int F = WIDE ? 2 : 4;
+  int r = 0;
+  for (; r + F <= n; r += F) {
+    BatchIds<WIDE> c[F];
+#pragma unroll
+    for (int j = 0; j < F; ++j) c[j] = batch_load<WIDE>(ids, at + r + j, lane);
+#pragma unroll
+    for (int j = 0; j < F; ++j) batch_fold4<PR, WIDE, FULL>(c[j], tab, tn, g, f, m);
+  }
+  if (r < n) {
+    BatchIds<WIDE> c[F - 1];
+#pragma unroll
+    for (int j = 0; j < F - 1; ++j)
+      if (r + j < n) c[j] = batch_load<WIDE>(ids, at + r + j, lane);
+#pragma unroll
+    for (int j = 0; j < F - 1; ++j)
+      if (r + j < n) batch_fold4<PR, WIDE, FULL>(c[j], tab, tn, g, f, m);
+  }
+}
+
+template <bool PR>
+__device__ __forceinline__ void batch_tree(int from, float& f, int32_t& m) {
+  for (int o = from; o > 0; o >>= 1) {
+    if (PR) f += __shfl_xor_sync(0xffffffffu, f, o);
+    else m = min(m, __shfl_xor_sync(0xffffffffu, m, o));
   }
 }
 
@@ -158,11 +239,121 @@ __device__ bool team_barrier(const BatchArgs& a, unsigned int* t, int team, int 
   return s_ok != 0;
 }
 
-__global__ void batch_kernel(BatchArgs a) {
+// What a superstep's sweep needs, in shared memory: the same for the whole
+// CTA, and more than the registers of 2048 threads per SM hold.
+struct BatchStep {
+  const void* ids;
+  const BatchUnit* units;
+  const uint32_t* g;      // current values (PageRank: contributions) in global memory
+  const void* src;        // current ranks or labels
+  void* dst;              // next ones
+  float* dcon;            // next contributions
+  const int32_t* od;
+  double damping, inv_n;
+  int n_units, member, team, step, dual, tn;
+  int tab, next;          // table's current and next buffer
+  int s_next;             // next unit of this CTA's share, claimed by warps as they finish
+};
+
+// The new value of local vertex k; 1 when it changed.
+template <bool PR>
+__device__ __forceinline__ unsigned batch_apply(const BatchStep& st, uint32_t* s_tab, int k, float acc, int32_t low,
+                                                uint32_t old_bits, int32_t od) {
+  if constexpr (PR) {
+    const float nv = static_cast<float>(__dadd_rn(__dmul_rn(static_cast<double>(acc), st.damping), st.inv_n));
+    const float old = __uint_as_float(old_bits);
+    static_cast<float*>(st.dst)[k] = nv;
+    const float c = nv / static_cast<float>(od > 0 ? od : 1);
+    if (st.dual) s_tab[st.next + k] = __float_as_uint(c);
+    else st.dcon[k] = c;
+    return nv != (st.step == 0 ? 0.f : old);
+  } else {
+    const int32_t old = st.dual ? static_cast<int32_t>(s_tab[st.tab + k]) : static_cast<int32_t>(old_bits);
+    const int32_t nv = min(old, low);
+    if (st.dual) s_tab[st.next + k] = static_cast<uint32_t>(nv);
+    else static_cast<int32_t*>(st.dst)[k] = nv;
+    return nv != (st.step == 0 ? 0 : old);
+  }
+}
+
+// One superstep's units of this CTA's share; returns the warp's changes.
+// Member `member` of the team takes units member, member + team, ..., claimed
+// from st.s_next.
+template <bool PR, bool WIDE, bool FULL>
+__device__ __forceinline__ unsigned batch_sweep(BatchStep& st, uint32_t* s_tab, int lane) {
+  unsigned changed = 0;
+  const uint32_t* tab = s_tab + st.tab;
+  const uint32_t* g = st.g;
+  const void* ids = st.ids;
+  const int tn = st.tn;
+  auto claim = [&]() -> int {
+    int k = 0;
+    if (lane == 0) k = atomicAdd(&st.s_next, 1);
+    const int64_t t = st.member + static_cast<int64_t>(__shfl_sync(0xffffffffu, k, 0)) * st.team;
+    return t < st.n_units ? static_cast<int>(t) : -1;
+  };
+  int t = claim();
+  int4 next = make_int4(0, 0, 0, 0);
+  if (t >= 0) next = *reinterpret_cast<const int4*>(st.units + t);
+  while (t >= 0) {
+    const int4 u = next;
+    t = claim();
+    if (t >= 0) next = *reinterpret_cast<const int4*>(st.units + t);  // in flight while u is swept
+    const int kind = u.y >> 8, cnt = u.y & 255;
+    uint32_t old = 0;
+    int32_t od = 0;
+    if (lane < cnt) {  // likewise
+      if (PR) od = st.od[u.x + lane];
+      if (PR || !st.dual) old = __ldcg(static_cast<const uint32_t*>(st.src) + u.x + lane);
+    }
+    float f = 0.f;
+    int32_t m = 0x7fffffff;
+    if (kind == kUnitTile) {
+      batch_rounds<PR, WIDE, FULL>(ids, u.z, u.w, lane, tab, tn, g, f, m);
+    } else if (kind == kUnitHalf) {
+      BatchIds<WIDE> c[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if (r < u.w) c[r] = batch_load<WIDE>(ids, u.z + r, lane);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        if (r < u.w) {
+          float fl = 0.f;
+          int32_t ml = 0x7fffffff;
+          batch_fold4<PR, WIDE, FULL>(c[r], tab, tn, g, fl, ml);
+          batch_tree<PR>(8, fl, ml);
+          const float fr = __shfl_sync(0xffffffffu, fl, (lane & 1) << 4);
+          const int32_t mr = __shfl_sync(0xffffffffu, ml, (lane & 1) << 4);
+          if ((lane >> 1) == r) {
+            f = fr;
+            m = mr;
+          }
+        }
+      }
+    } else {
+      for (int i = 0; i < cnt; ++i) {
+        float fl = 0.f;
+        int32_t ml = 0x7fffffff;
+        batch_rounds<PR, WIDE, FULL>(ids, u.z + static_cast<int64_t>(i) * u.w, u.w, lane, tab, tn, g, fl, ml);
+        batch_tree<PR>(16, fl, ml);
+        if (lane == i) {
+          f = fl;
+          m = ml;
+        }
+      }
+    }
+    if (lane < cnt) changed += batch_apply<PR>(st, s_tab, u.x + lane, f, m, old, od);
+    __syncwarp();
+  }
+  return __reduce_add_sync(0xffffffffu, changed);
+}
+
+__global__ void __launch_bounds__(1024, 1) batch_kernel(const __grid_constant__ BatchArgs a) {
+  extern __shared__ __align__(16) uint32_t s_tab[];
+  __shared__ BatchStep s_st;
   __shared__ int s_slot;
   __shared__ unsigned int s_changed;
-  __shared__ int s_next;  // next tile of this CTA's share, claimed by warps as they finish
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31;
   for (;;) {
     if (threadIdx.x == 0) s_slot = static_cast<int>(atomicAdd(a.ctr, 1u));
     __syncthreads();
@@ -174,149 +365,329 @@ __global__ void batch_kernel(BatchArgs a) {
     const int inst = sl.x, member = sl.y >> 16, team = sl.y & 0xffff;
     unsigned int* tstate = a.team + 4 * static_cast<int64_t>(inst);
     const int32_t vb = a.vbeg[inst], ve = a.vbeg[inst + 1], n = ve - vb;
-    const int tiles = (n + 31) / 32;
     const double inv_n = 1.0 / n;
     const int vt0 = member * blockDim.x + threadIdx.x, vstride = blockDim.x * team;
+    // The table: both buffers of an instance that one CTA holds and that fits
+    // twice (`dual`: nothing is kept in global memory then), else the current
+    // values of the first tn vertices; after each buffer the unused place's.
+    const bool dual = batch_dual(n, team, a.tab);
+    const int tn = batch_table(n, a.tab);
     int bar = 0;
     // The barrier that ends a phase: a CTA barrier, or the team's.
     auto sync_count = [&](unsigned mine, unsigned* total) -> bool {
-      if (team == 1) {
-        if (threadIdx.x == 0) s_changed = 0;
-        __syncthreads();
-        if (threadIdx.x == 0) s_next = 0;
-        if (lane == 0 && mine) atomicAdd(&s_changed, mine);
-        __syncthreads();
-        *total = s_changed;
-        __syncthreads();
-        return true;
-      }
       if (threadIdx.x == 0) s_changed = 0;
       __syncthreads();
-      if (threadIdx.x == 0) s_next = 0;
+      if (threadIdx.x == 0) s_st.s_next = 0;
       if (lane == 0 && mine) atomicAdd(&s_changed, mine);
       __syncthreads();
       const unsigned cta = s_changed;
+      if (team == 1) {
+        *total = cta;
+        __syncthreads();
+        return true;
+      }
       return team_barrier(a, tstate, team, member, bar++, threadIdx.x == 0 ? cta : 0u, total);
+    };
+    // The table's copy of the values a finished phase left in g (through L2:
+    // other CTAs of the team wrote them).
+    auto fill = [&](const uint32_t* g) {
+      for (int i = threadIdx.x; i < tn; i += blockDim.x) s_tab[i] = __ldcg(g + i);
+      __syncthreads();
+    };
+    if (threadIdx.x == 0) {
+      s_st.ids = a.ids + 32 * a.round_base[inst];
+      s_st.units = a.units + vb;
+      s_st.n_units = a.n_units[inst];
+      s_st.member = member;
+      s_st.team = team;
+      s_st.dual = dual;
+      s_st.tn = tn;
+      s_st.od = a.od + vb;
+      s_st.damping = a.damping;
+      s_st.inv_n = inv_n;
+    }
+    // Superstep `step` from buffer `cur` (x0, x1: ranks or labels; c0, c1:
+    // contributions); the changes of this warp.
+    auto sweep = [&](auto pr, int step, int cur, void* x0, void* x1, float* c0, float* c1) -> unsigned {
+      constexpr bool PR = decltype(pr)::value;
+      if (threadIdx.x == 0) {
+        s_st.step = step;
+        s_st.src = cur ? x1 : x0;
+        s_st.dst = cur ? x0 : x1;
+        s_st.dcon = cur ? c0 : c1;
+        s_st.g = static_cast<const uint32_t*>(PR ? (cur ? c1 : c0) : (cur ? x1 : x0));
+        s_st.tab = dual && cur ? n + 1 : 0;
+        s_st.next = cur ? 0 : n + 1;
+      }
+      __syncthreads();
+      const bool wide = n >= kBatchWide;
+      if (tn == n)
+        return wide ? batch_sweep<PR, true, true>(s_st, s_tab, lane) : batch_sweep<PR, false, true>(s_st, s_tab, lane);
+      return wide ? batch_sweep<PR, true, false>(s_st, s_tab, lane) : batch_sweep<PR, false, false>(s_st, s_tab, lane);
+    };
+    auto unused = [&](uint32_t x) {
+      if (threadIdx.x == 0) {
+        s_tab[tn] = x;
+        if (dual) s_tab[2 * n + 1] = x;
+      }
     };
     unsigned tot = 0;
     // ---- PageRank ----
-    for (int v = vb + vt0; v < ve; v += vstride) {
+    unused(0u);
+    for (int k = vt0; k < n; k += vstride) {
       const float r0 = static_cast<float>(inv_n);
-      const int32_t od = a.outdeg[v];
-      a.pr0[v] = r0;
-      a.con0[v] = r0 / static_cast<float>(od > 0 ? od : 1);
+      const int32_t od = a.od[vb + k];
+      a.pr0[vb + k] = r0;
+      const float c = r0 / static_cast<float>(od > 0 ? od : 1);
+      if (dual) s_tab[k] = __float_as_uint(c);
+      else a.con0[vb + k] = c;
     }
     if (!sync_count(0, &tot)) return;
+    if (!dual) fill(reinterpret_cast<const uint32_t*>(a.con0 + vb));
     int cur = 0, step = 0;
     for (step = 0; step < a.pr_iters; ++step) {
-      // Ternaries, not a[cur]: runtime indexing of a parameter array would
-      // copy the parameter block to local memory.
-      const float* con = cur ? a.con1 : a.con0;
-      const float* src = cur ? a.pr1 : a.pr0;
-      float* dst = cur ? a.pr0 : a.pr1;
-      float* dcon = cur ? a.con0 : a.con1;
-      unsigned changed = 0;
-      for (;;) {
-        int k = 0;
-        if (lane == 0) k = atomicAdd(&s_next, 1);
-        k = __shfl_sync(0xffffffffu, k, 0);
-        const int t = member + k * team;  // this CTA's tiles: member, member + team, ...
-        if (t >= tiles) break;
-        const int v = vb + 32 * t + lane;
-        const bool valid = v < ve;
-        int64_t beg = 0, end = 0;
-        if (valid) {
-          beg = a.off[v];
-          end = a.off[v + 1];
-        }
-        float acc = 0.f;
-        int32_t dummy = 0;
-        batch_vertex_lists<true>(a, con, nullptr, beg, end, valid, acc, dummy, lane);
-        if (valid) {
-          const float nv = static_cast<float>(__dadd_rn(__dmul_rn(static_cast<double>(acc), a.damping), inv_n));
-          const float old = src[v];
-          changed += nv != (step == 0 ? 0.f : old);
-          dst[v] = nv;
-          const int32_t od = a.outdeg[v];
-          dcon[v] = nv / static_cast<float>(od > 0 ? od : 1);
-        }
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) changed += __shfl_xor_sync(0xffffffffu, changed, o);
+      const unsigned changed = sweep(std::true_type(), step, cur, a.pr0 + vb, a.pr1 + vb, a.con0 + vb, a.con1 + vb);
       if (!sync_count(changed, &tot)) return;
       cur ^= 1;
       if (tot == 0 && step > 1) {
         ++step;
         break;
       }
+      if (!dual) fill(reinterpret_cast<const uint32_t*>((cur ? a.con1 : a.con0) + vb));
     }
-    for (int v = vb + vt0; v < ve; v += vstride) a.pr_out[v] = (cur ? a.pr1 : a.pr0)[v];
+    for (int k = vt0; k < n; k += vstride) a.pr_out[a.inv[vb + k]] = __ldcg((cur ? a.pr1 : a.pr0) + vb + k);
     if (threadIdx.x == 0 && member == 0) a.pr_steps[inst] = step < a.pr_iters ? step : a.pr_iters;
+    __syncthreads();
     // ---- CC ----
-    for (int v = vb + vt0; v < ve; v += vstride) a.lab0[v] = v - vb;
+    unused(0x7fffffffu);
+    for (int k = vt0; k < n; k += vstride) {
+      const int32_t label = a.inv[vb + k] - vb;
+      if (dual) s_tab[k] = static_cast<uint32_t>(label);
+      else a.lab0[vb + k] = label;
+    }
     if (!sync_count(0, &tot)) return;
+    if (!dual) fill(reinterpret_cast<const uint32_t*>(a.lab0 + vb));
     cur = 0;
     for (step = 0; step < a.cc_max; ++step) {
-      const int32_t* src = cur ? a.lab1 : a.lab0;
-      int32_t* dst = cur ? a.lab0 : a.lab1;
-      unsigned changed = 0;
-      for (;;) {
-        int k = 0;
-        if (lane == 0) k = atomicAdd(&s_next, 1);
-        k = __shfl_sync(0xffffffffu, k, 0);
-        const int t = member + k * team;
-        if (t >= tiles) break;
-        const int v = vb + 32 * t + lane;
-        const bool valid = v < ve;
-        int64_t beg = 0, end = 0;
-        int32_t old = 0;
-        if (valid) {
-          beg = a.off[v];
-          end = a.off[v + 1];
-          old = src[v];
-        }
-        float dummy = 0.f;
-        int32_t acc = old;
-        batch_vertex_lists<false>(a, nullptr, src, beg, end, valid, dummy, acc, lane);
-        if (valid) {
-          changed += acc != (step == 0 ? 0 : old);
-          dst[v] = acc;
-        }
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) changed += __shfl_xor_sync(0xffffffffu, changed, o);
+      const unsigned changed = sweep(std::false_type(), step, cur, a.lab0 + vb, a.lab1 + vb, nullptr, nullptr);
       if (!sync_count(changed, &tot)) return;
       cur ^= 1;
       if (tot == 0 && step > 1) {
         ++step;
         break;
       }
+      if (!dual) fill(reinterpret_cast<const uint32_t*>((cur ? a.lab1 : a.lab0) + vb));
     }
-    for (int v = vb + vt0; v < ve; v += vstride) a.cc_out[v] = (cur ? a.lab1 : a.lab0)[v];
+    for (int k = vt0; k < n; k += vstride)
+      a.cc_out[a.inv[vb + k]] =
+          dual ? static_cast<int32_t>(s_tab[(cur ? n + 1 : 0) + k]) : __ldcg((cur ? a.lab1 : a.lab0) + vb + k);
     if (threadIdx.x == 0 && member == 0) a.cc_steps[inst] = step < a.cc_max ? step : a.cc_max;
     __syncthreads();
   }
 }
 
-__global__ void batch_check_kernel(const int64_t* off, const int32_t* col, const int32_t* vbeg, int32_t n,
-                                   int32_t V, unsigned int* bad) {
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-    int lo = 0, hi = n;  // instance of v: vbeg[lo] <= v < vbeg[lo + 1]
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (vbeg[mid] <= v) lo = mid;
-      else hi = mid;
+// CTAs take the instances in turn: every edge must stay inside its instance
+// (read end to end, four ids a thread: a thread per vertex, walking its list,
+// took 3.6 ms for 290 M edges).
+__global__ void __launch_bounds__(512) batch_check_kernel(const int64_t* off, const int32_t* col, const int32_t* vbeg,
+                                                          int32_t n_inst, unsigned int* bad) {
+  unsigned c = 0;
+  for (int i = blockIdx.x / kCheckSplit; i < n_inst; i += gridDim.x / kCheckSplit) {
+    const int32_t vb = vbeg[i], ve = vbeg[i + 1];
+    const int64_t b = off[vb], e = off[ve], part = blockIdx.x % kCheckSplit;
+    for (int64_t q = (b & ~3ll) + 4 * (part * blockDim.x + threadIdx.x); q < e; q += 4 * kCheckSplit * blockDim.x) {
+      const int4 x = __ldcs(reinterpret_cast<const int4*>(col + q));
+      const int32_t cs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) c += q + j >= b && q + j < e && (cs[j] < vb || cs[j] >= ve);
     }
-    const int32_t b = vbeg[lo], e = vbeg[lo + 1];
-    unsigned c = 0;
-    for (int64_t k = off[v]; k < off[v + 1]; ++k) c += (col[k] < b || col[k] >= e);
-    if (c) atomicAdd(bad, c);
+  }
+  if (c) atomicAdd(bad, c);
+}
+
+// Length classes of an instance's lists, in the order of its new ids: across
+// the warp by rounds (63 or more first), across half a warp, then a lane's by
+// rounds.  lo: the first edge's position in its aligned group of four.
+constexpr int kClassCap = 63;
+constexpr int kClassHalf = kClassCap, kClassLane = kClassHalf + 1, kClasses = kClassLane + kClassCap + 1;
+__device__ __forceinline__ int batch_class(int64_t beg, int64_t len, int lane_max) {
+  if (len <= lane_max) {
+    const int64_t r = (len + 3) / 4;
+    return kClassLane + kClassCap - static_cast<int>(r < kClassCap ? r : kClassCap);
+  }
+  const int64_t q = (beg & 3) + len;
+  if (q <= 64) return kClassHalf;
+  const int64_t r = (q + 127) / 128;
+  return kClassCap - static_cast<int>(r < kClassCap ? r : kClassCap);
+}
+// Lists across the warp of up to this many rounds share a unit, four to each.
+constexpr int kWarpShare = 4;
+
+// An instance per CTA (taken in turn): its vertices in order of their
+// classes, and its units.  Within a class the order is that of the atomics:
+// no result depends on it.
+__global__ void __launch_bounds__(kBatchSortThreads) batch_sort_kernel(const __grid_constant__ BatchArgs a) {
+  __shared__ int s_at[kClasses + 1];
+  __shared__ int s_cur[kClasses];
+  __shared__ unsigned long long s_w[kBatchSortThreads / 32], s_run;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (int i = blockIdx.x; i < a.n_inst; i += gridDim.x) {
+    const int32_t vb = a.vbeg[i], n = a.vbeg[i + 1] - vb;
+    for (int c = threadIdx.x; c < kClasses; c += kBatchSortThreads) s_cur[c] = 0;
+    __syncthreads();
+    for (int k = threadIdx.x; k < n; k += kBatchSortThreads) {
+      const int64_t beg = a.off[vb + k];
+      atomicAdd(&s_cur[batch_class(beg, a.off[vb + k + 1] - beg, a.lane_max)], 1);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int run = 0;
+      for (int c = 0; c < kClasses; ++c) {
+        s_at[c] = run;
+        run += s_cur[c];
+        s_cur[c] = s_at[c];
+      }
+      s_at[kClasses] = run;
+      s_run = 0;
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < n; k += kBatchSortThreads) {
+      const int64_t beg = a.off[vb + k];
+      const int p = atomicAdd(&s_cur[batch_class(beg, a.off[vb + k + 1] - beg, a.lane_max)], 1);
+      a.perm[vb + k] = p;
+      a.inv[vb + p] = vb + k;
+      a.od[vb + p] = a.outdeg[vb + k];
+    }
+    __syncthreads();
+    // Units: the warp lists of many rounds one each, the others four to a
+    // unit, the half-warp lists eight to a unit, the lane lists 32.
+    const int n_one = s_at[kClassCap - kWarpShare], n_warp = s_at[kClassHalf], n_wide = s_at[kClassLane];
+    const int u_one = n_one, u_warp = u_one + (n_warp - n_one + 3) / 4, u_half = u_warp + (n_wide - n_warp + 7) / 8;
+    const int u_all = u_half + (n - n_wide + 31) / 32;
+    for (int u0 = 0; u0 < u_all; u0 += kBatchSortThreads) {
+      const int u = u0 + threadIdx.x;
+      BatchUnit x{0, 0, 0, 0};
+      unsigned long long total = 0;
+      if (u < u_all) {
+        int last;
+        if (u < u_warp) {
+          x.first = u < u_one ? u : n_one + 4 * (u - u_one);
+          last = u < u_one ? x.first + 1 : min(x.first + 4, n_warp);
+          x.kind_cnt = kUnitWarp << 8 | (last - x.first);
+        } else if (u < u_half) {
+          x.first = n_warp + 8 * (u - u_warp);
+          last = min(x.first + 8, n_wide);
+          x.kind_cnt = kUnitHalf << 8 | (last - x.first);
+          x.rounds = (last - x.first + 1) / 2;
+          total = x.rounds;
+        } else {
+          x.first = n_wide + 32 * (u - u_half);
+          last = min(x.first + 32, n);
+          x.kind_cnt = kUnitTile << 8 | (last - x.first);
+        }
+        if (u < u_warp || u >= u_half) {
+          int64_t most = 0;
+          for (int k = x.first; k < last; ++k) {
+            const int64_t beg = a.off[a.inv[vb + k]], len = a.off[a.inv[vb + k] + 1] - beg;
+            const int64_t r = u < u_warp ? ((beg & 3) + len + 127) / 128 : (len + 3) / 4;
+            most = r > most ? r : most;
+          }
+          x.rounds = static_cast<int32_t>(most);
+          total = u < u_warp ? static_cast<unsigned long long>(most) * (last - x.first) : most;
+        }
+      }
+      unsigned long long incl = total;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      if (lane == 31) s_w[wid] = incl;
+      __syncthreads();
+      unsigned long long before = s_run, all = 0;
+      for (int w = 0; w < kBatchSortThreads / 32; ++w) {
+        before += w < wid ? s_w[w] : 0;
+        all += s_w[w];
+      }
+      if (u < u_all) {
+        x.at = static_cast<int32_t>(before + incl - total);
+        a.units[vb + u] = x;
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) s_run += all;
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+      a.n_units[i] = u_all;
+      a.rounds[i] = n >= kBatchWide ? 2 * s_run : s_run;
+    }
+    __syncthreads();
+  }
+}
+
+// Writes the rounds: kFillSplit CTAs share an instance, a warp per unit.
+__global__ void __launch_bounds__(256) batch_fill_kernel(const __grid_constant__ BatchArgs a) {
+  const int lane = threadIdx.x & 31;
+  const int w0 = (blockIdx.x % kFillSplit) * 8 + (threadIdx.x >> 5);
+  for (int i = blockIdx.x / kFillSplit; i < a.n_inst; i += gridDim.x / kFillSplit) {
+    const int32_t vb = a.vbeg[i], n = a.vbeg[i + 1] - vb;
+    const int tn = batch_table(n, a.tab);
+    const bool wide = n >= kBatchWide;
+    uint2* ids = a.ids + 32 * a.round_base[i];
+    for (int t = w0; t < a.n_units[i]; t += kFillSplit * 8) {
+      const BatchUnit u = a.units[vb + t];
+      const int kind = u.kind_cnt >> 8, cnt = u.kind_cnt & 255;
+      // The vertex and the position of this lane's first place in each round.
+      int64_t beg = 0, len = 0;
+      int k_now = -1;
+      const int rounds = kind == kUnitWarp ? cnt * u.rounds : u.rounds;
+      for (int r = 0; r < rounds; ++r) {
+        int k;       // vertex of the unit
+        int64_t q;   // first edge of the lane's four, counted from the list's start
+        if (kind == kUnitTile) {
+          k = lane;
+          q = 4ll * r;
+        } else if (kind == kUnitHalf) {
+          k = 2 * r + (lane >> 4);
+          q = 4ll * (lane & 15);
+        } else {
+          k = r / u.rounds;
+          q = 128ll * (r % u.rounds) + 4ll * lane;
+        }
+        if (k != k_now) {
+          k_now = k;
+          len = 0;
+          if (k < cnt) {
+            const int32_t v = a.inv[vb + u.first + k];
+            beg = a.off[v];
+            len = a.off[v + 1] - beg;
+          }
+        }
+        if (kind != kUnitTile) q -= beg & 3;
+        int32_t c[4];
+        uint32_t id[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c[j] = q + j >= 0 && q + j < len ? __ldg(a.col + beg + q + j) : -1;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int p = c[j] >= 0 ? __ldg(a.perm + c[j]) : tn;
+          id[j] = static_cast<uint32_t>(c[j] >= 0 && p >= tn ? p + 1 : p);
+        }
+        const int64_t at = u.at + static_cast<int64_t>(r);
+        if (wide) reinterpret_cast<uint4*>(ids)[at * 32 + lane] = make_uint4(id[0], id[1], id[2], id[3]);
+        else ids[at * 32 + lane] = make_uint2(id[0] | id[1] << 16, id[2] | id[3] << 16);
+      }
+    }
   }
 }
 
 struct BatchDev {
   int32_t *vbeg = nullptr, *lab0 = nullptr, *lab1 = nullptr, *cc_out = nullptr;
   int32_t *pr_steps = nullptr, *cc_steps = nullptr;
+  int32_t *inv = nullptr, *perm = nullptr, *od = nullptr, *n_units = nullptr;
+  BatchUnit* units = nullptr;
+  unsigned long long *rounds = nullptr, *round_base = nullptr;
+  uint2* ids = nullptr;
   float *pr0 = nullptr, *pr1 = nullptr, *con0 = nullptr, *con1 = nullptr, *pr_out = nullptr;
   unsigned int* ctr = nullptr;
   int2* slots = nullptr;
@@ -334,6 +705,14 @@ struct BatchDev {
     dev_free(&cc_out);
     dev_free(&pr_steps);
     dev_free(&cc_steps);
+    dev_free(&inv);
+    dev_free(&perm);
+    dev_free(&od);
+    dev_free(&n_units);
+    dev_free(&units);
+    dev_free(&rounds);
+    dev_free(&round_base);
+    dev_free(&ids);
     dev_free(&pr0);
     dev_free(&pr1);
     dev_free(&con0);
@@ -370,10 +749,17 @@ gx_status batch_prepare(gx_engine* e, int32_t n, const int32_t* vbeg, BatchDev& 
   GX_TRY(dev_alloc(&d.pr_steps, static_cast<size_t>(n)));
   GX_TRY(dev_alloc(&d.cc_steps, static_cast<size_t>(n)));
   GX_TRY(dev_alloc(&d.ctr, 1));
+  GX_TRY(dev_alloc(&d.inv, static_cast<size_t>(V)));
+  GX_TRY(dev_alloc(&d.perm, static_cast<size_t>(V)));
+  GX_TRY(dev_alloc(&d.od, static_cast<size_t>(V)));
+  GX_TRY(dev_alloc(&d.units, static_cast<size_t>(V)));
+  GX_TRY(dev_alloc(&d.n_units, static_cast<size_t>(n)));
+  GX_TRY(dev_alloc(&d.rounds, static_cast<size_t>(n)));
+  GX_TRY(dev_alloc(&d.round_base, static_cast<size_t>(n)));
   GX_CUDA(cudaMemcpy(d.vbeg, vbeg, sizeof(int32_t) * (n + 1), cudaMemcpyHostToDevice));
   // Every edge must stay inside its instance (a block-diagonal CSC).
   GX_CUDA(cudaMemset(d.ctr, 0, sizeof(unsigned int)));
-  batch_check_kernel<<<e->n_sm * 8, 256, 0, e->s_comp>>>(e->d_off, e->d_col, d.vbeg, n, V, d.ctr);
+  batch_check_kernel<<<e->n_sm * 4, 512, 0, e->s_comp>>>(e->d_off, e->d_col, d.vbeg, n, d.ctr);
   unsigned int bad = 0;
   GX_CUDA(cudaMemcpyAsync(&bad, d.ctr, sizeof(bad), cudaMemcpyDeviceToHost, e->s_comp));
   GX_CUDA(cudaStreamSynchronize(e->s_comp));
@@ -398,6 +784,46 @@ gx_status batch_prepare(gx_engine* e, int32_t n, const int32_t* vbeg, BatchDev& 
   a.cc_out = d.cc_out;
   a.pr_steps = d.pr_steps;
   a.cc_steps = d.cc_steps;
+  a.inv = d.inv;
+  a.perm = d.perm;
+  a.od = d.od;
+  a.units = d.units;
+  a.n_units = d.n_units;
+  a.rounds = d.rounds;
+  a.round_base = d.round_base;
+  return GX_OK;
+}
+
+// Shared memory of a CTA's table: the SM's, less what the index loads need as
+// L1, shared out among the CTAs wanted (1 KB each is the system's).
+gx_status batch_table_bytes(gx_engine* e, const gx_batch_tuning& t, int* bytes) {
+  int smem_sm = 0, optin = 0, per_sm = 0;
+  GX_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, e->dev));
+  GX_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, e->dev));
+  cudaFuncAttributes attr{};
+  GX_CUDA(cudaFuncGetAttributes(&attr, batch_kernel));
+  const int fixed = static_cast<int>(attr.sharedSizeBytes);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel, t.threads, 0);
+  const int want = std::max(1, std::min(per_sm, t.ctas_per_sm));
+  *bytes = std::max(64, std::min(optin - fixed, (smem_sm - kBatchL1) / want - 1024 - fixed)) & ~15;
+  return GX_OK;
+}
+
+// The schedule of a call that names none: the default's two CTAs of 512
+// threads per SM, or one of 1024 with twice the table where most of the work
+// is in instances that the default's table does not hold whole (512 R-MAT
+// instances of scales 10 to 17: 32.6 -> 26.8 ms a call; 2000 of scales 6 to
+// 12, which it does hold: 2.2 ms against 2.6).
+gx_status batch_default_schedule(gx_engine* e, int32_t n, const int32_t* vbeg, const BatchDev& d, gx_batch_tuning* t) {
+  gx_batch_tuning_default(t);
+  int smem = 0;
+  GX_TRY(batch_table_bytes(e, *t, &smem));
+  int64_t in = 0, out = 0;
+  for (int32_t i = 0; i < n; ++i) (vbeg[i + 1] - vbeg[i] < smem / 4 ? in : out) += d.work[i];
+  if (out > in) {
+    t->threads = 1024;
+    t->ctas_per_sm = 1;
+  }
   return GX_OK;
 }
 
@@ -406,7 +832,11 @@ gx_status batch_prepare(gx_engine* e, int32_t n, const int32_t* vbeg, BatchDev& 
 gx_status batch_launch(gx_engine* e, BatchDev& d, BatchArgs& a, const gx_batch_tuning& t, float* ms) {
   cudaStream_t s = e->s_comp;
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel, t.threads, 0);
+  int smem = 0;
+  GX_TRY(batch_table_bytes(e, t, &smem));
+  a.tab = smem / 4;
+  GX_CUDA(cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel, t.threads, smem);
   if (per_sm < 1) return fail(GX_ERR_INVALID, "gx_batch: %d threads per CTA do not fit an SM", t.threads);
   const int blocks = std::min(per_sm, t.ctas_per_sm) * e->n_sm;
   // Work slots: an instance above half a CTA's fair share gets a team of up
@@ -425,28 +855,43 @@ gx_status batch_launch(gx_engine* e, BatchDev& d, BatchArgs& a, const gx_batch_t
   GX_CUDA(cudaMemcpy(d.slots, slots.data(), sizeof(int2) * slots.size(), cudaMemcpyHostToDevice));
   a.slots = d.slots;
   a.n_slots = static_cast<int32_t>(slots.size());
+  cudaEvent_t e0, e1;
+  GX_CUDA(cudaEventCreate(&e0));
+  GX_CUDA(cudaEventCreate(&e1));
+  std::unique_ptr<CUevent_st, cudaError_t (*)(cudaEvent_t)> e0_g(e0, cudaEventDestroy), e1_g(e1, cudaEventDestroy);
+  cudaEventRecord(e0, s);
+  // The instances rewritten for this schedule.
+  batch_sort_kernel<<<std::min(a.n_inst, e->n_sm * 4), kBatchSortThreads, 0, s>>>(a);
+  GX_CUDA(cudaGetLastError());
+  std::vector<unsigned long long> blocks_of(static_cast<size_t>(a.n_inst)), base(static_cast<size_t>(a.n_inst));
+  GX_CUDA(cudaMemcpyAsync(blocks_of.data(), d.rounds, sizeof(unsigned long long) * a.n_inst, cudaMemcpyDeviceToHost, s));
+  GX_CUDA(cudaStreamSynchronize(s));
+  unsigned long long n_blocks = 0;
+  for (int32_t i = 0; i < a.n_inst; ++i) {
+    base[i] = n_blocks;
+    n_blocks += blocks_of[i];
+  }
+  GX_TRY(dev_alloc(&d.ids, static_cast<size_t>(n_blocks) * 32));
+  a.ids = d.ids;
+  GX_CUDA(cudaMemcpyAsync(d.round_base, base.data(), sizeof(unsigned long long) * a.n_inst, cudaMemcpyHostToDevice, s));
+  batch_fill_kernel<<<std::min(a.n_inst, e->n_sm) * kFillSplit, 256, 0, s>>>(a);
+  GX_CUDA(cudaGetLastError());
   cudaGraph_t graph;
   cudaGraphExec_t exec;
   GX_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   cudaMemsetAsync(a.ctr, 0, sizeof(unsigned int), s);
   cudaMemsetAsync(a.team, 0, sizeof(unsigned int) * 4 * static_cast<size_t>(a.n_inst), s);
   cudaMemsetAsync(a.abort, 0, sizeof(unsigned int), s);
-  batch_kernel<<<blocks, t.threads, 0, s>>>(a);
+  batch_kernel<<<blocks, t.threads, smem, s>>>(a);
   GX_CUDA(cudaStreamEndCapture(s, &graph));
   cudaError_t err = cudaGraphInstantiate(&exec, graph, 0);
   cudaGraphDestroy(graph);
   if (err != cudaSuccess) return fail(GX_ERR_CUDA, "gx_batch: graph instantiate: %s", cudaGetErrorString(err));
-  cudaEvent_t e0, e1;
-  cudaEventCreate(&e0);
-  cudaEventCreate(&e1);
-  cudaEventRecord(e0, s);
   cudaGraphLaunch(exec, s);
   cudaEventRecord(e1, s);
   err = cudaEventSynchronize(e1);
   float t_ms = 0;
   cudaEventElapsedTime(&t_ms, e0, e1);
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
   cudaGraphExecDestroy(exec);
   if (err != cudaSuccess) return fail(GX_ERR_CUDA, "gx_batch: run failed: %s", cudaGetErrorString(err));
   unsigned int aborted = 0;
@@ -490,6 +935,7 @@ gx_status gx_batch_run(gx_engine* e, int32_t n_inst, const int32_t* inst_vbegin,
   BatchDev d;
   BatchArgs a;
   GX_TRY(batch_prepare(e, n_inst, inst_vbegin, d, a));
+  if (!tuning) GX_TRY(batch_default_schedule(e, n_inst, inst_vbegin, d, &t));
   a.pr_iters = pr_iters;
   a.cc_max = cc_max_iter;
   a.lane_max = t.lane_max;
@@ -513,7 +959,7 @@ gx_status gx_batch_run(gx_engine* e, int32_t n_inst, const int32_t* inst_vbegin,
     stats->edges_scanned = edges;
     stats->ms_total = ms;
     stats->ms_compute = ms;
-    stats->kernel_launches = 1;
+    stats->kernel_launches = 1;  // the supersteps; the call's preparation (check, sort, fill) is not counted
   }
   return GX_OK;
 }
