@@ -943,8 +943,8 @@ gx_status gx_batch_run(gx_engine* e, int32_t n_inst, const int32_t* inst_vbegin,
   float ms = 0;
   GX_TRY(batch_launch(e, d, a, t, &ms));
   const int32_t V = e->V;
-  if (pr_out) GX_CUDA(cudaMemcpy(pr_out, d.pr_out, sizeof(float) * V, cudaMemcpyDeviceToHost));
-  if (cc_out) GX_CUDA(cudaMemcpy(cc_out, d.cc_out, sizeof(int32_t) * V, cudaMemcpyDeviceToHost));
+  if (pr_out) GX_TRY(copy_to_host(e, pr_out, d.pr_out, sizeof(float) * static_cast<size_t>(V)));
+  if (cc_out) GX_TRY(copy_to_host(e, cc_out, d.cc_out, sizeof(int32_t) * static_cast<size_t>(V)));
   std::vector<int32_t> ps(n_inst), cs(n_inst);
   GX_CUDA(cudaMemcpy(ps.data(), d.pr_steps, sizeof(int32_t) * n_inst, cudaMemcpyDeviceToHost));
   GX_CUDA(cudaMemcpy(cs.data(), d.cc_steps, sizeof(int32_t) * n_inst, cudaMemcpyDeviceToHost));

@@ -19,6 +19,8 @@
 // compressed when that saves 30% of their bytes (encode_streamed).
 #include <cuda_runtime.h>
 #include <omp.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cstddef>
@@ -76,6 +78,53 @@ DevicePool* device_pool(int dev) {
     }
   }
   return g_pools[dev].pool ? &g_pools[dev] : nullptr;
+}
+
+// Where pages of a result's place are missing, writes a byte to every page with
+// the host's threads (the contents are about to be replaced).
+static void touch_host_pages(void* p, size_t bytes) {
+  const size_t page = static_cast<size_t>(sysconf(_SC_PAGESIZE));
+  const uintptr_t b = (reinterpret_cast<uintptr_t>(p) + page - 1) / page * page, e = reinterpret_cast<uintptr_t>(p) + bytes;
+  const int64_t n = e > b ? static_cast<int64_t>((e - b) / page) : 0;
+  if (n < 16) return;
+  std::vector<unsigned char> there(static_cast<size_t>(n));
+  if (mincore(reinterpret_cast<void*>(b), static_cast<size_t>(n) * page, there.data()) != 0) return;
+  int64_t missing = 0;
+  for (unsigned char x : there) missing += !(x & 1);
+  if (missing == 0) return;
+#pragma omp parallel for schedule(static)
+  for (int64_t i = 0; i < n; ++i) *reinterpret_cast<volatile unsigned char*>(b + static_cast<uintptr_t>(i) * page) = 0;
+}
+
+gx_status copy_to_host(gx_engine* e, void* dst, const void* src, size_t bytes) {
+  if (bytes < kStageFrom) {
+    touch_host_pages(dst, bytes);
+    GX_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost));
+    return GX_OK;
+  }
+  if (!e->h_stage) {
+    GX_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&e->h_stage), kStageSlots * kStageBytes, cudaHostAllocDefault));
+    for (cudaEvent_t& ev : e->stage_ready) GX_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  }
+  const size_t n = (bytes + kStageBytes - 1) / kStageBytes;
+  auto part = [&](size_t i) { return std::min(kStageBytes, bytes - i * kStageBytes); };
+  auto issue = [&](size_t i) -> cudaError_t {
+    cudaError_t err = cudaMemcpyAsync(e->h_stage + i % kStageSlots * kStageBytes,
+                                      static_cast<const char*>(src) + i * kStageBytes, part(i), cudaMemcpyDeviceToHost,
+                                      e->s_copy);
+    return err == cudaSuccess ? cudaEventRecord(e->stage_ready[i % kStageSlots], e->s_copy) : err;
+  };
+  for (size_t i = 0; i < std::min(n, kStageSlots); ++i) GX_CUDA(issue(i));
+  for (size_t i = 0; i < n; ++i) {
+    GX_CUDA(cudaEventSynchronize(e->stage_ready[i % kStageSlots]));
+    const char* from = e->h_stage + i % kStageSlots * kStageBytes;
+    char* to = static_cast<char*>(dst) + i * kStageBytes;
+    const int64_t len = static_cast<int64_t>(part(i)), piece = 64 * 1024;
+#pragma omp parallel for schedule(static)
+    for (int64_t k = 0; k < len; k += piece) memcpy(to + k, from + k, static_cast<size_t>(std::min(piece, len - k)));
+    if (i + kStageSlots < n) GX_CUDA(issue(i + kStageSlots));
+  }
+  return GX_OK;
 }
 
 }  // namespace gx
@@ -1722,8 +1771,7 @@ gx_status gx_get_values(gx_engine* e, void* host_out) {
     GX_TRY(values_to_caller(e, src, e->s_comp));
     src = e->d_stage;
   }
-  GX_CUDA(cudaMemcpy(host_out, src, sizeof(uint32_t) * e->V, cudaMemcpyDeviceToHost));
-  return GX_OK;
+  return copy_to_host(e, host_out, src, sizeof(uint32_t) * static_cast<size_t>(e->V));
 }
 
 gx_status gx_write_values_npy(gx_engine* e, const char* path) {

@@ -145,6 +145,8 @@ inline int app_kind(const gx_run_params& p) {
   return -1;
 }
 
+constexpr size_t kStageBytes = size_t(8) << 20, kStageSlots = 3, kStageFrom = size_t(128) << 20;
+
 }  // namespace gx
 
 struct gx_engine {
@@ -247,6 +249,10 @@ struct gx_engine {
   int64_t* d_off_old = nullptr;
   uint32_t* d_stage = nullptr;
 
+  // Pinned pieces through which large results go to the caller (copy_to_host).
+  char* h_stage = nullptr;
+  cudaEvent_t stage_ready[gx::kStageSlots] = {};
+
   std::vector<uint32_t> init_vals;
   bool has_init = false;
   bool device_init = false;          // next gx_run starts from d_val[0] as it is
@@ -348,6 +354,12 @@ struct gx_engine {
     gx::dev_free(&d_ctl);
     if (h_ctl) cudaFreeHost(h_ctl);
     h_ctl = nullptr;
+    if (h_stage) cudaFreeHost(h_stage);
+    h_stage = nullptr;
+    for (cudaEvent_t& ev : stage_ready) {
+      if (ev) cudaEventDestroy(ev);
+      ev = nullptr;
+    }
     if (s_comp) cudaStreamDestroy(s_comp);
     for (cudaStream_t cs : s_copies) cudaStreamDestroy(cs);
     s_copies.clear();
@@ -355,3 +367,17 @@ struct gx_engine {
   }
 };
 
+namespace gx {
+
+// Copies a finished result to the caller's memory.  A copy from the device
+// straight into pageable memory costs a fault from the device side, some 10 us
+// each and one at a time, for every page that is not there or that the kernel
+// has unmapped to watch its use.  So the host's threads touch the pages first
+// (28 MB, fresh: 24 -> 0.5 ms), and results of kStageFrom bytes go in pieces
+// through pinned memory, from where the threads move them: 268 MB took 225 ms
+// in a strided copy into fresh pages, 11 in a plain one, 2 into a buffer in
+// use, or 27 to 42 every few copies; through the pieces 3 to 5.  (Smaller ones
+// are slower that way: 64 MB takes a plain copy 0.4 ms, the pieces 1.1.)
+gx_status copy_to_host(gx_engine* e, void* dst, const void* src, size_t bytes);
+
+}  // namespace gx
