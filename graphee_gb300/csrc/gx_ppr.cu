@@ -12,10 +12,12 @@
 // All steps run in ONE persistent cooperative launch, captured in a CUDA
 // graph: CTAs sweep a step's work units, meet at a grid barrier (bounded by
 // config.wait_limit polls; a timeout raises an abort flag every CTA honours
-// and the call returns GX_ERR_TIMEOUT), and go on to the next step.  A unit
-// is one destination vertex, or a chunk of kPprChunk in-edges of a vertex
-// with more; its row is summed by a group of W/2 lanes (a float2 each), so a
-// warp works on 64/W units at once, from claims of kPprClaim units.  Chunked
+// and the call returns GX_ERR_TIMEOUT), and go on to the next step.  A row is
+// summed by a group of W/2 lanes (a float2 each), so a warp works on 64/W rows
+// at once.  What bounds a step is how many row gathers are in flight, and its
+// longest unit: units are the engine's edge-capped tiles, whose edges a group
+// streams eight at a time across the vertices' boundaries, and chunks of
+// kPprChunk in-edges of the vertices above kPprHeavy, a group each.  Chunked
 // vertices fold their partial rows in chunk order in the warp group that
 // finishes last, so results are deterministic.
 #include <cuda_runtime.h>
@@ -32,7 +34,8 @@ using namespace gx;
 namespace {
 
 constexpr int kPprMaxCols = 64;
-constexpr int kPprChunk = 1024;
+constexpr int kPprHeavy = 512;    // longest list a group streams inside its tile
+constexpr int kPprChunk = 256;    // edges of one chunk of a longer one
 constexpr int kPprThreads = 256;
 constexpr int kPprWarps = kPprThreads / 32;
 
@@ -42,14 +45,15 @@ struct PprArgs {
   const int32_t* outdeg;
   float* rs[2];             // R[u,:]/outdeg[u], double buffer [V][W]
   float* r_out;             // final R [V][W]
-  const int4* units;        // (v, chunk, n_chunks, partial base)
-  int32_t n_units;
+  const int2* tiles;        // the engine's units: tile (vb, ve), or x < 0 (not ours)
+  const int4* chunks;       // (v, chunk, n_chunks, partial base)
+  int32_t n_tiles, n_chunks;
   int32_t iters;
   unsigned int* ctr;        // kQueues work cursors per step
   unsigned int* arrive;     // grid-barrier arrival count per step
   unsigned int* abort;      // set when a grid barrier gives up
   unsigned int wait_limit;  // polls (of at least 64 ns) before it does
-  float* partial;           // [n_partial][W]
+  float* partial;           // [n_chunks][W]
   unsigned int* ticket;     // per chunked vertex, indexed by partial base
   const int32_t* src;       // [W] source vertex of each column (-1 past k)
   float alpha, restart;
@@ -81,107 +85,203 @@ __device__ bool ppr_grid_barrier(const PprArgs& a, int it) {
   return s_ok != 0;
 }
 
-template <int W>
-__device__ __forceinline__ void ppr_finish(const PprArgs& a, float* rs_out, float* r_out, int v, float2 acc,
-                                           int gl) {
-  float2 r = make_float2(a.alpha * acc.x, a.alpha * acc.y);
-  if (a.src[2 * gl] == v) r.x += a.restart;
-  if (a.src[2 * gl + 1] == v) r.y += a.restart;
-  const int32_t od = a.outdeg[v];
-  const float inv = 1.0f / static_cast<float>(od > 0 ? od : 1);
-  const size_t row = static_cast<size_t>(v) * W + 2 * gl;
-  if (r_out) *reinterpret_cast<float2*>(r_out + row) = r;
-  *reinterpret_cast<float2*>(rs_out + row) = make_float2(r.x * inv, r.y * inv);
+// The chunks of the vertices above kPprHeavy: counted (units null) or written,
+// each vertex's side by side from an index that an atomic gives out.
+__global__ void ppr_chunks_kernel(const int64_t* off, int32_t V, int4* units, unsigned int* count) {
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
+    const int64_t d = off[v + 1] - off[v];
+    if (d <= kPprHeavy) continue;
+    const int n = static_cast<int>((d + kPprChunk - 1) / kPprChunk);
+    const int base = static_cast<int>(atomicAdd(count, static_cast<unsigned>(n)));
+    if (units)
+      for (int c = 0; c < n; ++c) units[base + c] = make_int4(v, c, n, base);
+  }
 }
 
-// Units a warp claims per cursor atomic: most vertices of an R-MAT graph
-// have no in-edges, so a claim per unit would cost a round trip per empty row.
-constexpr int kPprClaim = 16;
+// What the lanes of a group hold: its columns and their sources.
+template <int W>
+struct PprGroup {
+  static constexpr int L = W / 2;   // lanes per row, a float2 each
+  static constexpr int G = 32 / L;  // groups of a warp
+  int gl, grp, s0, s1;
+  unsigned mask;
+
+  __device__ __forceinline__ void finish(const PprArgs& a, float* rs_out, bool last, int v, int32_t od,
+                                         float2 acc) const {
+    float2 r = make_float2(a.alpha * acc.x, a.alpha * acc.y);
+    if (s0 == v) r.x += a.restart;
+    if (s1 == v) r.y += a.restart;
+    const size_t row = static_cast<size_t>(v) * W + 2 * gl;
+    if (last) {
+      *reinterpret_cast<float2*>(a.r_out + row) = r;
+    } else {
+      const float inv = 1.0f / static_cast<float>(od > 0 ? od : 1);
+      *reinterpret_cast<float2*>(rs_out + row) = make_float2(r.x * inv, r.y * inv);
+    }
+  }
+
+  // Eight edges p[k .. k + 7] (16-byte aligned), those in [lo, hi) taken, in
+  // order; c holds their ids, loaded a step ahead.
+  __device__ __forceinline__ void ids(int32_t (&c)[8], const int32_t* p, int k, int hi) const {
+    int4 x = make_int4(0, 0, 0, 0), y = x;
+    if (k < hi) x = __ldg(reinterpret_cast<const int4*>(p + k));
+    if (k + 4 < hi) y = __ldg(reinterpret_cast<const int4*>(p + k + 4));
+    c[0] = x.x, c[1] = x.y, c[2] = x.z, c[3] = x.w, c[4] = y.x, c[5] = y.y, c[6] = y.z, c[7] = y.w;
+  }
+  __device__ __forceinline__ void rows(float2 (&x)[8], const int32_t (&c)[8], const float* rs_in, int k, int lo,
+                                       int hi) const {
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      x[t] = make_float2(0.f, 0.f);
+      if (k + t >= lo && k + t < hi)
+        x[t] = *(reinterpret_cast<const float2*>(rs_in + static_cast<size_t>(c[t]) * W) + gl);
+    }
+  }
+};
 
 template <int W>
-__global__ void __launch_bounds__(kPprThreads) ppr_kernel(const PprArgs a) {
-  constexpr int L = W / 2;   // lanes per row, a float2 each
-  constexpr int G = 32 / L;  // units a warp works on at once
+__global__ void __launch_bounds__(kPprThreads, 4) ppr_kernel(const __grid_constant__ PprArgs a) {
+  typedef PprGroup<W> Group;
+  constexpr int L = Group::L, G = Group::G;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int gl = lane % L, grp = lane / L;
-  const unsigned gmask = L == 32 ? 0xffffffffu : (((1u << L) - 1u) << (grp * L));
-  const int U = a.n_units;
+  Group q;
+  q.gl = lane % L;
+  q.grp = lane / L;
+  q.mask = L == 32 ? 0xffffffffu : (((1u << L) - 1u) << (q.grp * L));
+  q.s0 = a.src[2 * q.gl];
+  q.s1 = a.src[2 * q.gl + 1];
+  const int first_tile = (a.n_chunks + G - 1) / G, U = first_tile + a.n_tiles;
   const int nq = U / 256 < 1 ? 1 : (U / 256 < kQueues ? U / 256 : kQueues);
   for (int it = 0; it < a.iters; ++it) {
     const float* rs_in = (it & 1) ? a.rs[1] : a.rs[0];
     float* rs_out = (it & 1) ? a.rs[0] : a.rs[1];
-    float* r_out = it + 1 == a.iters ? a.r_out : nullptr;
+    const bool last = it + 1 == a.iters;
     unsigned int* ctr = a.ctr + static_cast<size_t>(kQueues) * kQueueStride * it;
-    int q = (blockIdx.x * kPprWarps + wid) % nq;
+    int qi = (blockIdx.x * kPprWarps + wid) % nq;
+    int claim = 0;  // in flight while the last unit is swept
+    if (lane == 0) claim = static_cast<int>(atomicAdd(ctr + qi * kQueueStride, 1u));
     for (;;) {
-      const int qb = static_cast<int>((static_cast<int64_t>(U) * q) / nq);
-      const int qe = static_cast<int>((static_cast<int64_t>(U) * (q + 1)) / nq);
-      int u0 = 0;
-      if (lane == 0) u0 = qb + static_cast<int>(atomicAdd(ctr + q * kQueueStride, static_cast<unsigned>(kPprClaim)));
-      u0 = __shfl_sync(0xffffffffu, u0, 0);
-      if (u0 >= qe) {
-        q = next_queue(ctr, q, nq, U, lane);
-        if (q < 0) break;
+      const int qb = static_cast<int>((static_cast<int64_t>(U) * qi) / nq);
+      const int qe = static_cast<int>((static_cast<int64_t>(U) * (qi + 1)) / nq);
+      const int u = qb + __shfl_sync(0xffffffffu, claim, 0);
+      if (u >= qe) {
+        qi = next_queue(ctr, qi, nq, U, lane);
+        if (qi < 0) break;
+        if (lane == 0) claim = static_cast<int>(atomicAdd(ctr + qi * kQueueStride, 1u));
         continue;
       }
-      // Group grp takes units u0 + grp, u0 + grp + G, ... of the claim.
-      for (int u = u0 + grp; u < u0 + kPprClaim && u < qe; u += G) {
-        const int4 un = a.units[u];
-        const int v = un.x;
-        const int64_t vb = a.off[v], ve = a.off[v + 1];
-        const int64_t b = vb + static_cast<int64_t>(un.y) * kPprChunk;
-        const int64_t e = ve < b + kPprChunk ? ve : b + kPprChunk;
-        float2 acc = make_float2(0.f, 0.f);
-        for (int64_t k0 = b; k0 < e; k0 += L) {
-          const int n = e - k0 < L ? static_cast<int>(e - k0) : L;
-          const int32_t mine = gl < n ? __ldcs(a.col + k0 + gl) : 0;
-          int j = 0;
-          for (; j + 8 <= n; j += 8) {
+      if (lane == 0) claim = static_cast<int>(atomicAdd(ctr + qi * kQueueStride, 1u));
+      if (u < first_tile) {
+        // ---- a chunk per group ----
+        const int h = u * G + q.grp;
+        if (h < a.n_chunks) {
+          const int4 un = a.chunks[h];
+          const int64_t vb = a.off[un.x], ve = a.off[un.x + 1];
+          const int64_t b = vb + static_cast<int64_t>(un.y) * kPprChunk;
+          const int lo = static_cast<int>(b & 3), hi = lo + static_cast<int>(ve - b < kPprChunk ? ve - b : kPprChunk);
+          const int32_t* p = a.col + (b & ~3ll);
+          float2 acc = make_float2(0.f, 0.f);
+          int32_t c[8];
+          q.ids(c, p, 0, hi);
+          for (int k = 0; k < hi; k += 8) {
             float2 x[8];
+            q.rows(x, c, rs_in, k, lo, hi);
+            q.ids(c, p, k + 8, hi);
 #pragma unroll
-            for (int t = 0; t < 8; ++t) {
-              const int32_t s = __shfl_sync(gmask, mine, j + t, L);
-              x[t] = __ldg(reinterpret_cast<const float2*>(rs_in + static_cast<size_t>(s) * W) + gl);
-            }
-#pragma unroll
-            for (int t = 0; t < 8; ++t) {
+            for (int t = 0; t < 8; ++t) {  // places outside hold 0
               acc.x += x[t].x;
               acc.y += x[t].y;
             }
           }
-          for (; j < n; ++j) {
-            const int32_t s = __shfl_sync(gmask, mine, j, L);
-            const float2 x = __ldg(reinterpret_cast<const float2*>(rs_in + static_cast<size_t>(s) * W) + gl);
-            acc.x += x.x;
-            acc.y += x.y;
-          }
-        }
-        if (un.z == 1) {
-          ppr_finish<W>(a, rs_out, r_out, v, acc, gl);
-        } else {
-          float2* part = reinterpret_cast<float2*>(a.partial + static_cast<size_t>(un.w + un.y) * W);
-          part[gl] = acc;
+          reinterpret_cast<float2*>(a.partial + static_cast<size_t>(un.w + un.y) * W)[q.gl] = acc;
           __threadfence();
-          __syncwarp(gmask);
+          __syncwarp(q.mask);
           unsigned t = 0;
-          if (gl == 0) t = atomicAdd(a.ticket + un.w, 1u);
-          t = __shfl_sync(gmask, t, 0, L);
+          if (q.gl == 0) t = atomicAdd(a.ticket + un.w, 1u);
+          t = __shfl_sync(q.mask, t, 0, L);
           if (t == static_cast<unsigned>(un.z) - 1) {
             __threadfence();
             float2 tot = make_float2(0.f, 0.f);
-            for (int c = 0; c < un.z; ++c) {
-              const volatile float* pp = a.partial + static_cast<size_t>(un.w + c) * W + 2 * gl;
-              tot.x += pp[0];
-              tot.y += pp[1];
+#pragma unroll 8
+            for (int i = 0; i < un.z; ++i) {
+              const float2 y =
+                  __ldcg(reinterpret_cast<const float2*>(a.partial + static_cast<size_t>(un.w + i) * W) + q.gl);
+              tot.x += y.x;
+              tot.y += y.y;
             }
-            ppr_finish<W>(a, rs_out, r_out, v, tot, gl);
-            if (gl == 0) a.ticket[un.w] = 0;
+            q.finish(a, rs_out, last, un.x, a.outdeg[un.x], tot);
+            if (q.gl == 0) a.ticket[un.w] = 0;
           }
         }
+        __syncwarp();
+        continue;
+      }
+      // ---- a tile: each group its share of the vertices, one per lane ----
+      const int2 tile = a.tiles[u - first_tile];
+      if (tile.x < 0) continue;
+      const int n = tile.y - tile.x, per = (n + G - 1) / G;
+      const int v0 = tile.x + q.grp * per;
+      const int cnt = min(per, tile.y - v0);  // may be negative: no vertex left
+      int64_t vb = 0, ve = 0;
+      int32_t od = 0;
+      if (q.gl < cnt) {
+        vb = a.off[v0 + q.gl];
+        ve = a.off[v0 + q.gl + 1];
+        od = a.outdeg[v0 + q.gl];
+      }
+      const unsigned heavy = __ballot_sync(q.mask, ve - vb > kPprHeavy) >> (q.grp * L);
+      for (int j = 0; j < cnt;) {
+        if ((heavy >> j) & 1u) {
+          ++j;
+          continue;
+        }
+        // A run of vertices up to the next heavy one: its edges are one stream.
+        const unsigned rest = heavy >> j;
+        const int jn = rest ? j + __ffs(rest) - 1 : cnt;
+        const int64_t base = __shfl_sync(q.mask, vb, j, L) & ~3ll;
+        const int lo = static_cast<int>(__shfl_sync(q.mask, vb, j, L) - base);
+        const int hi = static_cast<int>(__shfl_sync(q.mask, ve, jn - 1, L) - base);
+        const int my_end = static_cast<int>(ve - base);  // of the lane's vertex, when it is in the run
+        const int32_t* p = a.col + base;
+        int end = __shfl_sync(q.mask, my_end, j, L);
+        float2 acc = make_float2(0.f, 0.f);
+        int32_t c[8];
+        q.ids(c, p, 0, hi);
+        auto flush = [&]() {
+          q.finish(a, rs_out, last, v0 + j, __shfl_sync(q.mask, od, j, L), acc);
+          acc = make_float2(0.f, 0.f);
+          ++j;
+          end = __shfl_sync(q.mask, my_end, j < jn ? j : jn - 1, L);
+        };
+        for (int k = 0; k < hi; k += 8) {
+          float2 x[8];
+          q.rows(x, c, rs_in, k, lo, hi);
+          q.ids(c, p, k + 8, hi);
+#pragma unroll
+          for (int t = 0; t < 8; ++t) {
+            if (k + t < hi) {
+              while (k + t >= end) flush();
+              acc.x += x[t].x;
+              acc.y += x[t].y;
+            }
+          }
+        }
+        while (j < jn) flush();
       }
       __syncwarp();
     }
     if (!ppr_grid_barrier(a, it)) return;
+  }
+}
+
+// out[v][0, k) = in[perm ? perm[v] : v][0, k) of rows of W columns: the rows
+// as the caller numbers them, without the columns past k.
+__global__ void ppr_rows_kernel(const float* __restrict__ in, const int32_t* __restrict__ perm, int32_t V, int k, int W,
+                                float* __restrict__ out) {
+  const int64_t n = static_cast<int64_t>(V) * k, stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
+    const int32_t v = static_cast<int32_t>(i / k), j = static_cast<int32_t>(i % k);
+    out[i] = in[static_cast<size_t>(perm ? perm[v] : v) * W + j];
   }
 }
 
@@ -214,55 +314,60 @@ extern "C" gx_status gx_ppr(gx_engine* e, int32_t k, const int32_t* sources, int
   GX_CUDA(cudaSetDevice(e->dev));
   cudaStream_t s = e->s_comp;
   const int W = k <= 8 ? 8 : k <= 16 ? 16 : k <= 32 ? 32 : 64;
-  // Units: one per vertex, heavy vertices in chunks.
-  std::vector<int4> units;
-  units.reserve(static_cast<size_t>(V) + 1024);
-  int32_t n_part = 0;
-  for (int32_t v = 0; v < V; ++v) {
-    const int64_t d = e->off[v + 1] - e->off[v];
-    const int32_t nch = d > kPprChunk ? static_cast<int32_t>((d + kPprChunk - 1) / kPprChunk) : 1;
-    for (int32_t c = 0; c < nch; ++c) units.push_back(make_int4(v, c, nch, nch > 1 ? n_part : 0));
-    if (nch > 1) n_part += nch;
-  }
   const size_t rows = static_cast<size_t>(V) * W;
   const size_t steps = static_cast<size_t>(std::max(iters, 1));
-  float *rs0 = nullptr, *rs1 = nullptr, *r = nullptr, *partial = nullptr;
-  int4* d_units = nullptr;
-  int32_t* d_src = nullptr;
-  unsigned int *ctr = nullptr, *ticket = nullptr, *arrive = nullptr, *abort_flag = nullptr;
-  struct Guard {
-    std::vector<void*> p;
-    ~Guard() {
-      for (void* x : p) gx::pool_free(x);
-    }
-  } guard;
-  gx_status st = GX_OK;
-  if ((st = dev_alloc(&rs0, rows)) != GX_OK) return st;
-  guard.p.push_back(rs0);
-  if ((st = dev_alloc(&rs1, rows)) != GX_OK) return st;
-  guard.p.push_back(rs1);
-  if ((st = dev_alloc(&r, rows)) != GX_OK) return st;
-  guard.p.push_back(r);
-  if ((st = dev_alloc(&partial, static_cast<size_t>(std::max(n_part, 1)) * W)) != GX_OK) return st;
-  guard.p.push_back(partial);
-  if ((st = dev_alloc(&d_units, units.size())) != GX_OK) return st;
-  guard.p.push_back(d_units);
-  if ((st = dev_alloc(&d_src, kPprMaxCols)) != GX_OK) return st;
-  guard.p.push_back(d_src);
-  if ((st = dev_alloc(&ctr, static_cast<size_t>(kQueues) * kQueueStride * steps)) != GX_OK) return st;
-  guard.p.push_back(ctr);
-  if ((st = dev_alloc(&ticket, static_cast<size_t>(std::max(n_part, 1)))) != GX_OK) return st;
-  guard.p.push_back(ticket);
-  if ((st = dev_alloc(&arrive, steps)) != GX_OK) return st;
-  guard.p.push_back(arrive);
-  if ((st = dev_alloc(&abort_flag, 1)) != GX_OK) return st;
-  guard.p.push_back(abort_flag);
-
+  const int32_t n_tiles = static_cast<int32_t>(e->units.size());
   int32_t h_src[kPprMaxCols];
   for (int j = 0; j < kPprMaxCols; ++j) h_src[j] = j < k ? (e->relabeled ? e->h_perm[sources[j]] : sources[j]) : -1;
-  GX_CUDA(cudaMemcpyAsync(d_units, units.data(), sizeof(int4) * units.size(), cudaMemcpyHostToDevice, s));
+  // One block for everything of a known size: rows, cursors, flags.
+  struct Guard {
+    unsigned char *block = nullptr, *chunk_block = nullptr;
+    ~Guard() {
+      dev_free(&block);
+      dev_free(&chunk_block);
+    }
+  } guard;
+  size_t at = 0;
+  auto place = [&](size_t bytes) {
+    const size_t x = at;
+    at += (bytes + 255) & ~size_t(255);
+    return x;
+  };
+  const size_t o_rs0 = place(rows * sizeof(float)), o_rs1 = place(rows * sizeof(float)), o_r = place(rows * sizeof(float));
+  const size_t o_src = place(sizeof(h_src));
+  const size_t o_zero = at;  // cleared by the graph, in one piece
+  const size_t o_ctr = place(sizeof(unsigned int) * kQueues * kQueueStride * steps);
+  const size_t o_arrive = place(sizeof(unsigned int) * steps), o_abort = place(sizeof(unsigned int));
+  const size_t zero_bytes = at - o_zero;
+  const size_t o_count = place(2 * sizeof(unsigned int));
+  GX_TRY(dev_alloc(&guard.block, at));
+  float* rs0 = reinterpret_cast<float*>(guard.block + o_rs0);
+  float* rs1 = reinterpret_cast<float*>(guard.block + o_rs1);
+  float* r = reinterpret_cast<float*>(guard.block + o_r);
+  int32_t* d_src = reinterpret_cast<int32_t*>(guard.block + o_src);
+  unsigned int* abort_flag = reinterpret_cast<unsigned int*>(guard.block + o_abort);
+  unsigned int* count = reinterpret_cast<unsigned int*>(guard.block + o_count);
   GX_CUDA(cudaMemcpyAsync(d_src, h_src, sizeof(h_src), cudaMemcpyHostToDevice, s));
-  GX_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned int) * std::max(n_part, 1), s));
+  // Chunks of the long lists: counted, then written with their tickets clear.
+  GX_CUDA(cudaMemsetAsync(count, 0, 2 * sizeof(unsigned int), s));
+  const int plan_grid = std::max(1, std::min(e->n_sm * 4, (V + 255) / 256));
+  ppr_chunks_kernel<<<plan_grid, 256, 0, s>>>(e->d_off, V, nullptr, count);
+  GX_CUDA(cudaGetLastError());
+  unsigned int n_chunks = 0;
+  GX_CUDA(cudaMemcpyAsync(&n_chunks, count, sizeof(n_chunks), cudaMemcpyDeviceToHost, s));
+  GX_CUDA(cudaStreamSynchronize(s));
+  const size_t nc = std::max<size_t>(n_chunks, 1);
+  at = 0;
+  const size_t o_chunks = place(nc * sizeof(int4)), o_partial = place(nc * W * sizeof(float)),
+               o_ticket = place(nc * sizeof(unsigned int));
+  GX_TRY(dev_alloc(&guard.chunk_block, at));
+  int4* chunks = reinterpret_cast<int4*>(guard.chunk_block + o_chunks);
+  unsigned int* ticket = reinterpret_cast<unsigned int*>(guard.chunk_block + o_ticket);
+  if (n_chunks) {
+    GX_CUDA(cudaMemsetAsync(ticket, 0, nc * sizeof(unsigned int), s));
+    ppr_chunks_kernel<<<plan_grid, 256, 0, s>>>(e->d_off, V, chunks, count + 1);
+    GX_CUDA(cudaGetLastError());
+  }
 
   PprArgs a{};
   a.off = e->d_off;
@@ -271,14 +376,16 @@ extern "C" gx_status gx_ppr(gx_engine* e, int32_t k, const int32_t* sources, int
   a.rs[0] = rs0;
   a.rs[1] = rs1;
   a.r_out = r;
-  a.units = d_units;
-  a.n_units = static_cast<int32_t>(units.size());
+  a.tiles = e->d_units;
+  a.chunks = chunks;
+  a.n_tiles = n_tiles;
+  a.n_chunks = static_cast<int32_t>(n_chunks);
   a.iters = iters;
-  a.ctr = ctr;
-  a.arrive = arrive;
+  a.ctr = reinterpret_cast<unsigned int*>(guard.block + o_ctr);
+  a.arrive = reinterpret_cast<unsigned int*>(guard.block + o_arrive);
   a.abort = abort_flag;
   a.wait_limit = e->cfg.wait_limit;
-  a.partial = partial;
+  a.partial = reinterpret_cast<float*>(guard.chunk_block + o_partial);
   a.ticket = ticket;
   a.src = d_src;
   a.alpha = static_cast<float>(1.0 - restart);
@@ -287,8 +394,11 @@ extern "C" gx_status gx_ppr(gx_engine* e, int32_t k, const int32_t* sources, int
                                                                                            : ppr_kernel_for<64>();
   int per_sm = 0;
   GX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kPprThreads, 0));
-  // Co-resident CTAs only: the grid barrier waits for every one of them.
-  const int grid = std::max(1, per_sm) * e->n_sm;
+  // Co-resident CTAs only: the grid barrier waits for every one of them.  No
+  // more than have a unit per warp: each one more is an arrival every step.
+  const int64_t n_units = static_cast<int64_t>(n_tiles) + n_chunks;
+  const int grid = static_cast<int>(std::max<int64_t>(
+      1, std::min<int64_t>(std::max(1, per_sm) * e->n_sm, (n_units + kPprWarps - 1) / kPprWarps)));
   cudaLaunchConfig_t lc{};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -303,9 +413,7 @@ extern "C" gx_status gx_ppr(gx_engine* e, int32_t k, const int32_t* sources, int
   // The step's resets, R0 = S and the persistent launch, as one graph.
   auto enqueue = [&]() -> cudaError_t {
     cudaError_t err = cudaMemsetAsync(rs0, 0, rows * sizeof(float), s);
-    if (err == cudaSuccess) err = cudaMemsetAsync(ctr, 0, sizeof(unsigned int) * kQueues * kQueueStride * steps, s);
-    if (err == cudaSuccess) err = cudaMemsetAsync(arrive, 0, sizeof(unsigned int) * steps, s);
-    if (err == cudaSuccess) err = cudaMemsetAsync(abort_flag, 0, sizeof(unsigned int), s);
+    if (err == cudaSuccess) err = cudaMemsetAsync(guard.block + o_zero, 0, zero_bytes, s);
     if (err != cudaSuccess) return err;
     ppr_init_kernel<<<1, kPprMaxCols, 0, s>>>(rs0, e->d_outdeg, d_src, k, W);
     err = cudaGetLastError();
@@ -344,19 +452,17 @@ extern "C" gx_status gx_ppr(gx_engine* e, int32_t k, const int32_t* sources, int
     if (iters == 0) {
       memset(host_out, 0, sizeof(float) * static_cast<size_t>(V) * k);
       for (int j = 0; j < k; ++j) host_out[static_cast<size_t>(sources[j]) * k + j] = 1.f;
-    } else if (!e->relabeled) {
-      GX_CUDA(cudaMemcpy2D(host_out, sizeof(float) * k, r, sizeof(float) * W, sizeof(float) * k, V,
-                           cudaMemcpyDeviceToHost));
     } else {
-      // Rows in the engine's numbering: row v of the result is row perm[v].
-      std::vector<float> rows(static_cast<size_t>(V) * k);
-      GX_CUDA(cudaMemcpy2D(rows.data(), sizeof(float) * k, r, sizeof(float) * W, sizeof(float) * k, V,
-                           cudaMemcpyDeviceToHost));
-      const int32_t* perm = e->h_perm.data();
-#pragma omp parallel for schedule(static)
-      for (int32_t v = 0; v < V; ++v)
-        memcpy(host_out + static_cast<size_t>(v) * k, rows.data() + static_cast<size_t>(perm[v]) * k,
-               sizeof(float) * k);
+      // The caller's rows of k columns, put together on the device (rs0 is
+      // free by now) and copied in one piece.
+      const size_t bytes = sizeof(float) * static_cast<size_t>(V) * k;
+      if (e->relabeled || k != W) {
+        ppr_rows_kernel<<<e->n_sm * 8, 256, 0, s>>>(r, e->relabeled ? e->d_perm : nullptr, V, k, W, rs0);
+        GX_CUDA(cudaGetLastError());
+        GX_CUDA(cudaStreamSynchronize(s));
+        r = rs0;
+      }
+      GX_TRY(copy_to_host(e, host_out, r, bytes));
     }
   }
   if (stats) {
