@@ -3,29 +3,29 @@
 // directions, no self-loops).  No reference counterpart: the reference's
 // only "tc" (GraphH/list/system/GraphPS.h:15-95) counts reciprocal edges.
 //
-//  1. orient u -> v iff (deg u, u) < (deg v, v) (a DAG; every triangle has
-//     exactly one vertex whose two out-neighbours close it);
-//  2. build the oriented adjacency N+(u) with warp-ballot compaction, which
-//     keeps the ascending id order of the input lists;
-//  3. count sum over u, v in N+(u) of |N+(u) ∩ N+(v)|: a warp stages N+(u)
-//     in shared memory with an 8192-bit filter of its ids; its lanes test
-//     every w of N+(v) against the filter, and only the ids that pass are
-//     queued and binary-searched in the staged list, 32 at a time.
-//     Vertices are claimed in descending |N+(u)| order; lists too long for
-//     a warp's slice get a whole CTA (a 2^16-bit filter, warps splitting
-//     N+(u)), whose shared memory is sized to the longest such list so it
-//     runs beside the warp kernel; the rare list beyond kCtaList entries is
-//     searched in place in global memory.
-// Counts are exact (64-bit integer sums).
+//  1. orient u -> v iff (deg u, u) < (deg v, v): a DAG, in which every
+//     triangle has exactly one edge {u, v} whose ends share its third vertex
+//     as out-neighbour;
+//  2. write N+(v) in the room its CSC list leaves (no order is needed below,
+//     so no count pass or scan comes first), padded to whole 16-byte pieces;
+//  3. count sum over edges {x, y} of |N+(x) n N+(y)|: the end with the longer
+//     N+ (x) is staged, the shorter list is scanned (half the probes of
+//     scanning N+(v) for every u -> v on R-MAT).  A vertex with much to scan
+//     gets a CTA that stages N+(x) as a bitmap over the vertices in shared
+//     memory: a probe is one word's load and a shift, exact, and a warp reads
+//     128 entries of a scanned list at once.  The others get a warp with a
+//     small hash table of N+(x).
+// A bitmap holds tc_bits vertices.  A larger graph is renumbered by (degree,
+// id), and the bitmap stands for the highest ranks: N+ of a vertex among them
+// lies wholly among them, and a vertex below them is left to the warps.
+// Counts are exact (64-bit integer sums).  Symmetric R-MAT of scale 20 (4.4 G
+// probes of N+(v), 2.0 G of the shorter lists): 18.7 ms with a filter and
+// binary searches of N+(u) for every N+(v), 3.0 this way; issue-bound at about
+// 15 instructions a probe of a warp's 32; scale 24: 300 -> 86 ms.
 #include <cuda_runtime.h>
-#include <omp.h>
 
 #include <algorithm>
-#include <chrono>
-#include <cstring>
 #include <memory>
-#include <numeric>
-#include <vector>
 
 #include "gx_engine.h"
 #include "gx_nvtx.h"
@@ -34,315 +34,392 @@ using namespace gx;
 
 namespace {
 
-constexpr int kTcThreads = 256;
+constexpr int kTcThreads = 256;             // warp kernels
 constexpr int kTcWarps = kTcThreads / 32;
-constexpr int kWarpList = 1024;             // N+(u) entries staged per warp
-constexpr int kCtaList = 48 * 1024;         // entries staged per CTA (192 KB)
+// Vertices of a bitmap.  Small bitmaps leave an SM several CTAs, whose waits
+// at a vertex's end overlap, large ones leave fewer vertices to the warps:
+// symmetric R-MAT of 1 M vertices 3.0 ms with 2^18, 3.6 with 2^19, 4.9 with
+// all; 4 M 15.5, 17.7 with 2^19; 16 M 91, 86 with 2^19, 103 with 10^6.
+constexpr int64_t kTcBitsLeast = 1 << 18, kTcBitsMost = 1800000;  // 32 and 225 KB
+inline int64_t tc_bits(int64_t V) {
+  return std::min(V, std::max(kTcBitsLeast, std::min(V / 32, kTcBitsMost)));
+}
 constexpr int kTcGrab = 4;                  // vertices a warp claims per atomic
+// |N+| x degree, a bound of the probes, from which a vertex gets a CTA: 131,072
+// vertices 0.37 ms from 2048 to 8192, 0.61 at 16384, 3.1 at 65536 (a warp each
+// for hubs); 1 M vertices 3.0 from 2048 to 8192, 3.3 at 1024, 3.7 at 16384.
+constexpr int64_t kTcCtaWork = 4096;
+constexpr int64_t kTcCtaFirst = 1 << 21;    // ... and from which it is counted before the others
+constexpr int kTcPiece = 512;               // entries of a warp's hash table at a time
+constexpr int kTcSlots = 2048;
+constexpr int32_t kTcNone = -1;             // no vertex: padding, and an empty slot
 
-__global__ void tc_degree_kernel(const int64_t* off, int32_t V, int32_t* deg) {
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x)
-    deg[v] = static_cast<int32_t>(off[v + 1] - off[v]);
+// What a scan needs of a vertex: its N+.
+struct __align__(16) TcInfo {
+  int64_t start;  // in dcol, a multiple of 4
+  int32_t n;
+  int32_t pad;
+};
+
+struct TcArgs {
+  const int64_t* off;
+  const int32_t* col;
+  const int2* units;        // the engine's work units and heavy vertices
+  const int4* heavy;
+  int32_t n_units, chunk, heavy_deg, V;
+  const int32_t* deg;
+  const int32_t* rank;      // ranked graphs: position by (degree, id), else null
+  int32_t* n;               // |N+|
+  int32_t* dcol;            // N+ lists (ids, or ranks)
+  TcInfo* info;
+  int32_t base, bits;       // the bitmap stands for [base, base + bits)
+  uint32_t mix, mask;       // unranked: the number dcol holds for an id (tc_mixed)
+  int32_t *big, *small;     // vertices for CTAs and for warps; the CTAs' heaviest from big[V] down
+  unsigned int* ctr;        // claimed: units; listed: big, small, heaviest; claimed: big, small
+  unsigned long long* out;  // triangles, probes
+};
+
+__global__ void tc_degree_kernel(const int64_t* off, int32_t V, int32_t* deg, int32_t* n, unsigned long long* keys,
+                                 int vb) {
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
+    const int32_t d = static_cast<int32_t>(off[v + 1] - off[v]);
+    deg[v] = d;
+    n[v] = 0;
+    if (keys) keys[v] = static_cast<unsigned long long>(d) << vb | static_cast<unsigned long long>(v);
+  }
 }
 
-__device__ __forceinline__ bool tc_before(int32_t du, int32_t u, int32_t dv, int32_t v) {
-  return du < dv || (du == dv && u < v);
+__global__ void tc_rank_kernel(const unsigned long long* sorted, unsigned long long vmask, int32_t V, int32_t* rank) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < V; i += gridDim.x * blockDim.x)
+    rank[sorted[i] & vmask] = i;
 }
 
-// Warp per vertex u.  Its list is read 8 chunks of 32 at a time, all ids
-// and their degrees loaded before any is used, so a hub's long list costs
-// one dependent load chain per 256 entries, not per 32 (the hubs set the
-// kernels' length).  Self-loops never qualify: u is not before itself.
-constexpr int kOrientChunks = 8;
+// The number that stands for vertex y in N+: its rank, or its id mixed within
+// [0, V), by an odd factor modulo the next power of two until it lies there.
+// (As they are, R-MAT's hot ids, of few set bits, fall into few banks of the
+// bitmap: 12.5 wavefronts a load of 32 words, mixed 4.)
+__device__ __forceinline__ int32_t tc_mixed(const TcArgs& a, int32_t y) {
+  uint32_t x = static_cast<uint32_t>(y);
+  do {
+    x = (x * a.mix) & a.mask;
+  } while (x >= static_cast<uint32_t>(a.V));
+  return static_cast<int32_t>(x);
+}
 
-// The oriented graph is built in the caller's numbering: on an engine that
-// renumbered its vertices (inv non-null: engine vertex u is the caller's
-// inv[u]) the ids are mapped back while the lists are read, so N+ keeps the
-// input's ascending id order and the counting kernels below index by the
-// caller's ids.  deg stays in the engine's numbering.
+// Where N+(v) begins: at least as much room as its list, whole 16-byte pieces.
+__device__ __forceinline__ int64_t tc_start(int64_t off, int32_t v) { return (off + 4 * static_cast<int64_t>(v) + 3) & ~3ll; }
 
-// |N+(u)| per vertex.
-__global__ void tc_count_kernel(const int64_t* __restrict__ off, const int32_t* __restrict__ col,
-                                const int32_t* __restrict__ deg, const int32_t* __restrict__ inv, int32_t V,
-                                int32_t* __restrict__ cnt) {
+// The engine's units (tiles of at most 32 vertices, chunks of heavy ones), a
+// warp each: the unit's entries 128 at a time, every stage's loads in flight
+// together; an entry's vertex is found among the lanes' offsets, and the
+// entries kept for one vertex reserve their places with one atomic.
+// (A warp per vertex, with R-MAT's hubs, took 0.83 + 0.95 ms to count and fill
+// at symmetric scale 20.)
+__global__ void __launch_bounds__(kTcThreads) tc_fill_kernel(const __grid_constant__ TcArgs a) {
   const int lane = threadIdx.x & 31;
-  const int warps = gridDim.x * (blockDim.x >> 5);
-  for (int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < V; u += warps) {
-    const int32_t du = deg[u];
-    const int32_t uo = inv ? inv[u] : u;
-    const int64_t e1 = off[u + 1];
-    int c = 0;
-    for (int64_t base = off[u]; base < e1; base += 32 * kOrientChunks) {
-      int32_t v[kOrientChunks], dv[kOrientChunks];
+  for (;;) {
+    int t = 0;
+    if (lane == 0) t = static_cast<int>(atomicAdd(a.ctr, 1u));
+    t = __shfl_sync(0xffffffffu, t, 0);
+    if (t >= a.n_units) break;
+    const int2 u = a.units[t];
+    // The lane's vertex and its entries; a chunk is lane 0's.
+    int v = 0;
+    int64_t b = 0, e = 0;
+    if (u.x < 0) {
+      v = a.heavy[-u.x - 1].x;
+      b = a.off[v] + static_cast<int64_t>(u.y) * a.chunk;
+      e = min(a.off[v + 1], b + a.chunk);
+      if (lane > 0) b = e;
+    } else if (lane < u.y - u.x) {
+      v = u.x + lane;
+      b = a.off[v];
+      e = a.off[v + 1];
+      if (e - b > a.heavy_deg) e = b;  // its chunks' entries
+    }
+    const int len = static_cast<int>(e - b);
+    int pre = len;  // entries of the lanes before
 #pragma unroll
-      for (int j = 0; j < kOrientChunks; ++j) v[j] = base + 32 * j + lane < e1 ? col[base + 32 * j + lane] : 0;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, pre, o);
+      if (lane >= o) pre += x;
+    }
+    const int total = __shfl_sync(0xffffffffu, pre, 31);
+    pre -= len;
+    const int32_t dv = len > 0 ? (a.rank ? a.rank[v] : a.deg[v]) : 0;
+    const int64_t to = tc_start(a.off[v], v);
+    for (int k0 = 0; k0 < total; k0 += 128) {
+      int l[4], lo[4];
+      int32_t y[4], dy[4];
 #pragma unroll
-      for (int j = 0; j < kOrientChunks; ++j) dv[j] = base + 32 * j + lane < e1 ? deg[v[j]] : 0;
-      if (inv) {
+      for (int j = 0; j < 4; ++j) {
+        const int k = k0 + 32 * j + lane;
+        l[j] = 0;  // the last lane whose entries start at or before k (every lane takes part in every shuffle)
 #pragma unroll
-        for (int j = 0; j < kOrientChunks; ++j) v[j] = inv[v[j]];
+        for (int sp = 16; sp > 0; sp >>= 1) {
+          const int x = __shfl_sync(0xffffffffu, pre, l[j] + sp);
+          if (x <= k) l[j] += sp;
+        }
+        lo[j] = __shfl_sync(0xffffffffu, pre, l[j]);
+        const int64_t bl = __shfl_sync(0xffffffffu, b, l[j]);
+        y[j] = k < total ? __ldcs(a.col + bl + (k - lo[j])) : 0;
       }
 #pragma unroll
-      for (int j = 0; j < kOrientChunks; ++j) c += base + 32 * j + lane < e1 && tc_before(du, uo, dv[j], v[j]);
-    }
+      for (int j = 0; j < 4; ++j) dy[j] = a.rank ? a.rank[y[j]] : a.deg[y[j]];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    if (lane == 0) cnt[uo] = c;
+      for (int j = 0; j < 4; ++j) {
+        const int k = k0 + 32 * j + lane;
+        const int32_t x = __shfl_sync(0xffffffffu, v, l[j]), dx = __shfl_sync(0xffffffffu, dv, l[j]);
+        const int64_t tx = __shfl_sync(0xffffffffu, to, l[j]);
+        const int hi = lo[j] + __shfl_sync(0xffffffffu, len, l[j]);
+        const bool keep = k < total && (dx < dy[j] || (dx == dy[j] && x < y[j]));  // (ranks differ)
+        // Lanes first .. last - 1 hold this vertex's entries of the window.
+        const int w = k0 + 32 * j, first = max(lo[j] - w, 0), last = max(min(hi - w, 32), 0);
+        const unsigned mine = (last >= 32 ? 0xffffffffu : (1u << last) - 1u) & ~((1u << first) - 1u);
+        const unsigned m = __ballot_sync(0xffffffffu, keep) & mine;
+        int at = 0;
+        if (k < total && lane == first && m) at = atomicAdd(a.n + x, __popc(m));
+        at = __shfl_sync(0xffffffffu, at, first < 32 ? first : 0);
+        if (keep) a.dcol[tx + at + __popc(m & ((1u << lane) - 1u))] = a.rank ? dy[j] : tc_mixed(a, y[j]);
+      }
+    }
   }
 }
 
-// N+(u), in the input's ascending order: chunk by chunk, ballot + popc
-// compaction.
-__global__ void tc_fill_kernel(const int64_t* __restrict__ off, const int32_t* __restrict__ col,
-                               const int32_t* __restrict__ deg, const int32_t* __restrict__ inv, int32_t V,
-                               const int64_t* __restrict__ doff, int32_t* __restrict__ dcol) {
+// Padding, scan descriptors and the vertices to count from.
+__global__ void tc_list_kernel(const __grid_constant__ TcArgs a) {
   const int lane = threadIdx.x & 31;
-  const unsigned below = (1u << lane) - 1u;
-  const int warps = gridDim.x * (blockDim.x >> 5);
-  for (int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < V; u += warps) {
-    const int32_t du = deg[u];
-    const int32_t uo = inv ? inv[u] : u;
-    int64_t pos = doff[uo];
-    const int64_t e1 = off[u + 1];
-    for (int64_t base = off[u]; base < e1; base += 32 * kOrientChunks) {
-      int32_t v[kOrientChunks], dv[kOrientChunks];
-#pragma unroll
-      for (int j = 0; j < kOrientChunks; ++j) v[j] = base + 32 * j + lane < e1 ? col[base + 32 * j + lane] : 0;
-#pragma unroll
-      for (int j = 0; j < kOrientChunks; ++j) dv[j] = base + 32 * j + lane < e1 ? deg[v[j]] : 0;
-      if (inv) {
-#pragma unroll
-        for (int j = 0; j < kOrientChunks; ++j) v[j] = inv[v[j]];
-      }
-#pragma unroll
-      for (int j = 0; j < kOrientChunks; ++j) {
-        const bool keep = base + 32 * j + lane < e1 && tc_before(du, uo, dv[j], v[j]);
-        const unsigned m = __ballot_sync(0xffffffffu, keep);
-        if (keep) dcol[pos + __popc(m & below)] = v[j];
-        pos += __popc(m);
+  for (int v0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); v0 < a.V; v0 += gridDim.x * blockDim.x) {
+    const int v = v0 + lane;
+    bool big = false, small = false;
+    if (v < a.V) {
+      TcInfo x{tc_start(a.off[v], v), a.n[v], 0};
+      a.info[v] = x;
+      for (int k = x.n; k & 3; ++k) a.dcol[x.start + k] = kTcNone;
+      const bool in = !a.rank || a.rank[v] >= a.base;
+      big = in && static_cast<int64_t>(x.n) * a.deg[v] >= kTcCtaWork;
+      small = !big && x.n > 0;
+      if (big && static_cast<int64_t>(x.n) * a.deg[v] >= kTcCtaFirst) {
+        a.big[a.V - 1 - static_cast<int>(atomicAdd(a.ctr + 3, 1u))] = v;
+        big = false;
       }
     }
+    const unsigned mb = __ballot_sync(0xffffffffu, big), ms = __ballot_sync(0xffffffffu, small);
+    unsigned nb = 0, ns = 0;
+    if (lane == 0 && mb) nb = atomicAdd(a.ctr + 1, static_cast<unsigned>(__popc(mb)));
+    if (lane == 0 && ms) ns = atomicAdd(a.ctr + 2, static_cast<unsigned>(__popc(ms)));
+    nb = __shfl_sync(0xffffffffu, nb, 0);
+    ns = __shfl_sync(0xffffffffu, ns, 0);
+    const unsigned below = (1u << lane) - 1u;
+    if (big) a.big[nb + __popc(mb & below)] = v;
+    if (small) a.small[ns + __popc(ms & below)] = v;
   }
 }
 
-__device__ __forceinline__ bool tc_search(const int32_t* list, int n, int32_t w) {
-  int lo = 0, hi = n;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (list[mid] < w) lo = mid + 1;
-    else hi = mid;
+// Whether the edge {x, y} is counted with x staged: y's list is the shorter.
+__device__ __forceinline__ bool tc_scans(int32_t nx, int32_t x, int32_t ny, int32_t y) {
+  return ny > 0 && (ny < nx || (ny == nx && y < x));
+}
+
+template <int NT>
+__device__ __forceinline__ void tc_flush(unsigned long long cnt, unsigned long long work, unsigned long long* out) {
+  __shared__ unsigned long long s_red[2][NT / 32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+    work += __shfl_xor_sync(0xffffffffu, work, o);
   }
-  return lo < n && list[lo] == w;
-}
-
-// Bit filter of a staged list: bit h(w) is set for every w of the list, so a
-// clear bit proves w absent.  Multiplicative hashing spreads R-MAT's
-// structured ids over the 2^kFilterBits bits.
-constexpr int kFilterBits = 13;                          // a warp's list (<= 1024 ids)
-constexpr int kFilterWords = (1 << kFilterBits) / 32;
-constexpr int kCtaFilterBits = 16;                       // a CTA's list (> 1024 ids)
-constexpr int kCtaFilterWords = (1 << kCtaFilterBits) / 32;
-template <int BITS>
-__device__ __forceinline__ uint32_t tc_hash(int32_t w) {
-  return (static_cast<uint32_t>(w) * 2654435761u) >> (32 - BITS);
-}
-
-// Lanes of one warp test every w of N+(v) against the staged list's bit
-// filter.  Most probes miss (about 90% on R-MAT) and the filter rejects all
-// but 1-2% of those with one shared-memory load; the ids that pass are
-// appended to the warp's queue (ballot + prefix) and binary-searched 32 at a
-// time, so the searches run with every lane busy.  Two rounds of 32 ids go
-// through per loop step, each round's ids loaded a step ahead so the loads'
-// latency overlaps the filter tests.  qn (warp-uniform) is the queue's fill:
-// below 32 between steps, at most 95 after a step's appends (kQueue slots).
-// N+(v) lies at dcol[vb, vb + len).
-constexpr int kQueue = 96;
-template <int BITS>
-__device__ __forceinline__ void tc_probe_filtered(const int32_t* __restrict__ dcol, int64_t vb, int len,
-                                                  const int32_t* list, int n, const uint32_t* bits, int32_t* q,
-                                                  int& qn, int lane, unsigned long long& cnt,
-                                                  unsigned long long& work) {
-  const int32_t* nv = dcol + vb;
-  if (lane == 0) work += static_cast<unsigned long long>(len);
-  const unsigned below = (1u << lane) - 1u;
-  int32_t n0 = lane < len ? nv[lane] : 0, n1 = lane + 32 < len ? nv[lane + 32] : 0;
-  for (int base = 0; base < len; base += 64) {
-    const int j0 = base + lane, j1 = j0 + 32;
-    const int32_t w0 = n0, w1 = n1;
-    if (j0 + 64 < len) n0 = nv[j0 + 64];
-    if (j1 + 64 < len) n1 = nv[j1 + 64];
-    bool p0 = false, p1 = false;
-    if (j0 < len) {
-      const uint32_t h = tc_hash<BITS>(w0);
-      p0 = (bits[h >> 5] >> (h & 31)) & 1u;
-    }
-    if (j1 < len) {
-      const uint32_t h = tc_hash<BITS>(w1);
-      p1 = (bits[h >> 5] >> (h & 31)) & 1u;
-    }
-    const unsigned m0 = __ballot_sync(0xffffffffu, p0), m1 = __ballot_sync(0xffffffffu, p1);
-    if (p0) q[qn + __popc(m0 & below)] = w0;
-    qn += __popc(m0);
-    if (p1) q[qn + __popc(m1 & below)] = w1;
-    qn += __popc(m1);
-    while (qn >= 32) {
-      __syncwarp();
-      cnt += tc_search(list, n, q[lane]);
-      __syncwarp();
-      for (int i = lane; i < qn - 32; i += 32) q[i] = q[32 + i];
-      qn -= 32;
-    }
+  if ((threadIdx.x & 31) == 0) {
+    s_red[0][threadIdx.x >> 5] = cnt;
+    s_red[1][threadIdx.x >> 5] = work;
   }
-  __syncwarp();
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    unsigned long long t = 0;
+    for (int w = 0; w < NT / 32; ++w) t += s_red[threadIdx.x][w];
+    if (t) atomicAdd(out + threadIdx.x, t);
+  }
 }
 
-// Warp per vertex; vertices in `order` (descending |N+|) with |N+| <= kWarpList.
-__global__ void __launch_bounds__(kTcThreads) tc_warp_kernel(const int64_t* doff, const int32_t* dcol,
-                                                             const int32_t* order, int32_t n_order, unsigned int* ctr,
-                                                             unsigned long long* out) {
-  __shared__ int32_t s_list[kTcWarps][kWarpList];
-  __shared__ uint32_t s_bits[kTcWarps][kFilterWords];
-  __shared__ int32_t s_q[kTcWarps][kQueue];
-  __shared__ unsigned long long s_red[2][kTcWarps];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int32_t* list = s_list[wid];
-  uint32_t* bits = s_bits[wid];
-  int32_t* q = s_q[wid];
+// CTA per vertex of a.big: N+(x) as a bitmap; its warps claim 32 of x's
+// neighbours at a time, and each half of a warp reads kTcAhead of their lists
+// at once, 64 entries of each.
+constexpr int kTcAhead = 4;
+template <int NT>
+__global__ void __launch_bounds__(NT, 2048 / NT / 2) tc_cta_kernel(const __grid_constant__ TcArgs a) {
+  extern __shared__ __align__(16) uint32_t s_bits[];
+  __shared__ int s_i, s_next;
+  const int lane = threadIdx.x & 31;
+  const int n_first = static_cast<int>(a.ctr[3]), n_big = n_first + static_cast<int>(a.ctr[1]);
+  for (int i = threadIdx.x; i <= a.bits / 32; i += NT) s_bits[i] = 0u;
+  unsigned long long cnt = 0, work = 0;
+  for (;;) {
+    if (threadIdx.x == 0) {
+      s_i = static_cast<int>(atomicAdd(a.ctr + 4, 1u));
+      s_next = 0;
+    }
+    __syncthreads();
+    if (s_i >= n_big) break;
+    const int32_t x = a.big[s_i < n_first ? a.V - 1 - s_i : s_i - n_first];
+    const TcInfo ix = a.info[x];
+    for (int k = threadIdx.x; k < ix.n; k += NT) {
+      const uint32_t r = static_cast<uint32_t>(a.dcol[ix.start + k] - a.base);
+      atomicOr(&s_bits[r >> 5], 1u << (r & 31));
+    }
+    const int64_t b = a.off[x];
+    const int deg = static_cast<int>(a.off[x + 1] - b);
+    // Neighbours a warp claims at once: at least two claims for every warp.
+    const int grab = max(1, min(32, deg / (2 * (NT / 32))));
+    __syncthreads();
+    unsigned found = 0;
+    for (;;) {
+      int g = 0;
+      if (lane == 0) g = atomicAdd(&s_next, grab);
+      g = __shfl_sync(0xffffffffu, g, 0);
+      if (g >= deg) break;
+      TcInfo iy{0, 0, 0};
+      bool take = false;
+      if (lane < grab && g + lane < deg) {
+        const int32_t y = a.col[b + g + lane];
+        iy = a.info[y];
+        take = tc_scans(ix.n, x, iy.n, y);
+        if (take) work += static_cast<unsigned>(iy.n);
+      }
+      // Places outside the bitmap (padding, lower ranks) read its last bit,
+      // which is never set.
+      auto probe = [&](const int4& w) {
+        const int32_t id[4] = {w.x, w.y, w.z, w.w};
+        uint32_t r[4], x[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          r[j] = min(static_cast<uint32_t>(id[j] - a.base), static_cast<uint32_t>(a.bits));
+          x[j] = s_bits[r[j] >> 5];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) found += __funnelshift_r(x[j], 0u, r[j]) & 1u;
+      };
+      // Each half of the warp has the lists of its 16 lanes, 64 entries at a
+      // time: half of R-MAT's scanned lists are shorter than that.
+      const int half = lane & 16, hl = lane & 15;
+      unsigned m = (__ballot_sync(0xffffffffu, take) >> half) & 0xffffu;
+      while (__any_sync(0xffffffffu, m != 0)) {
+        const int4* p[kTcAhead];
+        int n[kTcAhead];
+        int4 w[kTcAhead];
+#pragma unroll
+        for (int j = 0; j < kTcAhead; ++j, m &= m - 1) {
+          const int l = half + (m ? __ffs(m) - 1 : 0);
+          const int64_t start = __shfl_sync(0xffffffffu, iy.start, l);
+          const int ny = __shfl_sync(0xffffffffu, iy.n, l);
+          n[j] = m ? ny : 0;
+          p[j] = reinterpret_cast<const int4*>(a.dcol + start) + hl;
+          if (4 * hl < n[j]) w[j] = __ldg(p[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < kTcAhead; ++j) {
+          if (4 * hl < n[j]) probe(w[j]);
+          for (int q = 64 + 4 * hl; q < n[j]; q += 64) {
+            p[j] += 16;
+            probe(__ldg(p[j]));
+          }
+        }
+      }
+    }
+    cnt += found;
+    __syncthreads();
+    for (int k = threadIdx.x; k < ix.n; k += NT)
+      s_bits[static_cast<uint32_t>(a.dcol[ix.start + k] - a.base) >> 5] = 0u;
+  }
+  tc_flush<NT>(cnt, work, a.out);
+}
+
+// Warp per vertex of a.small: N+(x) in a hash table (linear probing, at most a
+// quarter full, kTcPiece entries at a time), the scanned lists of 32
+// neighbours as one stream.
+__global__ void __launch_bounds__(kTcThreads) tc_warp_kernel(const __grid_constant__ TcArgs a) {
+  extern __shared__ __align__(16) int32_t s_tab[];
+  const int lane = threadIdx.x & 31;
+  int32_t* tab = s_tab + kTcSlots * (threadIdx.x >> 5);
+  const int n_small = static_cast<int>(a.ctr[2]);
   unsigned long long cnt = 0, work = 0;
   for (;;) {
     int i0 = 0;
-    if (lane == 0) i0 = static_cast<int>(atomicAdd(ctr, static_cast<unsigned>(kTcGrab)));
+    if (lane == 0) i0 = static_cast<int>(atomicAdd(a.ctr + 5, static_cast<unsigned>(kTcGrab)));
     i0 = __shfl_sync(0xffffffffu, i0, 0);
-    if (i0 >= n_order) break;
-    const int i1 = i0 + kTcGrab < n_order ? i0 + kTcGrab : n_order;
-    for (int i = i0; i < i1; ++i) {
-      const int32_t u = order[i];
-      const int64_t b = doff[u];
-      const int n = static_cast<int>(doff[u + 1] - b);
-      for (int k = lane; k < kFilterWords; k += 32) bits[k] = 0u;
-      __syncwarp();
-      for (int k = lane; k < n; k += 32) {
-        const int32_t x = dcol[b + k];
-        list[k] = x;
-        const uint32_t h = tc_hash<kFilterBits>(x);
-        atomicOr(&bits[h >> 5], 1u << (h & 31));
-      }
-      __syncwarp();
-      int qn = 0;
-      // Offsets of N+(v) for the next v are loaded while this one is probed.
-      int64_t vb = doff[list[0]], ve = doff[list[0] + 1];
-      for (int k = 0; k < n; ++k) {
-        int64_t nb = 0, ne = 0;
-        if (k + 1 < n) {
-          nb = doff[list[k + 1]];
-          ne = doff[list[k + 1] + 1];
+    if (i0 >= n_small) break;
+    for (int i = i0; i < min(i0 + kTcGrab, n_small); ++i) {
+      const int32_t x = a.small[i];
+      const TcInfo ix = a.info[x];
+      const int64_t b = a.off[x];
+      const int deg = static_cast<int>(a.off[x + 1] - b);
+      for (int p0 = 0; p0 < ix.n; p0 += kTcPiece) {
+        const int np = min(kTcPiece, ix.n - p0);
+        const int bits = 32 - __clz(max(4 * np - 1, 31));  // 32 slots or more, at most kTcSlots
+        for (int k = lane; k < (1 << bits); k += 32) tab[k] = kTcNone;
+        __syncwarp();
+        const auto slot = [&](int32_t w) { return static_cast<int>((static_cast<uint32_t>(w) * 2654435761u) >> (32 - bits)); };
+        const int mask = (1 << bits) - 1;
+        for (int k = lane; k < np; k += 32) {
+          const int32_t w = a.dcol[ix.start + p0 + k];
+          for (int h = slot(w); atomicCAS(tab + h, kTcNone, w) != kTcNone; h = (h + 1) & mask) {
+          }
         }
-        tc_probe_filtered<kFilterBits>(dcol, vb, static_cast<int>(ve - vb), list, n, bits, q, qn, lane, cnt, work);
-        vb = nb;
-        ve = ne;
+        __syncwarp();
+        for (int g = 0; g < deg; g += 32) {
+          TcInfo iy{0, 0, 0};
+          int len = 0;
+          if (g + lane < deg) {
+            const int32_t y = a.col[b + g + lane];
+            iy = a.info[y];
+            if (tc_scans(ix.n, x, iy.n, y)) len = iy.n;
+          }
+          int pre = len;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, pre, o);
+            if (lane >= o) pre += t;
+          }
+          const int total = __shfl_sync(0xffffffffu, pre, 31);
+          pre -= len;
+          work += static_cast<unsigned>(len);
+          for (int k0 = 0; k0 < total; k0 += 64) {
+            int32_t w[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              const int k = k0 + 32 * j + lane;
+              int l = 0;  // (every lane takes part in every shuffle)
+#pragma unroll
+              for (int sp = 16; sp > 0; sp >>= 1) {
+                const int t = __shfl_sync(0xffffffffu, pre, l + sp);
+                if (t <= k) l += sp;
+              }
+              const int lo = __shfl_sync(0xffffffffu, pre, l);
+              const int64_t start = __shfl_sync(0xffffffffu, iy.start, l);
+              w[j] = k < total ? __ldg(a.dcol + start + (k - lo)) : kTcNone;
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              if (w[j] != kTcNone) {
+                for (int h = slot(w[j]);; h = (h + 1) & mask) {
+                  const int32_t t = tab[h];
+                  if (t == w[j]) ++cnt;
+                  if (t == w[j] || t == kTcNone) break;
+                }
+              }
+            }
+          }
+          __syncwarp();
+        }
+        __syncwarp();
       }
-      // The queue's rest belongs to this list: searched before the next is staged.
-      if (lane < qn) cnt += tc_search(list, n, q[lane]);
-      __syncwarp();
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-    work += __shfl_xor_sync(0xffffffffu, work, o);
-  }
-  if (lane == 0) {
-    s_red[0][wid] = cnt;
-    s_red[1][wid] = work;
-  }
-  __syncthreads();
-  if (threadIdx.x < 2) {
-    unsigned long long t = 0;
-    for (int w = 0; w < kTcWarps; ++w) t += s_red[threadIdx.x][w];
-    if (t) atomicAdd(out + threadIdx.x, t);
-  }
+  tc_flush<kTcThreads>(cnt, work, a.out);
 }
 
-// CTA per vertex for |N+(u)| > kWarpList, claimed one at a time from ctr;
-// the CTA's warps split N+(u) and probe through the filter like the warp
-// kernel.  Dynamic shared memory holds the 2^16-bit filter, the warps'
-// queues, then room for `cap` list entries (the longest list of the launch,
-// at most kCtaList); a longer list is searched where it lies in global
-// memory, its filter still in shared memory.
-__global__ void __launch_bounds__(kTcThreads) tc_cta_kernel(const int64_t* doff, const int32_t* dcol,
-                                                            const int32_t* order, int32_t n_order, int cap,
-                                                            unsigned int* ctr, unsigned long long* out) {
-  extern __shared__ uint32_t s_dyn[];
-  uint32_t* bits = s_dyn;
-  int32_t* q = reinterpret_cast<int32_t*>(s_dyn + kCtaFilterWords) + kQueue * (threadIdx.x >> 5);
-  int32_t* s_big = reinterpret_cast<int32_t*>(s_dyn + kCtaFilterWords) + kQueue * kTcWarps;
-  __shared__ unsigned long long s_red[2][kTcWarps];
-  __shared__ int s_i;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  unsigned long long cnt = 0, work = 0;
-  for (;;) {
-    if (threadIdx.x == 0) s_i = static_cast<int>(atomicAdd(ctr, 1u));
-    __syncthreads();
-    const int i = s_i;
-    if (i >= n_order) break;
-    const int32_t u = order[i];
-    const int64_t b = doff[u];
-    const int n = static_cast<int>(doff[u + 1] - b);
-    const bool staged = n <= cap;
-    const int32_t* list = staged ? s_big : dcol + b;
-    for (int k = threadIdx.x; k < kCtaFilterWords; k += kTcThreads) bits[k] = 0u;
-    __syncthreads();
-    for (int k = threadIdx.x; k < n; k += kTcThreads) {
-      const int32_t x = dcol[b + k];
-      if (staged) s_big[k] = x;
-      const uint32_t h = tc_hash<kCtaFilterBits>(x);
-      atomicOr(&bits[h >> 5], 1u << (h & 31));
-    }
-    __syncthreads();
-    int qn = 0;
-    for (int k = wid; k < n; k += kTcWarps) {
-      const int32_t v = list[k];
-      const int64_t vb = doff[v];
-      tc_probe_filtered<kCtaFilterBits>(dcol, vb, static_cast<int>(doff[v + 1] - vb), list, n, bits, q, qn, lane,
-                                        cnt, work);
-    }
-    if (lane < qn) cnt += tc_search(list, n, q[lane]);
-    __syncthreads();
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-    work += __shfl_xor_sync(0xffffffffu, work, o);
-  }
-  if (lane == 0) {
-    s_red[0][wid] = cnt;
-    s_red[1][wid] = work;
-  }
-  __syncthreads();
-  if (threadIdx.x < 2) {
-    unsigned long long t = 0;
-    for (int w = 0; w < kTcWarps; ++w) t += s_red[threadIdx.x][w];
-    if (t) atomicAdd(out + threadIdx.x, t);
-  }
-}
-
-struct TcBuffers {
-  int32_t* deg = nullptr;
-  int32_t* cnt = nullptr;
-  int64_t* doff = nullptr;
-  int32_t* dcol = nullptr;
-  int32_t* order = nullptr;
-  unsigned long long* out = nullptr;
-  unsigned int* ctr = nullptr;
-  ~TcBuffers() {
-    dev_free(&deg);
-    dev_free(&cnt);
-    dev_free(&doff);
-    dev_free(&dcol);
-    dev_free(&order);
-    dev_free(&out);
-    dev_free(&ctr);
-  }
+struct TcBlock {
+  unsigned char* p = nullptr;
+  ~TcBlock() { dev_free(&p); }
 };
 
 }  // namespace
@@ -356,127 +433,107 @@ extern "C" gx_status gx_triangle_count(gx_engine* e, uint64_t* total, gx_run_sta
   GX_CUDA(cudaSetDevice(e->dev));
   const int32_t V = e->V;
   cudaStream_t s = e->s_comp;
-  TcBuffers b;
-  cudaEvent_t ev0, ev1;
+  cudaEvent_t ev0, ev1, listed, big_done;
   GX_CUDA(cudaEventCreate(&ev0));
+  std::unique_ptr<CUevent_st, cudaError_t (*)(cudaEvent_t)> g0(ev0, cudaEventDestroy);
   GX_CUDA(cudaEventCreate(&ev1));
+  std::unique_ptr<CUevent_st, cudaError_t (*)(cudaEvent_t)> g1(ev1, cudaEventDestroy);
+  GX_CUDA(cudaEventCreateWithFlags(&listed, cudaEventDisableTiming));
+  std::unique_ptr<CUevent_st, cudaError_t (*)(cudaEvent_t)> g2(listed, cudaEventDestroy);
+  GX_CUDA(cudaEventCreateWithFlags(&big_done, cudaEventDisableTiming));
+  std::unique_ptr<CUevent_st, cudaError_t (*)(cudaEvent_t)> g3(big_done, cudaEventDestroy);
   GX_CUDA(cudaEventRecord(ev0, s));
-  GX_TRY(dev_alloc(&b.deg, static_cast<size_t>(V)));
-  GX_TRY(dev_alloc(&b.cnt, static_cast<size_t>(V)));
-  GX_TRY(dev_alloc(&b.out, 2));
-  GX_TRY(dev_alloc(&b.ctr, 2));  // claim counters of the warp and CTA kernels
-  const int grid = e->n_sm * 8;
-  tc_degree_kernel<<<grid, 256, 0, s>>>(e->d_off, V, b.deg);
-  const int32_t* inv = e->relabeled ? e->d_inv : nullptr;
-  tc_count_kernel<<<grid, 256, 0, s>>>(e->d_off, e->d_col, b.deg, inv, V, b.cnt);
+  const bool ranked = V > tc_bits(V);
+  int vb = 1;
+  while (vb < 31 && (int64_t(1) << vb) < V) ++vb;
+  // One block for all arrays.
+  TcBlock block;
+  size_t at = 0;
+  auto place = [&](size_t bytes) {
+    const size_t x = at;
+    at += (bytes + 255) & ~size_t(255);
+    return x;
+  };
+  const size_t nv = static_cast<size_t>(V);
+  int64_t hist_n = 0, part_n = 0;
+  radix_scratch_sizes(V, &hist_n, &part_n);
+  const size_t o_deg = place(4 * nv), o_n = place(4 * nv), o_info = place(sizeof(TcInfo) * nv);
+  const size_t o_big = place(4 * nv), o_small = place(4 * nv), o_ctr = place(8 * sizeof(unsigned int)),
+               o_out = place(2 * sizeof(unsigned long long));
+  const size_t o_dcol = place(sizeof(int32_t) * (static_cast<size_t>(e->E) + 4 * nv + 8));
+  const size_t o_rank = place(ranked ? 4 * nv : 0), o_keys = place(ranked ? 16 * nv : 0),
+               o_hist = place(ranked ? 4 * static_cast<size_t>(hist_n) : 0),
+               o_offs = place(ranked ? 8 * static_cast<size_t>(hist_n) : 0),
+               o_part = place(ranked ? 8 * static_cast<size_t>(part_n) : 0);
+  GX_TRY(dev_alloc(&block.p, at));
+  TcArgs a{};
+  a.off = e->d_off;
+  a.col = e->d_col;
+  a.units = e->d_units;
+  a.heavy = e->d_heavy;
+  a.n_units = static_cast<int32_t>(e->units.size());
+  a.chunk = e->caps.chunk;
+  a.heavy_deg = e->caps.heavy;
+  a.V = V;
+  int32_t* deg = reinterpret_cast<int32_t*>(block.p + o_deg);
+  a.deg = deg;
+  a.n = reinterpret_cast<int32_t*>(block.p + o_n);
+  a.info = reinterpret_cast<TcInfo*>(block.p + o_info);
+  a.big = reinterpret_cast<int32_t*>(block.p + o_big);
+  a.small = reinterpret_cast<int32_t*>(block.p + o_small);
+  a.ctr = reinterpret_cast<unsigned int*>(block.p + o_ctr);
+  a.out = reinterpret_cast<unsigned long long*>(block.p + o_out);
+  a.dcol = reinterpret_cast<int32_t*>(block.p + o_dcol);
+  a.bits = static_cast<int32_t>(tc_bits(V));
+  a.base = V - a.bits;
+  a.mask = vb >= 32 ? 0xffffffffu : (1u << vb) - 1u;
+  a.mix = 2654435761u;
+  GX_CUDA(cudaMemsetAsync(a.ctr, 0, 8 * sizeof(unsigned int), s));
+  GX_CUDA(cudaMemsetAsync(a.out, 0, 2 * sizeof(unsigned long long), s));
+  const int grid_v = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(e->n_sm * 8, (V + 255) / 256)));
+  unsigned long long* keys = reinterpret_cast<unsigned long long*>(block.p + o_keys);
+  tc_degree_kernel<<<grid_v, 256, 0, s>>>(e->d_off, V, deg, a.n, ranked ? keys : nullptr, vb);
+  if (ranked) {
+    unsigned long long* sorted = nullptr;
+    GX_TRY(radix_sort_bits(keys, keys + nv, V, vb, 2 * vb, reinterpret_cast<uint32_t*>(block.p + o_hist),
+                           reinterpret_cast<unsigned long long*>(block.p + o_offs),
+                           reinterpret_cast<unsigned long long*>(block.p + o_part), s, &sorted));
+    int32_t* rank = reinterpret_cast<int32_t*>(block.p + o_rank);
+    tc_rank_kernel<<<grid_v, 256, 0, s>>>(sorted, (1ull << vb) - 1, V, rank);
+    a.rank = rank;
+  }
+  int per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tc_fill_kernel, kTcThreads, 0);
+  const int64_t grid_u = (static_cast<int64_t>(a.n_units) + kTcWarps - 1) / kTcWarps;
+  tc_fill_kernel<<<static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(std::max(1, per_sm) * e->n_sm, grid_u))),
+                   kTcThreads, 0, s>>>(a);
+  tc_list_kernel<<<grid_v, 256, 0, s>>>(a);
   GX_CUDA(cudaGetLastError());
-  // Offsets of N+ and the claim order (descending |N+|, by power-of-two bins).
-  // Host buffers are not zero-filled (every element is written below) and are
-  // first touched by the threads that fill them.
-  std::unique_ptr<int32_t[]> cnt(new int32_t[V]);
-  GX_CUDA(cudaMemcpyAsync(cnt.get(), b.cnt, sizeof(int32_t) * V, cudaMemcpyDeviceToHost, s));
-  GX_CUDA(cudaStreamSynchronize(s));
-  // Prefix sums and the claim order on the host threads: each thread scans
-  // and bins a contiguous block of vertices; blocks are joined in order.
-  const int nt = std::max(1, omp_get_max_threads());
-  std::unique_ptr<int64_t[]> doff(new int64_t[static_cast<size_t>(V) + 1]);
-  std::vector<int64_t> part(static_cast<size_t>(nt) + 1, 0);
-  std::vector<std::vector<std::vector<int32_t>>> tbins(nt, std::vector<std::vector<int32_t>>(34));
-#pragma omp parallel num_threads(nt)
-  {
-    const int t = omp_get_thread_num();
-    const int32_t lo = static_cast<int32_t>(static_cast<int64_t>(V) * t / nt);
-    const int32_t hi = static_cast<int32_t>(static_cast<int64_t>(V) * (t + 1) / nt);
-    int64_t run = 0;
-    for (int32_t v = lo; v < hi; ++v) {
-      run += cnt[v];
-      if (cnt[v] < 2) continue;  // no pair of out-neighbours, no triangle
-      tbins[t][cnt[v] > kWarpList ? 33 : 31 - __builtin_clz(static_cast<unsigned>(cnt[v]))].push_back(v);
-    }
-    part[t + 1] = run;
-#pragma omp barrier
-#pragma omp single
-    for (int i = 0; i < nt; ++i) part[i + 1] += part[i];
-    int64_t acc = part[t];
-    for (int32_t v = lo; v < hi; ++v) {
-      doff[v] = acc;
-      acc += cnt[v];
-    }
-  }
-  doff[V] = part[nt];
-  const int64_t m = doff[V];
-  // Claim order: the long lists sorted by (|N+| descending, id), then bins 32
-  // down to 0, each bin in thread order; copied in parallel to offsets
-  // computed first.
-  std::vector<int32_t> big;
-  for (int t = 0; t < nt; ++t) big.insert(big.end(), tbins[t][33].begin(), tbins[t][33].end());
-  std::sort(big.begin(), big.end(), [&](int32_t a, int32_t c) { return cnt[a] > cnt[c] || (cnt[a] == cnt[c] && a < c); });
-  const int32_t n_big = static_cast<int32_t>(big.size());
-  std::vector<int64_t> at(static_cast<size_t>(33) * nt);
-  int64_t n_order = n_big;
-  for (int k = 32; k >= 0; --k)
-    for (int t = 0; t < nt; ++t) {
-      at[static_cast<size_t>(k) * nt + t] = n_order;
-      n_order += static_cast<int64_t>(tbins[t][k].size());
-    }
-  std::unique_ptr<int32_t[]> order(new int32_t[std::max<int64_t>(n_order, 1)]);
-  if (n_big) memcpy(order.get(), big.data(), sizeof(int32_t) * n_big);
-#pragma omp parallel for schedule(dynamic, 1) num_threads(nt)
-  for (int i = 0; i < 33 * nt; ++i) {
-    const int k = i / nt, t = i % nt;
-    const std::vector<int32_t>& bin = tbins[t][k];
-    if (!bin.empty()) memcpy(order.get() + at[i], bin.data(), sizeof(int32_t) * bin.size());
-  }
-  const int32_t n_small = static_cast<int32_t>(n_order) - n_big;
-  GX_TRY(dev_alloc(&b.doff, static_cast<size_t>(V) + 1));
-  GX_TRY(dev_alloc(&b.dcol, static_cast<size_t>(m) + 1));
-  GX_TRY(dev_alloc(&b.order, static_cast<size_t>(n_order) + 1));
-  GX_CUDA(cudaMemcpyAsync(b.doff, doff.get(), sizeof(int64_t) * (V + 1), cudaMemcpyHostToDevice, s));
-  if (n_order > 0)
-    GX_CUDA(cudaMemcpyAsync(b.order, order.get(), sizeof(int32_t) * n_order, cudaMemcpyHostToDevice, s));
-  tc_fill_kernel<<<grid, 256, 0, s>>>(e->d_off, e->d_col, b.deg, inv, V, b.doff, b.dcol);
-  GX_CUDA(cudaMemsetAsync(b.out, 0, 2 * sizeof(unsigned long long), s));
-  GX_CUDA(cudaMemsetAsync(b.ctr, 0, 2 * sizeof(unsigned int), s));
-  // The long lists run on the copy stream beside the warp kernel, so the
-  // few CTAs they need do not hold the rest of the GPU idle.
-  cudaEvent_t filled = nullptr, big_done = nullptr;
-  if (n_big > 0) {
-    GX_CUDA(cudaEventCreateWithFlags(&filled, cudaEventDisableTiming));
-    GX_CUDA(cudaEventCreateWithFlags(&big_done, cudaEventDisableTiming));
-    GX_CUDA(cudaEventRecord(filled, s));
-    GX_CUDA(cudaStreamWaitEvent(e->s_copy, filled, 0));
-    // Shared memory for the longest list only (big[0]), so the CTAs leave
-    // room on their SMs for the warp kernel's.
-    const int cap = std::min(cnt[big[0]], kCtaList);
-    const size_t smem = sizeof(uint32_t) * (kCtaFilterWords + kQueue * kTcWarps + static_cast<size_t>(cap));
-    GX_CUDA(cudaFuncSetAttribute(tc_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tc_cta_kernel, kTcThreads, smem);
-    const int grid_cta = std::min(n_big, std::max(1, per_sm) * e->n_sm);
-    tc_cta_kernel<<<grid_cta, kTcThreads, smem, e->s_copy>>>(b.doff, b.dcol, b.order, n_big, cap, b.ctr + 1,
-                                                             b.out);
-    GX_CUDA(cudaEventRecord(big_done, e->s_copy));
-  }
-  if (n_small > 0) {
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tc_warp_kernel, kTcThreads, 0);
-    tc_warp_kernel<<<std::max(1, per_sm) * e->n_sm, kTcThreads, 0, s>>>(b.doff, b.dcol, b.order + n_big, n_small,
-                                                                        b.ctr, b.out);
-  }
+  // The CTAs' vertices on the copy stream, the warps' beside them.
+  GX_CUDA(cudaEventRecord(listed, s));
+  GX_CUDA(cudaStreamWaitEvent(e->s_copy, listed, 0));
+  const int smem_cta = (a.bits / 32 + 1) * 4, smem_warp = kTcSlots * kTcWarps * 4;
+  // As many CTAs as bitmaps fit an SM, their threads filling it: the fewer
+  // threads a vertex has, the fewer wait at its end.
+  const int fit = std::max(1, (220 * 1024) / (smem_cta + 2048));
+  void (*cta)(TcArgs) = fit >= 6 ? tc_cta_kernel<256> : fit >= 2 ? tc_cta_kernel<512> : tc_cta_kernel<1024>;
+  const int cta_threads = fit >= 6 ? 256 : fit >= 2 ? 512 : 1024;
+  GX_CUDA(cudaFuncSetAttribute(cta, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_cta));
+  GX_CUDA(cudaFuncSetAttribute(tc_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_warp));
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cta, cta_threads, smem_cta);
+  cta<<<std::max(1, per_sm) * e->n_sm, cta_threads, smem_cta, e->s_copy>>>(a);
   GX_CUDA(cudaGetLastError());
-  if (big_done) {
-    GX_CUDA(cudaStreamWaitEvent(s, big_done, 0));
-    cudaEventDestroy(filled);
-    cudaEventDestroy(big_done);
-  }
+  GX_CUDA(cudaEventRecord(big_done, e->s_copy));
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tc_warp_kernel, kTcThreads, smem_warp);
+  tc_warp_kernel<<<std::max(1, per_sm) * e->n_sm, kTcThreads, smem_warp, s>>>(a);
+  GX_CUDA(cudaGetLastError());
+  GX_CUDA(cudaStreamWaitEvent(s, big_done, 0));
   unsigned long long res[2] = {0, 0};
-  GX_CUDA(cudaMemcpyAsync(res, b.out, sizeof(res), cudaMemcpyDeviceToHost, s));
+  GX_CUDA(cudaMemcpyAsync(res, a.out, sizeof(res), cudaMemcpyDeviceToHost, s));
   GX_CUDA(cudaEventRecord(ev1, s));
   GX_CUDA(cudaEventSynchronize(ev1));
   float ms = 0;
   cudaEventElapsedTime(&ms, ev0, ev1);
-  cudaEventDestroy(ev0);
-  cudaEventDestroy(ev1);
   *total = res[0];
   if (stats) {
     *stats = gx_run_stats{};
@@ -484,7 +541,7 @@ extern "C" gx_status gx_triangle_count(gx_engine* e, uint64_t* total, gx_run_sta
     stats->edges_scanned = static_cast<int64_t>(res[1]);
     stats->ms_total = ms;
     stats->ms_compute = ms;
-    stats->kernel_launches = 4 + (n_big > 0) + (n_small > 0);
+    stats->kernel_launches = ranked ? 6 : 5;  // the sort's passes not counted
   }
   return GX_OK;
 }
