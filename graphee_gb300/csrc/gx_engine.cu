@@ -607,6 +607,13 @@ gx_status encode_streamed(gx_engine* e, const int32_t* col) {
   return GX_OK;
 }
 
+// Streamed shards side by side travel and are swept together up to this many
+// edges, resident ones up to twice as many: a launch of one small shard lasts
+// some 30 us, whatever it holds, and a copy of 2 MB half as long as its calls.
+// (Scale 24 in 256 shards, half of them streamed: 7.5 ms a superstep a shard at
+// a time, 3.8 in groups of 4 M edges, 2.6 of them copies.)
+constexpr int64_t kStreamGroup = int64_t(4) << 20;
+
 // Decides which shards stay in HBM under the budget (in shard order, like the
 // reference's insert-until-full edge cache, Global.h:170-244), uploads them,
 // and sets up the streaming ring for the rest.  When the plain shards exceed
@@ -651,9 +658,12 @@ gx_status plan_shards(gx_engine* e, const int32_t* src_col, bool col_on_device) 
   } else {
     GX_TRY(dev_alloc(&e->d_col, static_cast<size_t>(used) + 8));
     if (e->has_weights) GX_TRY(dev_alloc(&e->d_w, static_cast<size_t>(used) + 8));
+    // Consecutive resident shards lie end to end, as in the graph, so that one
+    // launch can sweep several.
     int64_t pos = 0;
     for (int32_t p = 0; p < P; ++p) {
       if (!e->resident[p]) continue;
+      if (p > 0 && e->resident[p - 1]) pos = e->dev_base[p - 1] + lo[p];
       const int64_t n = std::min(hi[p], e->E + 4) - lo[p];
       GX_CUDA(cudaMemcpy(e->d_col + pos, src_col + lo[p], n * sizeof(int32_t), cudaMemcpyHostToDevice));
       if (e->has_weights)
@@ -662,7 +672,10 @@ gx_status plan_shards(gx_engine* e, const int32_t* src_col, bool col_on_device) 
       pos += hi[p] - lo[p] + 4;
     }
     const int slots = std::max({2, e->cfg.stream_slots, static_cast<int>(e->s_copies.size())});
-    e->slot_elems = max_stream + 8;
+    int64_t streamed_elems = 0;
+    for (int32_t p = 0; p < P; ++p)
+      if (!e->resident[p]) streamed_elems += hi[p] - lo[p];
+    e->slot_elems = std::max(max_stream, std::min(streamed_elems, kStreamGroup)) + 8;
     for (auto ptr : e->slot_col) gx::pool_free(ptr);
     for (auto ptr : e->slot_w) gx::pool_free(ptr);
     for (auto ptr : e->slot_blob) gx::pool_free(ptr);
@@ -1126,7 +1139,7 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
       }
     }
   } else {
-    // Host-driven steps: one launch per shard, streamed shards through the
+    // Host-driven steps: one launch per group of shards, streamed ones through the
     // slot ring on the copy stream, overlapped with compute.  A Jacobi step
     // may sweep its shards in any order, so streamed shards are spread evenly
     // among the resident ones: the copy engine then works through the whole
@@ -1138,17 +1151,38 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
     if constexpr (APP == K_SSSP_UNIT || APP == K_SSSP_W || APP == K_CC) {
       if (c.async_mode) pull_comp = pull_kernel<APP, false, true, true>;
     }
-    std::vector<int32_t> order;
-    {
-      std::vector<int32_t> res, str;
-      for (int32_t p = 0; p < e->P; ++p) (e->resident[p] ? res : str).push_back(p);
-      const int64_t S = static_cast<int64_t>(str.size()), Pn = e->P;
+    // Shards [first, last) swept by one launch: consecutive, of one kind and
+    // fate (a compressed shard alone).
+    struct Group {
+      int32_t first, last;
+      bool active;
+    };
+    std::vector<Group> order, res, str;
+    auto travels_compressed = [&](int32_t p) { return e->comp && !e->resident[p] && e->cb_bytes[p] > 0; };
+    auto plan_order = [&](const std::vector<char>& on) {
+      res.clear();
+      str.clear();
+      order.clear();
+      for (int32_t p = 0; p < e->P;) {
+        const bool resident = e->resident[p] != 0, active = on[p] != 0;
+        const int64_t most = resident ? 2 * kStreamGroup : e->slot_elems - 8;
+        const bool alone = active && travels_compressed(p);
+        int32_t q = p + 1;
+        while (!alone && q < e->P && (e->resident[q] != 0) == resident && (on[q] != 0) == active &&
+               !(active && travels_compressed(q)) &&
+               (!active || ((e->off[e->bounds[q + 1]] + 3) & ~3ll) - (e->off[e->bounds[p]] & ~3ll) <= most))
+          ++q;
+        (resident ? res : str).push_back(Group{p, q, active});
+        p = q;
+      }
+      const int64_t S = static_cast<int64_t>(str.size()), Pn = S + static_cast<int64_t>(res.size());
       size_t i_r = 0, i_s = 0;
       for (int64_t pos = 0; pos < Pn; ++pos) {
-        const bool take_s = i_s < str.size() && (i_r >= res.size() || (2 * static_cast<int64_t>(i_s) + 1) * Pn <= 2 * pos * S);
+        const bool take_s =
+            i_s < str.size() && (i_r >= res.size() || (2 * static_cast<int64_t>(i_s) + 1) * Pn <= 2 * pos * S);
         order.push_back(take_s ? str[i_s++] : res[i_r++]);
       }
-    }
+    };
     cudaEvent_t c0, c1, k0, k1;
     GX_CUDA(cudaEventCreate(&c0));
     GX_CUDA(cudaEventCreate(&c1));
@@ -1191,14 +1225,16 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
       }
       GX_CUDA(cudaEventRecord(k0, e->s_comp));
       GX_CUDA(cudaEventRecord(c0, e->s_comp));
-      for (const int32_t p : order) {
+      plan_order(shard_on);
+      for (const Group& grp : order) {
+        const int32_t p = grp.first;
         PullArgs sp = pa;
         sp.u_begin = e->unit_begin[p];
-        sp.u_end = e->unit_begin[p + 1];
+        sp.u_end = e->unit_begin[grp.last];
         sp.ctr = e->d_work + static_cast<int64_t>(kQueueStride) * kQueues * (2 + p);
         if (sp.u_end == sp.u_begin) continue;
-        const bool active = shard_on[p] != 0;
-        const bool use_comp = e->comp && !e->resident[p] && active && e->cb_bytes[p] > 0;
+        const bool active = grp.active;
+        const bool use_comp = active && travels_compressed(p);
         if (use_comp) {
           cudaStream_t cs = e->s_copies[slot % e->s_copies.size()];
           GX_CUDA(cudaStreamWaitEvent(cs, e->slot_free[slot], 0));
@@ -1225,7 +1261,7 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
           sp.skip = 1;
         } else {
           const int64_t lo = e->off[e->bounds[p]] & ~3ll;
-          const int64_t n = std::min<int64_t>((e->off[e->bounds[p + 1]] + 3) & ~3ll, e->E + 4) - lo;
+          const int64_t n = std::min<int64_t>((e->off[e->bounds[grp.last]] + 3) & ~3ll, e->E + 4) - lo;
           // Slots alternate over the copy streams, so several copy engines
           // move shards at once.
           cudaStream_t cs = e->s_copies[slot % e->s_copies.size()];
@@ -1240,7 +1276,7 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
           GX_CUDA(cudaStreamWaitEvent(e->s_comp, e->slot_ready[slot], 0));
           sp.col = e->slot_col[slot] - lo;
           if (weighted) sp.w = e->slot_w[slot] - lo;
-          ++streamed;
+          streamed += grp.last - grp.first;
         }
         const PullShape shape = pull_shape(sp.u_end - sp.u_begin, grid_pull_max, kThreads);
         sp.grab = shape.grab;
