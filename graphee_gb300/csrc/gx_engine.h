@@ -232,7 +232,10 @@ struct gx_engine {
   bool out_built = false, out_weighted = false;
   gx::Ctl* d_ctl = nullptr;
   gx::Ctl* h_ctl = nullptr;
+  bool ctl_read = false;             // h_ctl holds d_ctl as the last run left it
+  gx::StepStats* h_run_stats = nullptr;  // the records run_kernel's wait brings (kRunSteps)
   gx::StepStats* d_stats = nullptr;
+  gx::RunScratch* d_run = nullptr;   // run_kernel's sums, barriers and cursors
   int32_t stats_cap = 0;
   unsigned int* d_work = nullptr;
   int32_t n_work = 0;
@@ -352,8 +355,11 @@ struct gx_engine {
     release_graph();
     drop_graphs();
     gx::dev_free(&d_ctl);
+    gx::dev_free(&d_run);
     if (h_ctl) cudaFreeHost(h_ctl);
     h_ctl = nullptr;
+    if (h_run_stats) cudaFreeHost(h_run_stats);
+    h_run_stats = nullptr;
     if (h_stage) cudaFreeHost(h_stage);
     h_stage = nullptr;
     for (cudaEvent_t& ev : stage_ready) {

@@ -180,7 +180,9 @@ __device__ __forceinline__ uint32_t sat_add(uint32_t a, uint32_t b) {
 // ASYNC (Gauss-Seidel, min apps only): values are read and written in one
 // buffer during the step, so gathers go through L2 (ld.cg), never the
 // read-only path.
-template <class T, bool ASYNC, bool HOT>
+// COH (run_kernel): values written earlier in the same launch, ordered by a
+// grid barrier, so plain loads.
+template <class T, bool ASYNC, bool HOT, bool COH = false>
 __device__ __forceinline__ T gather(const T* src, const T* hot, int32_t hot_n, int32_t u) {
   static_assert(sizeof(T) == 4, "4-byte values");
   if constexpr (HOT) {
@@ -193,18 +195,20 @@ __device__ __forceinline__ T gather(const T* src, const T* hot, int32_t hot_n, i
     return x;
   } else if constexpr (ASYNC) {
     return __ldcg(src + u);
+  } else if constexpr (COH) {
+    return src[u];
   } else {
     return __ldg(src + u);
   }
 }
 
-template <int APP, bool ASYNC = false, bool HOT = false>
+template <int APP, bool ASYNC = false, bool HOT = false, bool COH = false>
 __device__ __forceinline__ typename AppTraits<APP>::T edge_value(const PullArgs& a, const void* src_val,
                                                                  const float* src_con, int32_t u, uint32_t wt,
                                                                  const void* hot = nullptr) {
   if constexpr (is_pr<APP>()) {
     if (GX_GATHER_CG && !HOT) return __ldcg(src_con + u);
-    return gather<float, false, HOT>(src_con, static_cast<const float*>(hot), a.hot_n, u);
+    return gather<float, false, HOT, COH>(src_con, static_cast<const float*>(hot), a.hot_n, u);
   } else if constexpr (APP == K_SSSP_UNIT) {
     return gather<int32_t, ASYNC, HOT>(static_cast<const int32_t*>(src_val), static_cast<const int32_t*>(hot),
                                        a.hot_n, u) + 1;  // sssp.cpp:43
@@ -486,7 +490,7 @@ __device__ __forceinline__ uint4 load_w4(const PullArgs& a, int64_t k) {
 // Warp-cooperative reduction of the edge range [b, e) (all lanes call it with
 // the same range): lanes take 8 consecutive edges each per round, with
 // 128-bit loads; the per-lane partials are combined by a fixed xor tree.
-template <int APP, bool ASYNC = false, bool COMP = false, bool HOT = false>
+template <int APP, bool ASYNC = false, bool COMP = false, bool HOT = false, bool COH = false>
 __device__ __forceinline__ typename AppTraits<APP>::T warp_reduce_range(const PullArgs& a, const void* src_val,
                                                                         const float* src_con, int64_t b, int64_t e,
                                                                         int lane, const void* hot = nullptr) {
@@ -508,7 +512,7 @@ __device__ __forceinline__ typename AppTraits<APP>::T warp_reduce_range(const Pu
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int64_t k = (j < 4 ? q : q2) + (j & 3);
-      vals[j] = (k >= b && k < e) ? edge_value<APP, ASYNC, HOT>(a, src_val, src_con, cs[j], ws[j], hot)
+      vals[j] = (k >= b && k < e) ? edge_value<APP, ASYNC, HOT, COH>(a, src_val, src_con, cs[j], ws[j], hot)
                                   : identity<APP>();
     }
 #pragma unroll
@@ -533,7 +537,7 @@ __device__ __forceinline__ typename AppTraits<APP>::T warp_reduce_range(const Pu
 #define GX_GROUP_LANES 8
 #endif
 constexpr int kGroupLanes = GX_GROUP_LANES;
-template <int APP, bool ASYNC = false, bool COMP = false, bool HOT = false>
+template <int APP, bool ASYNC = false, bool COMP = false, bool HOT = false, bool COH = false>
 __device__ __forceinline__ typename AppTraits<APP>::T group_reduce_range(const PullArgs& a, const void* src_val,
                                                                          const float* src_con, int64_t b, int64_t e,
                                                                          int gl, int grp, const void* hot) {
@@ -555,7 +559,7 @@ __device__ __forceinline__ typename AppTraits<APP>::T group_reduce_range(const P
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int64_t k = (j < 4 ? q : q2) + (j & 3);
-      vals[j] = (k >= b && k < e) ? edge_value<APP, ASYNC, HOT>(a, src_val, src_con, cs[j], ws[j], hot)
+      vals[j] = (k >= b && k < e) ? edge_value<APP, ASYNC, HOT, COH>(a, src_val, src_con, cs[j], ws[j], hot)
                                   : identity<APP>();
     }
 #pragma unroll
@@ -586,43 +590,15 @@ __device__ __forceinline__ void expand_hubs(const PullArgs& a, int warp, int war
   }
 }
 
-template <int APP, bool EXACT, bool ASYNC = false, bool COMP = false, bool HOT = false>
-__global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLOCKS) pull_kernel(PullArgs a) {
+// The units of one pull: a.units [a.u_begin, a.u_end), claimed from `ctr`,
+// from values and contributions of buffer `cur`.  sbm (nullable): the bitmap
+// of the shards that a selective step sweeps.
+template <int APP, bool EXACT, bool ASYNC, bool COMP, bool HOT, bool COH>
+__device__ __forceinline__ void pull_sweep(const PullArgs& a, const ApplyCtx& c, int cur, const uint32_t* sbm,
+                                           const void* hot, unsigned int* ctr, LocalAcc& la) {
   typedef typename AppTraits<APP>::T T;
-  static_assert(!(HOT && ASYNC), "a Gauss-Seidel step changes the values the table would hold");
   constexpr int NW = pull_threads<HOT>() / 32;
   __shared__ __align__(16) T s_buf[EXACT ? NW : 1][EXACT ? kChunk : 4];
-  extern __shared__ __align__(16) unsigned char s_dyn[];
-  Ctl* ctl = a.ctl;
-  const int done = ctl->done, mode = ctl->mode;
-  if (done || mode == MODE_PUSH) {
-    if (!done) expand_hubs(a, blockIdx.x * NW + (threadIdx.x >> 5), gridDim.x * NW, threadIdx.x & 31);
-    return;
-  }
-  const void* hot = nullptr;
-  if constexpr (HOT) {
-    // The current step's values of sources [0, hot_n) (PageRank: their
-    // contributions), read through L2 in 16-byte pieces.
-    const int4* src = reinterpret_cast<const int4*>(
-        is_pr<APP>() ? static_cast<const void*>(ctl->cur ? a.con[1] : a.con[0])
-                     : static_cast<const void*>(ctl->cur ? a.val[1] : a.val[0]));
-    int4* dst = reinterpret_cast<int4*>(s_dyn);
-    for (int i = threadIdx.x; i < (a.hot_n >> 2); i += pull_threads<HOT>()) dst[i] = __ldcg(src + i);
-    __syncthreads();
-    hot = s_dyn;
-  }
-  ApplyCtx c;
-  c.step = ctl->step;
-  c.damping = ctl->damping;
-  c.inv_n = ctl->inv_n;
-  c.fx_scale = ctl->fx_scale;
-  c.base = ctl->base;
-  c.outdeg = ctl->push_ok ? a.outdeg : nullptr;
-  const int cur = ctl->cur;
-  // Selective steps skip the units of shards the last finalize left unmarked.
-  const uint32_t* sbm = (mode == MODE_SELECTIVE && ctl->shard_valid)
-                            ? ctl->shard_bm + static_cast<int64_t>(ctl->shard_cur) * ctl->shard_words
-                            : nullptr;
   // Ternaries, not a[cur]: indexing a parameter array with a runtime value
   // would copy the whole parameter block to local memory.
   const void* src_val = cur ? a.val[1] : a.val[0];
@@ -633,7 +609,6 @@ __global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLO
   const bool selective = sbm != nullptr;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   T* buf = s_buf[EXACT ? wid : 0];
-  LocalAcc la;
 
   // Units are split into up to kQueues contiguous ranges, each with its own
   // cursor; a warp starts on queue (warp id mod queues).  When its queue is
@@ -647,7 +622,7 @@ __global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLO
   if (a.grab) {
     qb = a.u_begin + static_cast<int>((static_cast<int64_t>(U) * q) / nq);
     qe = a.u_begin + static_cast<int>((static_cast<int64_t>(U) * (q + 1)) / nq);
-    if (lane == 0) claim = static_cast<int>(atomicAdd(a.ctr + q * kQueueStride, static_cast<unsigned>(a.grab)));
+    if (lane == 0) claim = static_cast<int>(atomicAdd(ctr + q * kQueueStride, static_cast<unsigned>(a.grab)));
   }
   for (;;) {
     const int u0 = qb + __shfl_sync(0xffffffffu, claim, 0);
@@ -657,15 +632,15 @@ __global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLO
       claim = U;
     } else {
       if (u0 >= qe) {
-        q = next_queue(a.ctr, q, nq, U, lane);
+        q = next_queue(ctr, q, nq, U, lane);
         if (q < 0) break;
         qb = a.u_begin + static_cast<int>((static_cast<int64_t>(U) * q) / nq);
         qe = a.u_begin + static_cast<int>((static_cast<int64_t>(U) * (q + 1)) / nq);
-        if (lane == 0) claim = static_cast<int>(atomicAdd(a.ctr + q * kQueueStride, static_cast<unsigned>(a.grab)));
+        if (lane == 0) claim = static_cast<int>(atomicAdd(ctr + q * kQueueStride, static_cast<unsigned>(a.grab)));
         continue;
       }
       cnt = qe - u0 < a.grab ? qe - u0 : a.grab;
-      if (lane == 0) claim = static_cast<int>(atomicAdd(a.ctr + q * kQueueStride, static_cast<unsigned>(a.grab)));
+      if (lane == 0) claim = static_cast<int>(atomicAdd(ctr + q * kQueueStride, static_cast<unsigned>(a.grab)));
     }
     // One coalesced load for the batch's descriptors.
     int2 myu = make_int2(0, 0);
@@ -714,7 +689,7 @@ __global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLO
         const int64_t b = vb + static_cast<int64_t>(wu.y) * a.chunk;
         const int64_t e = ve < b + a.chunk ? ve : b + a.chunk;
         T acc = identity<APP>();
-        if constexpr (APP != K_INDEG) acc = warp_reduce_range<APP, ASYNC, COMP, HOT>(a, src_val, src_con, b, e, lane, hot);
+        if constexpr (APP != K_INDEG) acc = warp_reduce_range<APP, ASYNC, COMP, HOT, COH>(a, src_val, src_con, b, e, lane, hot);
         T* part = static_cast<T*>(a.partial) + H.z;
         bool last = H.y == 1;
         if (lane == 0) {
@@ -743,7 +718,8 @@ __global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLO
             if constexpr (is_pr<APP>()) fin = tot;
             else if constexpr (APP == K_INDEG) fin = static_cast<T>(ve - vb);
             else fin = combine<APP>(old, tot);
-            if (apply_vertex<APP>(c, v, fin, old, od, dst_val, dst_con, la)) atomicOr(a.bm + (v >> 5), 1u << (v & 31));
+            if (apply_vertex<APP>(c, v, fin, old, od, dst_val, dst_con, la) && !COH)
+              atomicOr(a.bm + (v >> 5), 1u << (v & 31));
           }
         }
         continue;
@@ -802,7 +778,7 @@ __global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLO
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                   const int64_t kk = q + e;
-                  x[e] = (kk >= E0 && kk < E1) ? edge_value<APP, ASYNC, HOT>(a, src_val, src_con, cs[e], ws[e], hot)
+                  x[e] = (kk >= E0 && kk < E1) ? edge_value<APP, ASYNC, HOT, COH>(a, src_val, src_con, cs[e], ws[e], hot)
                                                 : identity<APP>();
                 }
                 store4(buf + 4 * (lane + 32 * j), x);
@@ -852,7 +828,7 @@ __global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLO
 #pragma unroll
               for (int j = 0; j < 8; ++j) {
                 const int64_t kk = k + j;
-                vals[j] = (kk >= beg && kk < lend) ? edge_value<APP, ASYNC, HOT>(a, src_val, src_con, cs[j], ws[j], hot)
+                vals[j] = (kk >= beg && kk < lend) ? edge_value<APP, ASYNC, HOT, COH>(a, src_val, src_con, cs[j], ws[j], hot)
                                                    : identity<APP>();
               }
 #pragma unroll
@@ -880,7 +856,7 @@ __global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLO
               const int64_t bl = __shfl_sync(0xffffffffu, beg, sl);
               const int64_t el = __shfl_sync(0xffffffffu, end, sl);
               T r = identity<APP>();
-              if (l >= 0) r = group_reduce_range<APP, ASYNC, COMP, HOT>(a, src_val, src_con, bl, el, gl, grp, hot);
+              if (l >= 0) r = group_reduce_range<APP, ASYNC, COMP, HOT, COH>(a, src_val, src_con, bl, el, gl, grp, hot);
 #pragma unroll
               for (int g = 0; g < NG; ++g) {
                 const int lg = __shfl_sync(0xffffffffu, l, kGroupLanes * g);
@@ -894,7 +870,7 @@ __global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLO
             const int l = __ffs(m) - 1;
             const int64_t bl = __shfl_sync(0xffffffffu, beg, l);
             const int64_t el = __shfl_sync(0xffffffffu, end, l);
-            const T r = warp_reduce_range<APP, ASYNC, COMP, HOT>(a, src_val, src_con, bl, el, lane, hot);
+            const T r = warp_reduce_range<APP, ASYNC, COMP, HOT, COH>(a, src_val, src_con, bl, el, lane, hot);
             if (lane == l) acc = combine<APP>(acc, r);
           }
         }
@@ -904,10 +880,51 @@ __global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLO
         la.edges += end - beg;
         act = apply_vertex<APP>(c, v, acc, old, od, dst_val, dst_con, la);
       }
-      const unsigned m = __ballot_sync(0xffffffffu, act);
-      if (lane == 0) bitmap_set_tile(a.bm, vb, m);
+      if constexpr (!COH) {
+        const unsigned m = __ballot_sync(0xffffffffu, act);
+        if (lane == 0) bitmap_set_tile(a.bm, vb, m);
+      }
     }
   }
+}
+
+template <int APP, bool EXACT, bool ASYNC = false, bool COMP = false, bool HOT = false>
+__global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLOCKS) pull_kernel(PullArgs a) {
+  static_assert(!(HOT && ASYNC), "a Gauss-Seidel step changes the values the table would hold");
+  constexpr int NW = pull_threads<HOT>() / 32;
+  extern __shared__ __align__(16) unsigned char s_dyn[];
+  Ctl* ctl = a.ctl;
+  const int done = ctl->done, mode = ctl->mode;
+  if (done || mode == MODE_PUSH) {
+    if (!done) expand_hubs(a, blockIdx.x * NW + (threadIdx.x >> 5), gridDim.x * NW, threadIdx.x & 31);
+    return;
+  }
+  const void* hot = nullptr;
+  if constexpr (HOT) {
+    // The current step's values of sources [0, hot_n) (PageRank: their
+    // contributions), read through L2 in 16-byte pieces.
+    const int4* src = reinterpret_cast<const int4*>(
+        is_pr<APP>() ? static_cast<const void*>(ctl->cur ? a.con[1] : a.con[0])
+                     : static_cast<const void*>(ctl->cur ? a.val[1] : a.val[0]));
+    int4* dst = reinterpret_cast<int4*>(s_dyn);
+    for (int i = threadIdx.x; i < (a.hot_n >> 2); i += pull_threads<HOT>()) dst[i] = __ldcg(src + i);
+    __syncthreads();
+    hot = s_dyn;
+  }
+  ApplyCtx c;
+  c.step = ctl->step;
+  c.damping = ctl->damping;
+  c.inv_n = ctl->inv_n;
+  c.fx_scale = ctl->fx_scale;
+  c.base = ctl->base;
+  c.outdeg = ctl->push_ok ? a.outdeg : nullptr;
+  const int cur = ctl->cur;
+  // Selective steps skip the units of shards the last finalize left unmarked.
+  const uint32_t* sbm = (mode == MODE_SELECTIVE && ctl->shard_valid)
+                            ? ctl->shard_bm + static_cast<int64_t>(ctl->shard_cur) * ctl->shard_words
+                            : nullptr;
+  LocalAcc la;
+  pull_sweep<APP, EXACT, ASYNC, COMP, HOT, false>(a, c, cur, sbm, hot, a.ctr, la);
   flush_block<NW>(ctl, la);
 }
 
@@ -1192,6 +1209,121 @@ __global__ void __launch_bounds__(kThreads) finalize_kernel(FinArgs a) {
   if (c.mark_mode == MARK_OUT && mark) {
     uint32_t* old_bm = c.shard_bm + static_cast<int64_t>(c.shard_cur) * c.shard_words;
     for (int i = threadIdx.x; i < c.shard_words; i += kThreads) old_bm[i] = 0;
+  }
+}
+
+// PageRank's dense supersteps in one cooperative launch: every step is the
+// pull's sweep, one grid barrier, and the step's tail (finalize_kernel's) from
+// sums that each CTA reads for itself.  It ends when the run does, after
+// kRunSteps, or before a selective step, whose shards the step-by-step launches
+// mark and skip; until then PageRank needs no frontier bitmap.  Per superstep
+// it saves two launches, the bitmap's sweep and the last CTA's work.
+constexpr int kRunSteps = 64;
+struct RunSums {
+  unsigned long long changed, active, edges, resid_fx, dangl_fx, pad[3];
+};
+struct RunScratch {  // cleared before each launch
+  RunSums sums[kRunSteps];
+  unsigned int arrive[kRunSteps][32];                     // a barrier to a 128-byte line
+  unsigned int ctr[kRunSteps][kQueues * kQueueStride];    // work-unit cursors
+};
+struct RunArgs {
+  PullArgs pull;
+  StepStats* stats;
+  RunScratch* run;
+  unsigned int wait_limit;  // polls (of at least 32 ns) of a barrier
+};
+
+template <int APP>
+__global__ void __launch_bounds__(kThreads, GX_PULL_MIN_BLOCKS) run_kernel(const __grid_constant__ RunArgs r) {
+  __shared__ unsigned long long s_red[5][kWarps];
+  __shared__ RunSums s_sum;
+  __shared__ int s_ok;
+  Ctl* ctl = r.pull.ctl;
+  if (ctl->done) return;
+  ApplyCtx c;
+  c.damping = ctl->damping;
+  c.inv_n = ctl->inv_n;
+  c.fx_scale = ctl->fx_scale;
+  c.base = ctl->base;
+  c.outdeg = nullptr;
+  int step = ctl->step, cur = ctl->cur;
+  const int max_iter = ctl->max_iter, n = ctl->n_vertices;
+  const double tolerance = ctl->tolerance, threshold = ctl->sel_threshold;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  bool done = false, selective = false;
+  for (int i = 0; i < kRunSteps && !done && !selective; ++i) {
+    c.step = step;
+    LocalAcc la;
+    pull_sweep<APP, false, false, false, false, true>(r.pull, c, cur, nullptr, nullptr, r.run->ctr[i], la);
+    const unsigned long long x[5] = {warp_sum(la.changed), warp_sum(la.active), warp_sum(la.edges), warp_sum(la.resid),
+                                     warp_sum(la.dangl)};
+    if (lane == 0)
+#pragma unroll
+      for (int k = 0; k < 5; ++k) s_red[k][wid] = x[k];
+    __syncthreads();
+    RunSums* sums = r.run->sums + i;
+    if (threadIdx.x < 5) {
+      unsigned long long t = 0;
+      for (int w = 0; w < kWarps; ++w) t += s_red[threadIdx.x][w];
+      if (t) atomicAdd(&sums->changed + threadIdx.x, t);
+      __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      unsigned int* at = r.run->arrive[i];
+      atomicAdd(at, 1u);
+      int ok = 1;
+      const volatile unsigned int* seen = at;
+      const volatile int* error = &ctl->error;
+      for (unsigned int p = 0; *seen < gridDim.x; ++p) {
+        if (*error || p >= r.wait_limit) {
+          atomicExch(&ctl->error, 4);
+          ok = 0;
+          break;
+        }
+        __nanosleep(32);
+      }
+      __threadfence();
+      s_ok = ok && *error == 0;
+      s_sum.changed = __ldcg(&sums->changed);
+      s_sum.active = __ldcg(&sums->active);
+      s_sum.edges = __ldcg(&sums->edges);
+      s_sum.resid_fx = __ldcg(&sums->resid_fx);
+      s_sum.dangl_fx = __ldcg(&sums->dangl_fx);
+    }
+    __syncthreads();
+    if (!s_ok) return;
+    const float ratio = static_cast<float>(static_cast<double>(s_sum.changed) / n);
+    selective = static_cast<double>(ratio) < threshold;
+    done = (s_sum.changed == 0 && step > 1) || step + 1 >= max_iter;
+    if (tolerance > 0 && static_cast<double>(s_sum.resid_fx) / c.fx_scale < tolerance) done = true;
+    if (APP == K_PR_STD) {
+      const double D = static_cast<double>(s_sum.dangl_fx) / c.fx_scale;
+      c.base = (1.0 - c.damping) * c.inv_n + c.damping * D * c.inv_n;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      StepStats s;
+      s.changed = s_sum.changed;
+      s.active = s_sum.active;
+      s.edges = s_sum.edges;
+      s.resid_fx = s_sum.resid_fx;
+      s.dangl_fx = s_sum.dangl_fx;
+      s.shards_active = -1;
+      s.mode = MODE_DENSE;
+      r.stats[step] = s;
+    }
+    ++step;
+    cur ^= 1;
+    __syncthreads();  // s_red, s_sum are read before the next step writes them
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    ctl->step = step;
+    ctl->cur = cur;
+    ctl->base = c.base;
+    ctl->mode = selective ? MODE_SELECTIVE : MODE_DENSE;
+    ctl->done = done;
   }
 }
 
