@@ -1050,9 +1050,16 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
         &pev, [](std::vector<cudaEvent_t>* v) {
           for (auto ev : *v) cudaEventDestroy(ev);
         });
+    // CC's first step from the ids as labels needs no gather.
+    void (*pull_first)(PullArgs) = nullptr;
+    if constexpr (APP == K_CC) {
+      if (!use_init && !e->relabeled && !c.async_mode && !e->cfg.exact_order && pa.hot_n == 0)
+        pull_first = pull_kernel<APP, false, false, false, false, VIA_ID>;
+    }
+    bool first = pull_first != nullptr;  // the next batch begins with it
     auto enqueue = [&](int i) -> gx_status {
       if (prof) GX_CUDA(cudaEventRecord(pev[2 * i], e->s_comp));
-      pull<<<grid_pull, threads_pull, hot_smem, e->s_comp>>>(pa);
+      (first && i == 0 ? pull_first : pull)<<<grid_pull, threads_pull, hot_smem, e->s_comp>>>(pa);
       if (prof) GX_CUDA(cudaEventRecord(pev[2 * i + 1], e->s_comp));
       if (push_ok) push_kernel<APP><<<grid_push, kThreads, 0, e->s_comp>>>(qa);
       finalize_kernel<APP><<<grid_fin, kThreads, 0, e->s_comp>>>(fa);
@@ -1108,7 +1115,7 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
     cudaGraphExec_t exec = nullptr;
     // Profiling times each pull launch with its own events, so it launches
     // directly instead of replaying a graph.
-    if (e->cfg.use_graph && !prof && !every && !ended) {
+    auto replay = [&](cudaGraphExec_t* out) -> gx_status {
       // A replay bakes in kernels, launch shapes and arguments only, so an
       // executable graph captured by an earlier run with the same bytes of
       // all three is replayed again instead of captured anew.
@@ -1126,8 +1133,10 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
       key.pa = pa;
       key.qa = qa;
       key.fa = fa;
-      exec = e->cached_graph(key);
-      if (!exec) {
+      key.first = first;
+      cudaGraphExec_t x = e->cached_graph(key);
+      if (!x) {
+        const int32_t counted = launches;
         cudaGraph_t graph;
         GX_CUDA(cudaStreamBeginCapture(e->s_comp, cudaStreamCaptureModeThreadLocal));
         for (int i = 0; i < K; ++i) {
@@ -1138,13 +1147,17 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
           }
         }
         GX_CUDA(cudaStreamEndCapture(e->s_comp, &graph));
-        cudaError_t err = cudaGraphInstantiate(&exec, graph, 0);
+        cudaError_t err = cudaGraphInstantiate(&x, graph, 0);
         cudaGraphDestroy(graph);
         if (err != cudaSuccess) return fail(GX_ERR_CUDA, "cudaGraphInstantiate: %s", cudaGetErrorString(err));
-        e->keep_graph(key, exec);
+        e->keep_graph(key, x);
+        launches = counted;
       }
-      launches = 0;
-    }
+      *out = x;
+      return GX_OK;
+    };
+    const bool use_exec = e->cfg.use_graph && !prof && !every && !ended;
+    if (use_exec) launches = 0;
     launches += run_launches;
     const int per_step = push_ok ? 3 : 2;
     // After run_kernel the batch of K steps that it left in goes on from its
@@ -1152,12 +1165,15 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
     // two looks are the same with and without it.
     int batch = run_launches == 0 ? K : (K - (steps_before - prm.first_step) % K) % K;
     for (int launched = steps_before; !ended && launched < prm.max_iter; launched += batch, batch = K) {
-      if (exec && batch == K) {
+      if (use_exec && batch == K) {
+        if (!exec || first) GX_TRY(replay(&exec));
         GX_CUDA(cudaGraphLaunch(exec, e->s_comp));
+        if (first) exec = nullptr;  // the next batch's is another
         launches += K * per_step;
       } else {
         for (int i = 0; i < batch; ++i) GX_TRY(enqueue(i));
       }
+      first = false;
       GX_CUDA(cudaMemcpyAsync(e->h_ctl, e->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, e->s_comp));
       cudaError_t err = cudaStreamSynchronize(e->s_comp);
       if (err != cudaSuccess) return fail(GX_ERR_CUDA, "superstep loop: %s", cudaGetErrorString(err));

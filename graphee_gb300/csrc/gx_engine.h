@@ -124,7 +124,7 @@ gx_status scan_u32(const uint32_t* in, int64_t m, unsigned long long* out, unsig
 // What a captured superstep graph depends on: the kernels, their launch
 // shapes and their argument bytes (zero-filled before use, padding included).
 struct GraphKey {
-  int app, k, push;
+  int app, k, push, first;
   const void* pull;
   int grid_pull, threads_pull;
   size_t smem_pull;

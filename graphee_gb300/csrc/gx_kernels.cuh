@@ -180,9 +180,13 @@ __device__ __forceinline__ uint32_t sat_add(uint32_t a, uint32_t b) {
 // ASYNC (Gauss-Seidel, min apps only): values are read and written in one
 // buffer during the step, so gathers go through L2 (ld.cg), never the
 // read-only path.
-// COH (run_kernel): values written earlier in the same launch, ordered by a
-// grid barrier, so plain loads.
-template <class T, bool ASYNC, bool HOT, bool COH = false>
+// VIA says how a source's value is had otherwise:
+enum : int {
+  VIA_CONST = 0,  // through the read-only path
+  VIA_PLAIN = 1,  // plain loads: values written earlier in the same launch, ordered by a grid barrier (run_kernel)
+  VIA_ID = 2      // not at all: the value is the source's id (CC's first step)
+};
+template <class T, bool ASYNC, bool HOT, int VIA = VIA_CONST>
 __device__ __forceinline__ T gather(const T* src, const T* hot, int32_t hot_n, int32_t u) {
   static_assert(sizeof(T) == 4, "4-byte values");
   if constexpr (HOT) {
@@ -195,26 +199,28 @@ __device__ __forceinline__ T gather(const T* src, const T* hot, int32_t hot_n, i
     return x;
   } else if constexpr (ASYNC) {
     return __ldcg(src + u);
-  } else if constexpr (COH) {
+  } else if constexpr (VIA == VIA_PLAIN) {
     return src[u];
   } else {
     return __ldg(src + u);
   }
 }
 
-template <int APP, bool ASYNC = false, bool HOT = false, bool COH = false>
+template <int APP, bool ASYNC = false, bool HOT = false, int VIA = VIA_CONST>
 __device__ __forceinline__ typename AppTraits<APP>::T edge_value(const PullArgs& a, const void* src_val,
                                                                  const float* src_con, int32_t u, uint32_t wt,
                                                                  const void* hot = nullptr) {
   if constexpr (is_pr<APP>()) {
     if (GX_GATHER_CG && !HOT) return __ldcg(src_con + u);
-    return gather<float, false, HOT, COH>(src_con, static_cast<const float*>(hot), a.hot_n, u);
+    return gather<float, false, HOT, VIA>(src_con, static_cast<const float*>(hot), a.hot_n, u);
   } else if constexpr (APP == K_SSSP_UNIT) {
     return gather<int32_t, ASYNC, HOT>(static_cast<const int32_t*>(src_val), static_cast<const int32_t*>(hot),
                                        a.hot_n, u) + 1;  // sssp.cpp:43
   } else if constexpr (APP == K_SSSP_W) {
     return sat_add(gather<uint32_t, ASYNC, HOT>(static_cast<const uint32_t*>(src_val),
                                                 static_cast<const uint32_t*>(hot), a.hot_n, u), wt);
+  } else if constexpr (VIA == VIA_ID) {
+    return u;
   } else {
     return gather<int32_t, ASYNC, HOT>(static_cast<const int32_t*>(src_val), static_cast<const int32_t*>(hot),
                                        a.hot_n, u);  // cc.cpp:42
@@ -490,7 +496,7 @@ __device__ __forceinline__ uint4 load_w4(const PullArgs& a, int64_t k) {
 // Warp-cooperative reduction of the edge range [b, e) (all lanes call it with
 // the same range): lanes take 8 consecutive edges each per round, with
 // 128-bit loads; the per-lane partials are combined by a fixed xor tree.
-template <int APP, bool ASYNC = false, bool COMP = false, bool HOT = false, bool COH = false>
+template <int APP, bool ASYNC = false, bool COMP = false, bool HOT = false, int VIA = VIA_CONST>
 __device__ __forceinline__ typename AppTraits<APP>::T warp_reduce_range(const PullArgs& a, const void* src_val,
                                                                         const float* src_con, int64_t b, int64_t e,
                                                                         int lane, const void* hot = nullptr) {
@@ -512,7 +518,7 @@ __device__ __forceinline__ typename AppTraits<APP>::T warp_reduce_range(const Pu
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int64_t k = (j < 4 ? q : q2) + (j & 3);
-      vals[j] = (k >= b && k < e) ? edge_value<APP, ASYNC, HOT, COH>(a, src_val, src_con, cs[j], ws[j], hot)
+      vals[j] = (k >= b && k < e) ? edge_value<APP, ASYNC, HOT, VIA>(a, src_val, src_con, cs[j], ws[j], hot)
                                   : identity<APP>();
     }
 #pragma unroll
@@ -537,7 +543,7 @@ __device__ __forceinline__ typename AppTraits<APP>::T warp_reduce_range(const Pu
 #define GX_GROUP_LANES 8
 #endif
 constexpr int kGroupLanes = GX_GROUP_LANES;
-template <int APP, bool ASYNC = false, bool COMP = false, bool HOT = false, bool COH = false>
+template <int APP, bool ASYNC = false, bool COMP = false, bool HOT = false, int VIA = VIA_CONST>
 __device__ __forceinline__ typename AppTraits<APP>::T group_reduce_range(const PullArgs& a, const void* src_val,
                                                                          const float* src_con, int64_t b, int64_t e,
                                                                          int gl, int grp, const void* hot) {
@@ -559,7 +565,7 @@ __device__ __forceinline__ typename AppTraits<APP>::T group_reduce_range(const P
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int64_t k = (j < 4 ? q : q2) + (j & 3);
-      vals[j] = (k >= b && k < e) ? edge_value<APP, ASYNC, HOT, COH>(a, src_val, src_con, cs[j], ws[j], hot)
+      vals[j] = (k >= b && k < e) ? edge_value<APP, ASYNC, HOT, VIA>(a, src_val, src_con, cs[j], ws[j], hot)
                                   : identity<APP>();
     }
 #pragma unroll
@@ -593,7 +599,7 @@ __device__ __forceinline__ void expand_hubs(const PullArgs& a, int warp, int war
 // The units of one pull: a.units [a.u_begin, a.u_end), claimed from `ctr`,
 // from values and contributions of buffer `cur`.  sbm (nullable): the bitmap
 // of the shards that a selective step sweeps.
-template <int APP, bool EXACT, bool ASYNC, bool COMP, bool HOT, bool COH>
+template <int APP, bool EXACT, bool ASYNC, bool COMP, bool HOT, int VIA>
 __device__ __forceinline__ void pull_sweep(const PullArgs& a, const ApplyCtx& c, int cur, const uint32_t* sbm,
                                            const void* hot, unsigned int* ctr, LocalAcc& la) {
   typedef typename AppTraits<APP>::T T;
@@ -689,7 +695,7 @@ __device__ __forceinline__ void pull_sweep(const PullArgs& a, const ApplyCtx& c,
         const int64_t b = vb + static_cast<int64_t>(wu.y) * a.chunk;
         const int64_t e = ve < b + a.chunk ? ve : b + a.chunk;
         T acc = identity<APP>();
-        if constexpr (APP != K_INDEG) acc = warp_reduce_range<APP, ASYNC, COMP, HOT, COH>(a, src_val, src_con, b, e, lane, hot);
+        if constexpr (APP != K_INDEG) acc = warp_reduce_range<APP, ASYNC, COMP, HOT, VIA>(a, src_val, src_con, b, e, lane, hot);
         T* part = static_cast<T*>(a.partial) + H.z;
         bool last = H.y == 1;
         if (lane == 0) {
@@ -718,7 +724,7 @@ __device__ __forceinline__ void pull_sweep(const PullArgs& a, const ApplyCtx& c,
             if constexpr (is_pr<APP>()) fin = tot;
             else if constexpr (APP == K_INDEG) fin = static_cast<T>(ve - vb);
             else fin = combine<APP>(old, tot);
-            if (apply_vertex<APP>(c, v, fin, old, od, dst_val, dst_con, la) && !COH)
+            if (apply_vertex<APP>(c, v, fin, old, od, dst_val, dst_con, la) && VIA != VIA_PLAIN)
               atomicOr(a.bm + (v >> 5), 1u << (v & 31));
           }
         }
@@ -778,7 +784,7 @@ __device__ __forceinline__ void pull_sweep(const PullArgs& a, const ApplyCtx& c,
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                   const int64_t kk = q + e;
-                  x[e] = (kk >= E0 && kk < E1) ? edge_value<APP, ASYNC, HOT, COH>(a, src_val, src_con, cs[e], ws[e], hot)
+                  x[e] = (kk >= E0 && kk < E1) ? edge_value<APP, ASYNC, HOT, VIA>(a, src_val, src_con, cs[e], ws[e], hot)
                                                 : identity<APP>();
                 }
                 store4(buf + 4 * (lane + 32 * j), x);
@@ -828,7 +834,7 @@ __device__ __forceinline__ void pull_sweep(const PullArgs& a, const ApplyCtx& c,
 #pragma unroll
               for (int j = 0; j < 8; ++j) {
                 const int64_t kk = k + j;
-                vals[j] = (kk >= beg && kk < lend) ? edge_value<APP, ASYNC, HOT, COH>(a, src_val, src_con, cs[j], ws[j], hot)
+                vals[j] = (kk >= beg && kk < lend) ? edge_value<APP, ASYNC, HOT, VIA>(a, src_val, src_con, cs[j], ws[j], hot)
                                                    : identity<APP>();
               }
 #pragma unroll
@@ -856,7 +862,7 @@ __device__ __forceinline__ void pull_sweep(const PullArgs& a, const ApplyCtx& c,
               const int64_t bl = __shfl_sync(0xffffffffu, beg, sl);
               const int64_t el = __shfl_sync(0xffffffffu, end, sl);
               T r = identity<APP>();
-              if (l >= 0) r = group_reduce_range<APP, ASYNC, COMP, HOT, COH>(a, src_val, src_con, bl, el, gl, grp, hot);
+              if (l >= 0) r = group_reduce_range<APP, ASYNC, COMP, HOT, VIA>(a, src_val, src_con, bl, el, gl, grp, hot);
 #pragma unroll
               for (int g = 0; g < NG; ++g) {
                 const int lg = __shfl_sync(0xffffffffu, l, kGroupLanes * g);
@@ -870,7 +876,7 @@ __device__ __forceinline__ void pull_sweep(const PullArgs& a, const ApplyCtx& c,
             const int l = __ffs(m) - 1;
             const int64_t bl = __shfl_sync(0xffffffffu, beg, l);
             const int64_t el = __shfl_sync(0xffffffffu, end, l);
-            const T r = warp_reduce_range<APP, ASYNC, COMP, HOT, COH>(a, src_val, src_con, bl, el, lane, hot);
+            const T r = warp_reduce_range<APP, ASYNC, COMP, HOT, VIA>(a, src_val, src_con, bl, el, lane, hot);
             if (lane == l) acc = combine<APP>(acc, r);
           }
         }
@@ -880,7 +886,7 @@ __device__ __forceinline__ void pull_sweep(const PullArgs& a, const ApplyCtx& c,
         la.edges += end - beg;
         act = apply_vertex<APP>(c, v, acc, old, od, dst_val, dst_con, la);
       }
-      if constexpr (!COH) {
+      if constexpr (VIA != VIA_PLAIN) {
         const unsigned m = __ballot_sync(0xffffffffu, act);
         if (lane == 0) bitmap_set_tile(a.bm, vb, m);
       }
@@ -888,7 +894,10 @@ __device__ __forceinline__ void pull_sweep(const PullArgs& a, const ApplyCtx& c,
   }
 }
 
-template <int APP, bool EXACT, bool ASYNC = false, bool COMP = false, bool HOT = false>
+// VIA_ID is CC's first step from the ids as labels, in the caller's numbering:
+// the source ids are the candidates, and nothing is gathered (symmetric scale
+// 22, 128 M entries: 0.43 -> 0.25 ms).
+template <int APP, bool EXACT, bool ASYNC = false, bool COMP = false, bool HOT = false, int VIA = VIA_CONST>
 __global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLOCKS) pull_kernel(PullArgs a) {
   static_assert(!(HOT && ASYNC), "a Gauss-Seidel step changes the values the table would hold");
   constexpr int NW = pull_threads<HOT>() / 32;
@@ -924,7 +933,7 @@ __global__ void __launch_bounds__(pull_threads<HOT>(), HOT ? 1 : GX_PULL_MIN_BLO
                             ? ctl->shard_bm + static_cast<int64_t>(ctl->shard_cur) * ctl->shard_words
                             : nullptr;
   LocalAcc la;
-  pull_sweep<APP, EXACT, ASYNC, COMP, HOT, false>(a, c, cur, sbm, hot, a.ctr, la);
+  pull_sweep<APP, EXACT, ASYNC, COMP, HOT, VIA>(a, c, cur, sbm, hot, a.ctr, la);
   flush_block<NW>(ctl, la);
 }
 
@@ -1255,7 +1264,7 @@ __global__ void __launch_bounds__(kThreads, GX_PULL_MIN_BLOCKS) run_kernel(const
   for (int i = 0; i < kRunSteps && !done && !selective; ++i) {
     c.step = step;
     LocalAcc la;
-    pull_sweep<APP, false, false, false, false, true>(r.pull, c, cur, nullptr, nullptr, r.run->ctr[i], la);
+    pull_sweep<APP, false, false, false, false, VIA_PLAIN>(r.pull, c, cur, nullptr, nullptr, r.run->ctr[i], la);
     const unsigned long long x[5] = {warp_sum(la.changed), warp_sum(la.active), warp_sum(la.edges), warp_sum(la.resid),
                                      warp_sum(la.dangl)};
     if (lane == 0)
