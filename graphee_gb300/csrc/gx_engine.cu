@@ -764,11 +764,17 @@ gx_status build_shard_sets(gx_engine* e) {
 gx_status build_out_edges(gx_engine* e, bool weighted) {
   if (e->out_built && (!weighted || e->out_weighted)) return GX_OK;
   const int32_t V = e->V;
-  std::vector<int64_t> ooff(static_cast<size_t>(V) + 1, 0);
-  for (int32_t v = 0; v < V; ++v) ooff[v + 1] = ooff[v] + e->outdeg[v];
-  if (ooff[V] != e->E)
+  int64_t total = 0;
+  int negative = 0;
+#pragma omp parallel for reduction(+ : total) reduction(| : negative)
+  for (int32_t v = 0; v < V; ++v) {
+    total += e->outdeg[v];
+    negative |= e->outdeg[v] < 0;
+  }
+  if (negative) return fail(GX_ERR_FORMAT, "vertexout.npy holds a negative out-degree");
+  if (total != e->E)
     return fail(GX_ERR_FORMAT, "vertexout.npy sums to %lld out-edges but the shards hold %lld edges",
-                static_cast<long long>(ooff[V]), static_cast<long long>(e->E));
+                static_cast<long long>(total), static_cast<long long>(e->E));
   // Push frontier: one entry per kPushChunk out-edges of each vertex, so
   // V + E / kPushChunk + 1 entries hold any frontier.
   e->frontier_cap = static_cast<unsigned long long>(V) + static_cast<unsigned long long>(e->E) / kPushChunk + 1;
@@ -777,16 +783,28 @@ gx_status build_out_edges(gx_engine* e, bool weighted) {
   GX_TRY(dev_alloc(&e->d_ooff, static_cast<size_t>(V) + 1));
   GX_TRY(dev_alloc(&e->d_ocol, static_cast<size_t>(e->E) + 8));
   if (weighted) GX_TRY(dev_alloc(&e->d_ow, static_cast<size_t>(e->E) + 8));
-  unsigned long long* cursor = nullptr;
-  GX_TRY(dev_alloc(&cursor, static_cast<size_t>(V) + 1));
-  GX_CUDA(cudaMemcpy(e->d_ooff, ooff.data(), ooff.size() * sizeof(int64_t), cudaMemcpyHostToDevice));
-  GX_CUDA(cudaMemcpy(cursor, ooff.data(), ooff.size() * sizeof(int64_t), cudaMemcpyHostToDevice));
-  transpose_kernel<<<e->n_sm * 8, 256, 0, e->s_comp>>>(e->d_off, e->d_col, weighted ? e->d_w : nullptr, V, cursor,
-                                                        e->d_ocol, weighted ? e->d_ow : nullptr);
-  cudaError_t err = cudaGetLastError();
-  if (err == cudaSuccess) err = cudaStreamSynchronize(e->s_comp);
-  gx::pool_free(cursor);
-  if (err != cudaSuccess) return fail(GX_ERR_CUDA, "transpose: %s", cudaGetErrorString(err));
+  struct Scratch {
+    unsigned long long* p = nullptr;
+    ~Scratch() { dev_free(&p); }
+  } part, cursor;
+  int64_t hist_n = 0, part_n = 0;
+  radix_scratch_sizes(V, &hist_n, &part_n);
+  GX_TRY(dev_alloc(&part.p, static_cast<size_t>(part_n)));
+  GX_TRY(scan_u32(reinterpret_cast<const uint32_t*>(e->d_outdeg), V, reinterpret_cast<unsigned long long*>(e->d_ooff),
+                  part.p, e->s_comp));
+  store_i64_kernel<<<1, 1, 0, e->s_comp>>>(e->d_ooff + V, e->E);
+  gx_status st = GX_OK;
+  if (!transpose_by_buckets(e, weighted, &st)) {
+    // Few edges, too many for its tables, or no room for its copy.
+    GX_TRY(dev_alloc(&cursor.p, static_cast<size_t>(V) + 1));
+    GX_CUDA(cudaMemcpyAsync(cursor.p, e->d_ooff, sizeof(int64_t) * V, cudaMemcpyDeviceToDevice, e->s_comp));
+    transpose_kernel<<<e->n_sm * 8, 256, 0, e->s_comp>>>(e->d_off, e->d_col, weighted ? e->d_w : nullptr, V, cursor.p,
+                                                          e->d_ocol, weighted ? e->d_ow : nullptr);
+    cudaError_t err = cudaGetLastError();
+    if (err == cudaSuccess) err = cudaStreamSynchronize(e->s_comp);
+    if (err != cudaSuccess) return fail(GX_ERR_CUDA, "transpose: %s", cudaGetErrorString(err));
+  }
+  if (st != GX_OK) return st;
   e->out_built = true;
   e->out_weighted = weighted;
   return GX_OK;

@@ -87,3 +87,26 @@ def test_push_hubs(copies, relabel):
             assert np.array_equal(e.values(), ref)
             assert [e.iter_stats(i)["changed"] for i in range(st["iterations"])] == list(changed)
             assert st["push_iterations"] == st["iterations"]
+
+
+@pytest.mark.parametrize("relabel", [0, 1])
+def test_out_edges_by_buckets(relabel):
+    """Enough edges for the bucketed transpose: buckets of one slice and of several, hubs among sources and
+    destinations, a last bucket that is not full.  Weighted distances and labels depend on every out-edge."""
+    V, n = 5 * 16384 + 77, 5 << 20
+    rng = np.random.default_rng(4)
+    src = np.concatenate([rng.integers(0, V, n), np.repeat([0, 16383, 16384, V - 1], V), rng.integers(0, 16384, n // 4)])
+    dst = np.concatenate([rng.integers(0, V, n), np.tile(np.arange(V), 4), np.minimum(rng.integers(0, V, n // 4), 99)])
+    off, col = gx.build_csc(V, src, dst)
+    g = gx.Graph(V, off, col, None, 9)
+    g.weights = gx.edge_weights(2, g)
+    assert g.E > 4 << 20
+    a = (g.V, g.P, g.bounds, g.off, g.col, g.outdeg)
+    with gx.Engine(relabel=relabel, push_edge_fraction=1.0) as e:
+        e.load(g)
+        for source in (1, V - 2):
+            st = e.run(gx.APP_SSSP, 1000, source=source, weighted=True)
+            assert st["push_iterations"] == st["iterations"]
+            assert np.array_equal(e.values(), O.run(O.SSSP, *a, 1000, weights=g.weights, source=source)[0])
+        e.run(gx.APP_CC, 1000)
+        assert np.array_equal(e.values(), O.run(O.CC, *a, 1000)[0])
