@@ -610,9 +610,10 @@ gx_status encode_streamed(gx_engine* e, const int32_t* col) {
 // Streamed shards side by side travel and are swept together up to this many
 // edges, resident ones up to twice as many: a launch of one small shard lasts
 // some 30 us, whatever it holds, and a copy of 2 MB half as long as its calls.
-// (Scale 24 in 256 shards, half of them streamed: 7.5 ms a superstep a shard at
-// a time, 3.8 in groups of 4 M edges, 2.6 of them copies.)
-constexpr int64_t kStreamGroup = int64_t(4) << 20;
+// Scale 24 in 256 shards, half of them streamed, a superstep: a shard at a time
+// 7.5 ms, groups of 1 M edges 6.0, 2 M 4.6, 4 M 3.5, 8 M 3.0, 16 M 3.0, of
+// which the link takes 2.6.
+constexpr int64_t kStreamGroup = int64_t(8) << 20;
 
 // Decides which shards stay in HBM under the budget (in shard order, like the
 // reference's insert-until-full edge cache, Global.h:170-244), uploads them,
