@@ -156,18 +156,23 @@ __device__ __forceinline__ BatchIds<WIDE> batch_load(const void* ids, int64_t ro
   else r.x = __ldcs(static_cast<const uint2*>(ids) + round * 32 + lane);
   return r;
 }
-template <bool PR, bool WIDE, bool FULL>
-__device__ __forceinline__ void batch_fold4(const BatchIds<WIDE>& c, const uint32_t* tab, int tn, const uint32_t* g,
-                                            float& f, int32_t& m) {
+template <bool WIDE, bool FULL>
+__device__ __forceinline__ void batch_gather4(const BatchIds<WIDE>& c, const uint32_t* tab, int tn, const uint32_t* g,
+                                              uint32_t (&v)[4]) {
   uint32_t id[4];
   if constexpr (WIDE) {
     id[0] = c.x.x, id[1] = c.x.y, id[2] = c.x.z, id[3] = c.x.w;
   } else {
     id[0] = c.x.x & 0xffffu, id[1] = c.x.x >> 16, id[2] = c.x.y & 0xffffu, id[3] = c.x.y >> 16;
   }
-  uint32_t v[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) v[j] = batch_gather<FULL>(tab, tn, g, static_cast<int32_t>(id[j]));
+}
+template <bool PR, bool WIDE, bool FULL>
+__device__ __forceinline__ void batch_fold4(const BatchIds<WIDE>& c, const uint32_t* tab, int tn, const uint32_t* g,
+                                            float& f, int32_t& m) {
+  uint32_t v[4];
+  batch_gather4<WIDE, FULL>(c, tab, tn, g, v);
 #pragma unroll
   for (int j = 0; j < 4; ++j) batch_fold<PR>(v[j], f, m);
 }
@@ -182,8 +187,13 @@ __device__ __forceinline__ void batch_rounds(const void* ids, int64_t at, int n,
     BatchIds<WIDE> c[F];
 #pragma unroll
     for (int j = 0; j < F; ++j) c[j] = batch_load<WIDE>(ids, at + r + j, lane);
+    uint32_t v[F][4];  // every round's gathers in flight, then their folds in order
 #pragma unroll
-    for (int j = 0; j < F; ++j) batch_fold4<PR, WIDE, FULL>(c[j], tab, tn, g, f, m);
+    for (int j = 0; j < F; ++j) batch_gather4<WIDE, FULL>(c[j], tab, tn, g, v[j]);
+#pragma unroll
+    for (int j = 0; j < F; ++j)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) batch_fold<PR>(v[j][k], f, m);
   }
   if (r < n) {
     BatchIds<WIDE> c[F - 1];
