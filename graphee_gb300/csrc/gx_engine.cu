@@ -96,15 +96,31 @@ static void touch_host_pages(void* p, size_t bytes) {
   for (int64_t i = 0; i < n; ++i) *reinterpret_cast<volatile unsigned char*>(b + static_cast<uintptr_t>(i) * page) = 0;
 }
 
+// The engine's pinned pieces, from the first large result on; false when the
+// host has no memory for them.
+static bool stage_slots(gx_engine* e) {
+  if (e->h_stage) return true;
+  cudaError_t err = cudaSuccess;
+  for (cudaEvent_t& ev : e->stage_ready)
+    if (!ev && err == cudaSuccess) err = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+  if (err == cudaSuccess)
+    err = cudaHostAlloc(reinterpret_cast<void**>(&e->h_stage), kStageSlots * kStageBytes, cudaHostAllocDefault);
+  if (err == cudaSuccess) return true;
+  cudaGetLastError();
+  e->h_stage = nullptr;
+  return false;
+}
+
 gx_status copy_to_host(gx_engine* e, void* dst, const void* src, size_t bytes) {
-  if (bytes < kStageFrom) {
-    touch_host_pages(dst, bytes);
+  // Only the caller's pageable memory gains by the host's hands: memory that
+  // CUDA knows (pinned, managed, a device's) is the copy's own business.
+  cudaPointerAttributes at;
+  const bool known = cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type != cudaMemoryTypeUnregistered;
+  if (known) cudaGetLastError();
+  if (!known && bytes < kStageFrom) touch_host_pages(dst, bytes);
+  if (known || bytes < kStageFrom || !stage_slots(e)) {
     GX_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost));
     return GX_OK;
-  }
-  if (!e->h_stage) {
-    GX_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&e->h_stage), kStageSlots * kStageBytes, cudaHostAllocDefault));
-    for (cudaEvent_t& ev : e->stage_ready) GX_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   }
   const size_t n = (bytes + kStageBytes - 1) / kStageBytes;
   auto part = [&](size_t i) { return std::min(kStageBytes, bytes - i * kStageBytes); };
@@ -236,6 +252,20 @@ gx_status values_to_caller(gx_engine* e, const void* d_vals, cudaStream_t s) {
   GX_CUDA(cudaGetLastError());
   GX_CUDA(cudaStreamSynchronize(s));
   return GX_OK;
+}
+
+// run_kernel's scratch (60 KB) and the records' landing place, from the first
+// run on; false without room for them: such a run's steps are launched singly.
+bool run_scratch(gx_engine* e) {
+  if (!e->d_run && dev_alloc(&e->d_run, 1) != GX_OK) return false;
+  if (!e->h_run_stats &&
+      cudaHostAlloc(reinterpret_cast<void**>(&e->h_run_stats), sizeof(StepStats) * kRunSteps, cudaHostAllocDefault) !=
+          cudaSuccess) {
+    cudaGetLastError();
+    e->h_run_stats = nullptr;
+    return false;
+  }
+  return true;
 }
 
 gx_status alloc_ctl(gx_engine* e) {
@@ -1093,10 +1123,8 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
       // the dense supersteps in run_kernel, at every size (per superstep, from
       // the replayed launches: 1000 vertices 14.6 -> 7.8 us, 1 M 98 -> 91, 7 M
       // 457 -> 454, 67 M 4.17 -> 4.15 ms).
-      if (e->cfg.use_graph && !prof && !every && !e->cfg.exact_order && pa.hot_n == 0 && c.mark_mode == MARK_NONE) {
-        if (!e->d_run) GX_TRY(dev_alloc(&e->d_run, 1));
-        if (!e->h_run_stats)
-          GX_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&e->h_run_stats), sizeof(StepStats) * kRunSteps, cudaHostAllocDefault));
+      if (e->cfg.use_graph && !prof && !every && !e->cfg.exact_order && pa.hot_n == 0 && c.mark_mode == MARK_NONE &&
+          run_scratch(e)) {
         RunArgs ra;
         memset(&ra, 0, sizeof(ra));
         ra.pull = pa;
