@@ -323,33 +323,42 @@ constexpr int kMinChunk = 256;     // shortest: one round of warp_reduce_range
 #define GX_LANE_MAX 16
 #endif
 constexpr int kLaneMaxDegree = GX_LANE_MAX;  // longest list a lane walks alone
-// Units a warp claims per atomic.  The next claim is issued before this one's
-// units are swept, so only its count matters: at 7 M vertices a superstep
-// takes 0.467 ms with 2, 0.477 with 3, 0.479 with 1.
-constexpr int kGrab = 2;
+// Units a warp claims per atomic, when it has swept the last: a claim issued
+// ahead holds units that others could sweep (7 M vertices, a run of standard
+// PageRank: 7.98 ms with it, 7.67 without).  Claims of 1, 2, 3 and 4: 7 M
+// vertices 8.25, 7.70, 7.64 and 7.74 ms, 67 M (20 supersteps) 84.2, 80.0, 79.4
+// and 79.0, 1 M 1.61, 1.55, 1.55 and 1.60.
+constexpr int kGrab = 3;
 // PageRank loads a tile's offsets, old values and out-degrees a unit ahead
 // (0.467 -> 0.457 ms at 7 M vertices); the min apps, a register short of
 // holding them, lose by it (weighted SSSP at scale 24: 6.45 -> 6.54 ms).
 template <int APP> constexpr bool tile_prefetch() { return is_pr<APP>(); }
-constexpr int kQueues = 64;          // work-unit cursors per launch
+// Work-unit cursors per launch, at most 32.  Neighbouring vertices share
+// sources, so the fewer places the graph is swept at, the more gathers meet in
+// L1 and L2, until the claims wait for each other: 64, 16, 8, 6 and 4 cursors,
+// 20 supersteps at 1 M vertices 1.81, 1.70, 1.62, 1.61 and 1.65 ms, 7 M
+// (standard) 7.94, 7.95, 7.73, 7.67 and 7.73, 17 M 20.1, 19.9, 19.5, 19.5 and
+// 19.6.  (A cursor per SM or CTA instead: +8 to 13 %, -1 to +2 %.)
+constexpr int kQueues = 6;
 // A cursor to a 128-byte line: atomics on one line are served one after the
-// other.  With the 64 cursors in two lines single-unit claims set the time of
-// a launch: 16 M edges, 0.139 -> 0.099 ms a superstep.
+// other.  (64 cursors in two lines, one unit to a claim: 16 M edges took 0.139
+// ms a superstep, 0.099 with a line each.)
 constexpr int kQueueStride = 32;
 
 // How a graph of E edges is cut for a GPU that holds `warps` pull warps.  A
 // unit is a serial chain of loads, and a launch is never shorter than its
-// longest unit: the caps shrink until every warp has about four units, down
+// longest unit: the caps shrink until every warp has about three units, down
 // to one round of a warp's loads, and reach their full size (2048-edge tiles
-// and chunks, 4096-edge lists whole) at 40 M edges.  Measured per superstep
-// (two claimed at once): 16 M edges 0.099 ms with 4 units a warp, 0.111 with
-// 2, 0.104 with 6 and 8; 0.128 with the full-size caps and four claimed at
-// once.  A graph of 1000 vertices: 34 -> 14 us.
+// and chunks, 4096-edge lists whole) at 30 M edges.  20 supersteps with 2, 3,
+// 4, 6 and 8 units a warp: 1 M vertices (16 M edges) 1.62, 1.57, 1.62, 1.77 and
+// 1.83 ms; 0.5 M 0.99, 0.99 and 1.09 with 2, 3 and 4; 2 M 2.62, 2.62 and 2.59.
+// With the full-size caps 1 M vertices took 2.8 ms and 1000 vertices 34
+// instead of 14 us a superstep.
 struct UnitCaps {
   int32_t tile, chunk, heavy;
 };
 inline UnitCaps unit_caps(int64_t E, int64_t warps, int32_t tile_edges, int32_t heavy_degree) {
-  const int64_t even = E / (4 * (warps > 0 ? warps : 1));
+  const int64_t even = E / (3 * (warps > 0 ? warps : 1));
   const int64_t most = tile_edges > 32 ? tile_edges : 32;
   UnitCaps c;
   c.tile = static_cast<int32_t>(even < 64 ? (most < 64 ? most : 64) : even < most ? even : most);
@@ -381,21 +390,15 @@ inline PullShape pull_shape(int64_t U, int grid, int threads) {
 // Returns the first queue after q (cyclically) whose cursor is below its
 // size, reading every cursor in one round trip, or -1 when all are drained.
 __device__ __forceinline__ int next_queue(const unsigned int* ctr, int q, int nq, int64_t U, int lane) {
-  bool ok0 = false, ok1 = false;
+  bool ok = false;
   if (lane < nq) {
     const int64_t size = (U * (lane + 1)) / nq - (U * lane) / nq;
-    ok0 = static_cast<int64_t>(*reinterpret_cast<const volatile unsigned int*>(ctr + lane * kQueueStride)) < size;
+    ok = static_cast<int64_t>(*reinterpret_cast<const volatile unsigned int*>(ctr + lane * kQueueStride)) < size;
   }
-  if (lane + 32 < nq) {
-    const int j = lane + 32;
-    const int64_t size = (U * (j + 1)) / nq - (U * j) / nq;
-    ok1 = static_cast<int64_t>(*reinterpret_cast<const volatile unsigned int*>(ctr + j * kQueueStride)) < size;
-  }
-  const unsigned long long left = static_cast<unsigned long long>(__ballot_sync(0xffffffffu, ok0)) |
-                                  (static_cast<unsigned long long>(__ballot_sync(0xffffffffu, ok1)) << 32);
+  const unsigned left = __ballot_sync(0xffffffffu, ok);
   if (!left) return -1;
-  const unsigned long long after = q + 1 < 64 ? (left >> (q + 1)) << (q + 1) : 0ull;
-  return __ffsll(static_cast<long long>(after ? after : left)) - 1;
+  const unsigned after = left & (0xffffffffu << q << 1);
+  return __ffs(static_cast<int>(after ? after : left)) - 1;
 }
 
 template <class T>
@@ -628,9 +631,9 @@ __device__ __forceinline__ void pull_sweep(const PullArgs& a, const ApplyCtx& c,
   if (a.grab) {
     qb = a.u_begin + static_cast<int>((static_cast<int64_t>(U) * q) / nq);
     qe = a.u_begin + static_cast<int>((static_cast<int64_t>(U) * (q + 1)) / nq);
-    if (lane == 0) claim = static_cast<int>(atomicAdd(ctr + q * kQueueStride, static_cast<unsigned>(a.grab)));
   }
   for (;;) {
+    if (a.grab && lane == 0) claim = static_cast<int>(atomicAdd(ctr + q * kQueueStride, static_cast<unsigned>(a.grab)));
     const int u0 = qb + __shfl_sync(0xffffffffu, claim, 0);
     int cnt = 1;
     if (a.grab == 0) {  // at most as many units as warps
@@ -642,11 +645,9 @@ __device__ __forceinline__ void pull_sweep(const PullArgs& a, const ApplyCtx& c,
         if (q < 0) break;
         qb = a.u_begin + static_cast<int>((static_cast<int64_t>(U) * q) / nq);
         qe = a.u_begin + static_cast<int>((static_cast<int64_t>(U) * (q + 1)) / nq);
-        if (lane == 0) claim = static_cast<int>(atomicAdd(ctr + q * kQueueStride, static_cast<unsigned>(a.grab)));
         continue;
       }
       cnt = qe - u0 < a.grab ? qe - u0 : a.grab;
-      if (lane == 0) claim = static_cast<int>(atomicAdd(ctr + q * kQueueStride, static_cast<unsigned>(a.grab)));
     }
     // One coalesced load for the batch's descriptors.
     int2 myu = make_int2(0, 0);
