@@ -1120,9 +1120,10 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
     int32_t run_launches = 0;
     if constexpr (is_pr<APP>()) {
       // Default-mode PageRank whose selective steps have nothing to mark yet:
-      // the dense supersteps in run_kernel, at every size (per superstep, from
-      // the replayed launches: 1000 vertices 14.6 -> 7.8 us, 1 M 98 -> 91, 7 M
-      // 457 -> 454, 67 M 4.17 -> 4.15 ms).
+      // the dense supersteps in run_kernel, at every size (a superstep against
+      // the replayed launches': 1000 vertices 7.8 for 14.6 us, 1 M 7 us less,
+      // 7 M 3, 67 M 20).  SSSP and CC keep the launches: with pull, push and
+      // finalize in one such kernel they took 3 to 17 % longer.
       if (e->cfg.use_graph && !prof && !every && !e->cfg.exact_order && pa.hot_n == 0 && c.mark_mode == MARK_NONE &&
           run_scratch(e)) {
         RunArgs ra;

@@ -1,8 +1,10 @@
 // Device kernels of the superstep loop (GraphPS<T>::run,
 // GraphMP/system/GraphPS.h:256-386) for one GB300.
 //
-// One superstep is three launches that read a device control block, so a
-// run of K supersteps can be replayed as one CUDA graph with no host sync:
+// PageRank's dense supersteps run up to 64 to one cooperative launch
+// (run_kernel).  Any other superstep is three launches that read a device
+// control block, so a run of K supersteps can be replayed as one CUDA graph
+// with no host sync:
 //   pull_kernel<APP>      gather-apply over in-edges (CSC) of the swept shards
 //   push_kernel<APP>      sparse min-plus / min-label over out-edges of the frontier
 //   finalize_kernel<APP>  step statistics, frontier compaction, shard activation,
@@ -330,8 +332,8 @@ constexpr int kLaneMaxDegree = GX_LANE_MAX;  // longest list a lane walks alone
 // and 79.0, 1 M 1.61, 1.55, 1.55 and 1.60.
 constexpr int kGrab = 3;
 // PageRank loads a tile's offsets, old values and out-degrees a unit ahead
-// (0.467 -> 0.457 ms at 7 M vertices); the min apps, a register short of
-// holding them, lose by it (weighted SSSP at scale 24: 6.45 -> 6.54 ms).
+// (17 M vertices, 20 supersteps: 19.50 -> 19.31 ms); the min apps, a register
+// short of holding them, lose by it (weighted SSSP there: 5.62 -> 5.69 ms).
 template <int APP> constexpr bool tile_prefetch() { return is_pr<APP>(); }
 // Work-unit cursors per launch, at most 32.  Neighbouring vertices share
 // sources, so the fewer places the graph is swept at, the more gathers meet in

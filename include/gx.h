@@ -78,7 +78,7 @@ typedef struct gx_config {
   uint32_t wait_limit;         /* polls (each of at least 64 ns) a device-side wait makes before it gives
                                   up and the call returns GX_ERR_TIMEOUT; bounds the CTA-team barrier
                                   of gx_batch_run and the grid barrier of gx_ppr (default 1<<24, over
-                                  a second) */
+                                  a second); gx_run's grid barrier (PageRank) makes at least 1<<24 */
   int32_t verbose;             /* per-iteration log lines on stderr (default 0) */
   int32_t profile;             /* time every pull launch with CUDA events (default 0) */
   int32_t compress_cache;      /* with a budget the plain shards exceed: keep every shard compressed
