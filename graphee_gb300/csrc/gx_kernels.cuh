@@ -15,6 +15,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 namespace gx {
 
 enum AppKind : int { K_PR_REF = 0, K_PR_STD = 1, K_SSSP_UNIT = 2, K_SSSP_W = 3, K_CC = 4, K_INDEG = 5 };
@@ -319,7 +321,7 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long x) {
 // memory and each lane folds its own slice; no vertex is chunked.
 // Results are deterministic run to run in both modes.
 // ---------------------------------------------------------------------------
-constexpr int kHeavyChunk = 2048;  // longest heavy chunk
+constexpr int kHeavyChunk = 4096;  // longest heavy chunk
 constexpr int kMinChunk = 256;     // shortest: one round of warp_reduce_range
 #ifndef GX_LANE_MAX
 #define GX_LANE_MAX 16
@@ -351,9 +353,14 @@ constexpr int kQueueStride = 32;
 // unit is a serial chain of loads, and a launch is never shorter than its
 // longest unit: the caps shrink until every warp has about three units, down
 // to one round of a warp's loads, and reach their full size (2048-edge tiles
-// and chunks, 4096-edge lists whole) at 30 M edges.  20 supersteps with 2, 3,
+// at 30 M edges, chunks of 4096 at 60 M).  20 supersteps with 2, 3,
 // 4, 6 and 8 units a warp: 1 M vertices (16 M edges) 1.62, 1.57, 1.62, 1.77 and
 // 1.83 ms; 0.5 M 0.99, 0.99 and 1.09 with 2, 3 and 4; 2 M 2.62, 2.62 and 2.59.
+// Chunks of 2048, 4096 and 8192 at most: 7 M vertices (standard) 7.66, 7.58 and
+// 7.86 ms, 17 M relabelled 17.8, 17.3 and 17.7, 67 M relabelled 79.4, 77.8 and
+// 77.7, weighted SSSP at 17 M 5.59, 5.59 and 5.78: a chunk starts with loads
+// that nothing overlaps, and a launch ends with the last one.  Tiles of 1024
+// instead of 2048 edges: 8.03 (7 M), 20.4 (17 M), 87.0 (67 M).
 // With the full-size caps 1 M vertices took 2.8 ms and 1000 vertices 34
 // instead of 14 us a superstep.
 struct UnitCaps {
@@ -364,7 +371,7 @@ inline UnitCaps unit_caps(int64_t E, int64_t warps, int32_t tile_edges, int32_t 
   const int64_t most = tile_edges > 32 ? tile_edges : 32;
   UnitCaps c;
   c.tile = static_cast<int32_t>(even < 64 ? (most < 64 ? most : 64) : even < most ? even : most);
-  const int64_t ch = (static_cast<int64_t>(c.tile) + kMinChunk - 1) / kMinChunk * kMinChunk;
+  const int64_t ch = (std::max(even, static_cast<int64_t>(c.tile)) + kMinChunk - 1) / kMinChunk * kMinChunk;
   c.chunk = static_cast<int32_t>(ch < kHeavyChunk ? ch : kHeavyChunk);
   const int32_t own = heavy_degree > 32 ? heavy_degree : 32;
   c.heavy = own < 2 * c.chunk ? own : 2 * c.chunk;
