@@ -888,12 +888,14 @@ gx_status batch_launch(gx_engine* e, BatchDev& d, BatchArgs& a, const gx_batch_t
   GX_CUDA(cudaGetLastError());
   cudaGraph_t graph;
   cudaGraphExec_t exec;
+  std::unique_lock<std::shared_mutex> capturing(capture_mutex());
   GX_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   cudaMemsetAsync(a.ctr, 0, sizeof(unsigned int), s);
   cudaMemsetAsync(a.team, 0, sizeof(unsigned int) * 4 * static_cast<size_t>(a.n_inst), s);
   cudaMemsetAsync(a.abort, 0, sizeof(unsigned int), s);
   batch_kernel<<<blocks, t.threads, smem, s>>>(a);
   GX_CUDA(cudaStreamEndCapture(s, &graph));
+  capturing.unlock();
   cudaError_t err = cudaGraphInstantiate(&exec, graph, 0);
   cudaGraphDestroy(graph);
   if (err != cudaSuccess) return fail(GX_ERR_CUDA, "gx_batch: graph instantiate: %s", cudaGetErrorString(err));

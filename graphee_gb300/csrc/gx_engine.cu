@@ -46,6 +46,11 @@ int current_device() {
   return d;
 }
 
+std::shared_mutex& capture_mutex() {
+  static std::shared_mutex mu;
+  return mu;
+}
+
 static std::mutex g_pool_mu;
 static DevicePool g_pools[64];
 static bool g_pool_tried[64];
@@ -1186,6 +1191,7 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
       if (!x) {
         const int32_t counted = launches;
         cudaGraph_t graph;
+        std::unique_lock<std::shared_mutex> capturing(capture_mutex());
         GX_CUDA(cudaStreamBeginCapture(e->s_comp, cudaStreamCaptureModeThreadLocal));
         for (int i = 0; i < K; ++i) {
           gx_status st = enqueue(i);
@@ -1195,6 +1201,7 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
           }
         }
         GX_CUDA(cudaStreamEndCapture(e->s_comp, &graph));
+        capturing.unlock();
         cudaError_t err = cudaGraphInstantiate(&x, graph, 0);
         cudaGraphDestroy(graph);
         if (err != cudaSuccess) return fail(GX_ERR_CUDA, "cudaGraphInstantiate: %s", cudaGetErrorString(err));

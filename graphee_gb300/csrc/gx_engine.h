@@ -5,6 +5,8 @@
 
 #include <cstring>
 #include <memory>
+#include <mutex>
+#include <shared_mutex>
 #include <utility>
 #include <vector>
 
@@ -48,6 +50,12 @@ inline cudaError_t pool_malloc(void** p, size_t bytes) {
   return err;
 }
 
+// Held, exclusively, while a stream is captured, and, shared, during a wait for
+// the whole device: the two must not meet, whichever threads and engines they
+// are of.  (Such a wait would cover the captured stream, which CUDA does not
+// allow; with two threads it crashed inside the driver.)
+std::shared_mutex& capture_mutex();
+
 // Frees a block of the pool once no work on the device can still use it
 // (a pool block is never freed with cudaFree, which neither waits for that
 // work nor goes through the pool's bookkeeping).
@@ -58,7 +66,10 @@ inline void pool_free(void* p) {
     cudaFree(p);
     return;
   }
-  cudaDeviceSynchronize();
+  {
+    std::shared_lock<std::shared_mutex> no_capture(capture_mutex());
+    cudaDeviceSynchronize();
+  }
   cudaFreeAsync(p, dp->stream);
   cudaStreamSynchronize(dp->stream);
 }

@@ -422,9 +422,11 @@ extern "C" gx_status gx_ppr(gx_engine* e, int32_t k, const int32_t* sources, int
   };
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
+  std::unique_lock<std::shared_mutex> capturing(capture_mutex());
   GX_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   cudaError_t cap_err = enqueue();
   cudaError_t end_err = cudaStreamEndCapture(s, &graph);
+  capturing.unlock();
   if (cap_err != cudaSuccess || end_err != cudaSuccess) {
     if (graph) cudaGraphDestroy(graph);
     return fail(GX_ERR_CUDA, "gx_ppr: capture: %s", cudaGetErrorString(cap_err != cudaSuccess ? cap_err : end_err));
