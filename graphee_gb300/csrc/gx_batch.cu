@@ -845,7 +845,7 @@ gx_status batch_launch(gx_engine* e, BatchDev& d, BatchArgs& a, const gx_batch_t
   int smem = 0;
   GX_TRY(batch_table_bytes(e, t, &smem));
   a.tab = smem / 4;
-  GX_CUDA(cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  GX_CUDA(allow_dynamic_smem(e->dev, reinterpret_cast<const void*>(batch_kernel)));
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel, t.threads, smem);
   if (per_sm < 1) return fail(GX_ERR_INVALID, "gx_batch: %d threads per CTA do not fit an SM", t.threads);
   const int blocks = std::min(per_sm, t.ctas_per_sm) * e->n_sm;

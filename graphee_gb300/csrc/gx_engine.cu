@@ -1036,8 +1036,7 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
       const int64_t n = std::min<int64_t>({static_cast<int64_t>(e->cfg.hot_vertices), V, cap}) & ~int64_t(3);
       if (n > 0) {
         hot_smem = static_cast<size_t>(n) * sizeof(T);
-        GX_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(hk), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(hot_smem)));
+        GX_CUDA(allow_dynamic_smem(e->dev, reinterpret_cast<const void*>(hk)));
         int per_sm = 0;
         GX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void*>(hk), kHotThreads,
                                                               hot_smem));

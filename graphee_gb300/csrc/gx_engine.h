@@ -96,6 +96,22 @@ void dev_free(T** p) {
   *p = nullptr;
 }
 
+// Lets launches of fn have all the dynamic shared memory that a CTA can have.
+// The limit belongs to the function in its context, not to a call: engines on
+// other threads rely on it too, so every call sets this one value, never its
+// own launch's size, which a smaller one set between here and the launch would
+// make fail.  (What a launch asks for decides its occupancy, not the limit.)
+inline cudaError_t allow_dynamic_smem(int dev, const void* fn) {
+  cudaFuncAttributes attr{};
+  int most = 0;
+  cudaError_t err = cudaFuncGetAttributes(&attr, fn);
+  if (err == cudaSuccess) err = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (err == cudaSuccess)
+    err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               most - static_cast<int>(attr.sharedSizeBytes));
+  return err;
+}
+
 // std::vector storage without value-initialisation: large host arrays are
 // filled by parallel loops, which also place their pages.
 template <class T>

@@ -518,8 +518,8 @@ extern "C" gx_status gx_triangle_count(gx_engine* e, uint64_t* total, gx_run_sta
   const int fit = std::max(1, (220 * 1024) / (smem_cta + 2048));
   void (*cta)(TcArgs) = fit >= 6 ? tc_cta_kernel<256> : fit >= 2 ? tc_cta_kernel<512> : tc_cta_kernel<1024>;
   const int cta_threads = fit >= 6 ? 256 : fit >= 2 ? 512 : 1024;
-  GX_CUDA(cudaFuncSetAttribute(cta, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_cta));
-  GX_CUDA(cudaFuncSetAttribute(tc_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_warp));
+  GX_CUDA(allow_dynamic_smem(e->dev, reinterpret_cast<const void*>(cta)));
+  GX_CUDA(allow_dynamic_smem(e->dev, reinterpret_cast<const void*>(tc_warp_kernel)));
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cta, cta_threads, smem_cta);
   cta<<<std::max(1, per_sm) * e->n_sm, cta_threads, smem_cta, e->s_copy>>>(a);
   GX_CUDA(cudaGetLastError());

@@ -226,8 +226,8 @@ bool transpose_by_buckets(gx_engine* e, bool weighted, gx_status* status) {
     GX_CUDA(cudaMemsetAsync(a.ctr, 0, 4, s));
     // Batches of about 64 units, fewer where that would leave SMs without.
     const int smem_b = 12 * nb, smem_p = 4 * kBucket;
-    GX_CUDA(cudaFuncSetAttribute(tr_bucket_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_b));
-    GX_CUDA(cudaFuncSetAttribute(tr_place_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_p));
+    GX_CUDA(allow_dynamic_smem(e->dev, reinterpret_cast<const void*>(tr_bucket_kernel)));
+    GX_CUDA(allow_dynamic_smem(e->dev, reinterpret_cast<const void*>(tr_place_kernel)));
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tr_bucket_kernel, kTrThreads, smem_b);
     const int grid = std::max(1, per_sm) * e->n_sm;
