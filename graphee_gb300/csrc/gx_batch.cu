@@ -886,24 +886,33 @@ gx_status batch_launch(gx_engine* e, BatchDev& d, BatchArgs& a, const gx_batch_t
   GX_CUDA(cudaMemcpyAsync(d.round_base, base.data(), sizeof(unsigned long long) * a.n_inst, cudaMemcpyHostToDevice, s));
   batch_fill_kernel<<<std::min(a.n_inst, e->n_sm) * kFillSplit, 256, 0, s>>>(a);
   GX_CUDA(cudaGetLastError());
-  cudaGraph_t graph;
-  cudaGraphExec_t exec;
+  // Every status counts: a graph that lacks the kernel would end well, with
+  // the results as the memory happened to be.
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t exec = nullptr;
   std::unique_lock<std::shared_mutex> capturing(capture_mutex());
   GX_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-  cudaMemsetAsync(a.ctr, 0, sizeof(unsigned int), s);
-  cudaMemsetAsync(a.team, 0, sizeof(unsigned int) * 4 * static_cast<size_t>(a.n_inst), s);
-  cudaMemsetAsync(a.abort, 0, sizeof(unsigned int), s);
-  batch_kernel<<<blocks, t.threads, smem, s>>>(a);
-  GX_CUDA(cudaStreamEndCapture(s, &graph));
+  cudaError_t err = cudaMemsetAsync(a.ctr, 0, sizeof(unsigned int), s);
+  if (err == cudaSuccess) err = cudaMemsetAsync(a.team, 0, sizeof(unsigned int) * 4 * static_cast<size_t>(a.n_inst), s);
+  if (err == cudaSuccess) err = cudaMemsetAsync(a.abort, 0, sizeof(unsigned int), s);
+  if (err == cudaSuccess) {
+    batch_kernel<<<blocks, t.threads, smem, s>>>(a);
+    err = cudaGetLastError();
+  }
+  const cudaError_t end_err = cudaStreamEndCapture(s, &graph);
   capturing.unlock();
-  cudaError_t err = cudaGraphInstantiate(&exec, graph, 0);
-  cudaGraphDestroy(graph);
-  if (err != cudaSuccess) return fail(GX_ERR_CUDA, "gx_batch: graph instantiate: %s", cudaGetErrorString(err));
-  cudaGraphLaunch(exec, s);
-  cudaEventRecord(e1, s);
-  err = cudaEventSynchronize(e1);
+  if (err == cudaSuccess) err = end_err;
+  if (err == cudaSuccess) err = cudaGraphInstantiate(&exec, graph, 0);
+  if (graph) cudaGraphDestroy(graph);
+  if (err != cudaSuccess) {
+    cudaGetLastError();
+    return fail(GX_ERR_CUDA, "gx_batch: launch: %s", cudaGetErrorString(err));
+  }
+  err = cudaGraphLaunch(exec, s);
+  if (err == cudaSuccess) err = cudaEventRecord(e1, s);
+  if (err == cudaSuccess) err = cudaEventSynchronize(e1);
   float t_ms = 0;
-  cudaEventElapsedTime(&t_ms, e0, e1);
+  if (err == cudaSuccess) cudaEventElapsedTime(&t_ms, e0, e1);
   cudaGraphExecDestroy(exec);
   if (err != cudaSuccess) return fail(GX_ERR_CUDA, "gx_batch: run failed: %s", cudaGetErrorString(err));
   unsigned int aborted = 0;
