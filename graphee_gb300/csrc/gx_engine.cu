@@ -1499,7 +1499,7 @@ void gx_config_default(gx_config* cfg) {
   cfg->stream_slots = 4;
   cfg->copy_streams = 1;
   cfg->selective_threshold = 0.001;
-  cfg->heavy_degree = 4096;
+  cfg->heavy_degree = kHeavyDegree;
   cfg->tile_edges = 2048;
   cfg->exact_order = 0;
   cfg->push_sparse = 1;

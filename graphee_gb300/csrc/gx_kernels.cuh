@@ -363,6 +363,9 @@ constexpr int kQueueStride = 32;
 // instead of 2048 edges: 8.03 (7 M), 20.4 (17 M), 87.0 (67 M).
 // With the full-size caps 1 M vertices took 2.8 ms and 1000 vertices 34
 // instead of 14 us a superstep.
+// A heavy_degree above the default is the caller's own and holds at every size;
+// the default, and less, shrinks with the chunks.
+constexpr int32_t kHeavyDegree = 4096;
 struct UnitCaps {
   int32_t tile, chunk, heavy;
 };
@@ -374,7 +377,7 @@ inline UnitCaps unit_caps(int64_t E, int64_t warps, int32_t tile_edges, int32_t 
   const int64_t ch = (std::max(even, static_cast<int64_t>(c.tile)) + kMinChunk - 1) / kMinChunk * kMinChunk;
   c.chunk = static_cast<int32_t>(ch < kHeavyChunk ? ch : kHeavyChunk);
   const int32_t own = heavy_degree > 32 ? heavy_degree : 32;
-  c.heavy = own < 2 * c.chunk ? own : 2 * c.chunk;
+  c.heavy = own > kHeavyDegree || own < 2 * c.chunk ? own : 2 * c.chunk;
   return c;
 }
 

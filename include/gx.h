@@ -67,7 +67,8 @@ typedef struct gx_config {
   double selective_threshold;  /* BF_THRE (GraphMP/system/Global.h:57), default 0.001 */
   int32_t heavy_degree;        /* in-degree above which a vertex gets its own warp units, split
                                   into chunks of at most 4096 edges (default 4096, minimum 32;
-                                  graphs below 60 M edges use smaller bounds, down to 512 and 256) */
+                                  graphs below 60 M edges use smaller chunks, down to 256, and
+                                  bounds, down to 512, unless this is above 4096) */
   int32_t tile_edges;          /* most edges of one warp tile (default 2048; graphs below 30 M
                                   edges use smaller tiles, down to 64) */
   int32_t exact_order;         /* 1: fold every vertex's in-edges in edge order, as the reference's
