@@ -413,6 +413,10 @@ namespace gx {
 // are slower that way: 64 MB takes a plain copy 0.4 ms, the pieces 1.1.)
 gx_status copy_to_host(gx_engine* e, void* dst, const void* src, size_t bytes);
 
+inline gx_status out_degrees_wrong() {
+  return fail(GX_ERR_FORMAT, "vertexout.npy does not count the source ids of the shards");
+}
+
 // Fills e->d_ocol (and d_ow) from the CSC by way of buckets of sources
 // (gx_transpose.cu), with e->d_ooff in place; the work is done on return.
 // False, with nothing written, where its tables do not reach or its scratch

@@ -1555,17 +1555,26 @@ static __global__ void scatter_values_kernel(const uint32_t* in, const int32_t* 
 // Out-edge CSR from the CSC (counting sort by source; order within a source
 // is unspecified, which min-plus / min-label do not observe).
 static __global__ void transpose_kernel(const int64_t* off, const int32_t* col, const uint32_t* w, int n,
-                                 unsigned long long* cursor, int32_t* ocol, uint32_t* ow) {
+                                 unsigned long long* cursor, int32_t* ocol, uint32_t* ow, unsigned long long E) {
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
   for (int v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += warps) {
     for (int64_t k = off[v] + lane; k < off[v + 1]; k += 32) {
       const int u = col[k];
       const unsigned long long p = atomicAdd(cursor + u, 1ull);
-      ocol[p] = v;
-      if (w) ow[p] = w[k];
+      if (p < E) {  // always, when the out-degrees count the edges
+        ocol[p] = v;
+        if (w) ow[p] = w[k];
+      }
     }
   }
+}
+
+// Whether every source's last place is where the next one's places begin.
+static __global__ void transpose_check_kernel(const unsigned long long* cursor, const int64_t* ooff, int n,
+                                              unsigned int* bad) {
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+    if (cursor[v] != static_cast<unsigned long long>(ooff[v + 1])) *bad = 1;
 }
 
 }  // namespace gx

@@ -9,6 +9,9 @@
 //     reserves their places (with an atomic each where the bucket has several
 //     slices) and writes the destinations into them; a slice's writes stay
 //     within its bucket's part of the CSR, which L2 holds.
+// The out-degrees are the caller's: that they count the edges is checked on the
+// way (the buckets' next places at the end of the first pass, before its output
+// is read, then every source's), and nothing is written outside the CSR.
 // The order within a source is unspecified, which min-plus, min-label and
 // marking do not observe.  One atomic and one random write per edge
 // (transpose_kernel), with R-MAT's hubs drawing thousands of atomics to one
@@ -52,7 +55,7 @@ struct TrArgs {
   const int64_t* ooff;
   unsigned long long* bucket_at;  // next place of each bucket
   unsigned long long* source_at;  // next place of each source
-  unsigned int* ctr;              // batches claimed
+  unsigned int* ctr;              // batches claimed; sources with more edges than outdeg says
   uint16_t* src;
   int32_t* dst;
   uint32_t* wt;
@@ -152,7 +155,9 @@ __global__ void __launch_bounds__(kTrThreads) tr_place_kernel(const __grid_const
     if (only) {
       s_src[i] = static_cast<unsigned int>(a.ooff[v0 + i] - start);
     } else if (s_src[i]) {
-      s_src[i] = static_cast<unsigned int>(atomicAdd(a.source_at + v0 + i, static_cast<unsigned long long>(s_src[i])) - start);
+      const unsigned long long n = s_src[i], p = atomicAdd(a.source_at + v0 + i, n);
+      if (p + n > static_cast<unsigned long long>(a.ooff[v0 + i + 1])) a.ctr[1] = 1;
+      s_src[i] = static_cast<unsigned int>(p - start);
     }
   }
   __syncthreads();
@@ -163,6 +168,11 @@ __global__ void __launch_bounds__(kTrThreads) tr_place_kernel(const __grid_const
       a.ocol[p] = a.dst[sl.begin + k];
       if (a.w) a.ow[p] = a.wt[sl.begin + k];
     }
+  }
+  if (only) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < nv; i += kTrThreads)
+      if (s_src[i] > static_cast<unsigned int>(a.ooff[v0 + i + 1] - start)) a.ctr[1] = 1;
   }
 }
 
@@ -195,7 +205,7 @@ bool transpose_by_buckets(gx_engine* e, bool weighted, gx_status* status) {
   const size_t n = static_cast<size_t>(E);
   const size_t o_src = place(2 * n), o_dst = place(4 * n), o_wt = place(weighted ? 4 * n : 0);
   const size_t o_bucket = place(8 * (static_cast<size_t>(nb) + 1)), o_source = place(8 * static_cast<size_t>(V)),
-               o_ctr = place(4);
+               o_ctr = place(8);
   if (dev_alloc(&block.p, at) != GX_OK) return false;  // no room: the caller's one-pass kernel
   auto run = [&]() -> gx_status {
     TrArgs a{};
@@ -219,11 +229,11 @@ bool transpose_by_buckets(gx_engine* e, bool weighted, gx_status* status) {
     a.wt = reinterpret_cast<uint32_t*>(block.p + o_wt);
     a.ocol = e->d_ocol;
     a.ow = e->d_ow;
-    std::vector<unsigned long long> start(static_cast<size_t>(nb) + 1);
+    std::vector<unsigned long long> start(static_cast<size_t>(nb) + 1), end(static_cast<size_t>(nb));
     tr_bucket_starts_kernel<<<(nb + 256) / 256, 256, 0, s>>>(e->d_ooff, V, nb, a.bucket_at);
     GX_CUDA(cudaMemcpyAsync(start.data(), a.bucket_at, 8 * start.size(), cudaMemcpyDeviceToHost, s));
     GX_CUDA(cudaMemcpyAsync(a.source_at, e->d_ooff, 8 * static_cast<size_t>(V), cudaMemcpyDeviceToDevice, s));
-    GX_CUDA(cudaMemsetAsync(a.ctr, 0, 4, s));
+    GX_CUDA(cudaMemsetAsync(a.ctr, 0, 8, s));
     // Batches of about 64 units, fewer where that would leave SMs without.
     const int smem_b = 12 * nb, smem_p = 4 * kBucket;
     GX_CUDA(allow_dynamic_smem(e->dev, reinterpret_cast<const void*>(tr_bucket_kernel)));
@@ -234,7 +244,10 @@ bool transpose_by_buckets(gx_engine* e, bool weighted, gx_status* status) {
     a.batch = std::max(1, std::min(64, a.n_units / grid));
     tr_bucket_kernel<<<grid, kTrThreads, smem_b, s>>>(a);
     GX_CUDA(cudaGetLastError());
-    GX_CUDA(cudaStreamSynchronize(s));  // `start` has arrived
+    GX_CUDA(cudaMemcpyAsync(end.data(), a.bucket_at, 8 * end.size(), cudaMemcpyDeviceToHost, s));
+    GX_CUDA(cudaStreamSynchronize(s));  // `start` and `end` have arrived
+    for (int32_t b = 0; b < nb; ++b)
+      if (end[b] != start[b + 1]) return out_degrees_wrong();
     std::vector<TrSlice> slices;
     for (int32_t b = 0; b < nb; ++b) {
       const int64_t lo = static_cast<int64_t>(start[b]), hi = static_cast<int64_t>(start[b + 1]);
@@ -249,8 +262,12 @@ bool transpose_by_buckets(gx_engine* e, bool weighted, gx_status* status) {
     a.slices = reinterpret_cast<const TrSlice*>(sblock.p);
     tr_place_kernel<<<static_cast<unsigned>(slices.size()), kTrThreads, smem_p, s>>>(a);
     GX_CUDA(cudaGetLastError());
+    // Every bucket has as many edges as its sources' out-degrees say, so a
+    // source with fewer has one with more beside it.
+    unsigned int over = 0;
+    GX_CUDA(cudaMemcpyAsync(&over, a.ctr + 1, 4, cudaMemcpyDeviceToHost, s));
     GX_CUDA(cudaStreamSynchronize(s));
-    return GX_OK;
+    return over ? out_degrees_wrong() : GX_OK;
   };
   *status = run();
   return true;
