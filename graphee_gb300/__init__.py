@@ -24,6 +24,7 @@ GX_OK, GX_ERR_INVALID, GX_ERR_IO, GX_ERR_FORMAT, GX_ERR_OOM, GX_ERR_CUDA, GX_ERR
 STATUS_NAMES = ["OK", "INVALID", "IO", "FORMAT", "OOM", "CUDA", "TIMEOUT", "NODEVICE", "STATE"]
 
 APP_PAGERANK_REF, APP_PAGERANK_STD, APP_SSSP, APP_CC, APP_INDEGREE = range(5)
+BOUND_BLOCK = 0
 BUILD_DROP_SELF, BUILD_DEDUP, BUILD_SYMMETRIZE = 1, 2, 4
 GPS_INF = 10000          # GraphMP/system/Global.h:50
 INF_WEIGHTED = 0xFFFFFFFF
@@ -111,6 +112,7 @@ def lib() -> C.CDLL:
         "gx_create": (C.c_int, [P, P]),
         "gx_destroy": (C.c_int, [P]),
         "gx_set_wait_limit": (C.c_int, [P, C.c_uint32]),
+        "gx_set_bound": (C.c_int, [P, C.c_int, I64]),
         "gx_release_cached_memory": (C.c_int, [I32]),
         "gx_build_csc_gpu": (C.c_int, [I32, I32, I64, P, P, I32, P, P, P]),
         "gx_rmat_csc_gpu": (C.c_int, [I32, I32, I64, D, D, D, U64, I32, P, P, P]),
@@ -390,6 +392,10 @@ class Engine:
         """Polls a device-side wait makes before the call gives up with
         GX_ERR_TIMEOUT (config.wait_limit)."""
         _check(lib().gx_set_wait_limit(self._h, polls), "gx_set_wait_limit")
+
+    def set_bound(self, which: int, value: int) -> None:
+        """One of the BOUND_* for the engine's later calls; 0 restores the default (gx_set_bound)."""
+        _check(lib().gx_set_bound(self._h, which, value), "gx_set_bound")
 
     def load(self, g: Graph) -> "Engine":
         _check(lib().gx_load_csc(self._h, g.V, g.P, _ptr(g.bounds), _ptr(g.off), _ptr(g.col), _ptr(g.outdeg)),

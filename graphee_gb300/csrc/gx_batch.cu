@@ -953,6 +953,7 @@ gx_status gx_batch_run(gx_engine* e, int32_t n_inst, const int32_t* inst_vbegin,
   if (tuning) t = *tuning;
   GX_TRY(check_tuning(t));
   GX_CUDA(cudaSetDevice(e->dev));
+  BlockBound bound(e->block_bound);
   BatchDev d;
   BatchArgs a;
   GX_TRY(batch_prepare(e, n_inst, inst_vbegin, d, a));
@@ -992,6 +993,7 @@ gx_status gx_batch_autotune(gx_engine* e, int32_t n_inst, const int32_t* inst_vb
   if (!e->loaded || !e->all_resident) return fail(GX_ERR_STATE, "gx_batch_autotune: load the packed graph first");
   if (e->relabeled) return fail(GX_ERR_STATE, "gx_batch_autotune: the engine renumbered the vertices (config.relabel)");
   GX_CUDA(cudaSetDevice(e->dev));
+  BlockBound bound(e->block_bound);
   BatchDev d;
   BatchArgs a;
   GX_TRY(batch_prepare(e, n_inst, inst_vbegin, d, a));

@@ -800,6 +800,7 @@ gx_status build_shard_sets(gx_engine* e) {
 gx_status build_out_edges(gx_engine* e, bool weighted) {
   if (e->out_built && (!weighted || e->out_weighted)) return GX_OK;
   const int32_t V = e->V;
+  e->out_built = false;  // its arrays are replaced: a failure below leaves none
   int64_t total = 0;
   int negative = 0;
 #pragma omp parallel for reduction(+ : total) reduction(| : negative)
@@ -1582,6 +1583,14 @@ gx_status gx_set_wait_limit(gx_engine* e, uint32_t polls) {
   return GX_OK;
 }
 
+gx_status gx_set_bound(gx_engine* e, gx_bound which, int64_t value) {
+  if (!e || value < 0) return fail(GX_ERR_INVALID, "gx_set_bound: engine NULL or value negative");
+  switch (which) {
+    case GX_BOUND_BLOCK: e->block_bound = static_cast<size_t>(value); return GX_OK;
+  }
+  return fail(GX_ERR_INVALID, "gx_set_bound: unknown bound %d", static_cast<int>(which));
+}
+
 gx_status gx_release_cached_memory(int32_t device) {
   int n = 0;
   if (cudaGetDeviceCount(&n) != cudaSuccess || n == 0) {
@@ -1618,6 +1627,7 @@ gx_status gx_load_csc(gx_engine* e, int32_t V, int32_t P, const int32_t* bounds,
   const int64_t E = off[V];
   if (E > (int64_t(1) << 40)) return fail(GX_ERR_INVALID, "gx_load_csc: too many edges");
   GX_CUDA(cudaSetDevice(e->dev));
+  BlockBound bound(e->block_bound);
   e->release_graph();
   e->V = V;
   e->P = P;
@@ -1811,6 +1821,7 @@ gx_status gx_set_weights(gx_engine* e, const uint32_t* w) {
   if (!e->loaded) return fail(GX_ERR_STATE, "gx_set_weights: no graph loaded");
   GX_CUDA(cudaSetDevice(e->dev));
   if (!e->all_resident && !e->h_col) return fail(GX_ERR_STATE, "gx_set_weights: streaming source missing");
+  BlockBound bound(e->block_bound);
   if (e->all_resident && e->cfg.cache_budget_bytes < 0) {
     // No budget: the weights go straight to the device (a relabelled engine
     // moves them into its own layout there).
@@ -1908,6 +1919,7 @@ gx_status gx_run(gx_engine* e, const gx_run_params* prm, gx_run_stats* stats) {
   if (prm->checkpoint_every < 0 || (prm->checkpoint_every > 0 && !prm->checkpoint_prefix))
     return fail(GX_ERR_INVALID, "gx_run: checkpoint_every needs checkpoint_prefix");
   GX_CUDA(cudaSetDevice(e->dev));
+  BlockBound bound(e->block_bound);
   gx_run_params p = *prm;
   if (p.max_iter == 0) {
     e->last_steps = 0;

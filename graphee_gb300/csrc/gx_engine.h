@@ -74,6 +74,17 @@ inline void pool_free(void* p) {
   cudaStreamSynchronize(dp->stream);
 }
 
+// Largest block that dev_alloc hands out to this thread's call, 0: any
+// (GX_BOUND_BLOCK of the engine it works on).
+inline thread_local size_t block_bound = 0;
+struct BlockBound {
+  size_t before = block_bound;
+  explicit BlockBound(size_t bytes) { block_bound = bytes; }
+  ~BlockBound() { block_bound = before; }
+  BlockBound(const BlockBound&) = delete;
+  BlockBound& operator=(const BlockBound&) = delete;
+};
+
 template <class T>
 gx_status dev_alloc(T** p, size_t n) {
   if (*p) {
@@ -81,6 +92,8 @@ gx_status dev_alloc(T** p, size_t n) {
     *p = nullptr;
   }
   if (n == 0) n = 1;
+  if (block_bound && n * sizeof(T) > block_bound)
+    return fail(GX_ERR_OOM, "device allocation of %zu bytes: the engine's bound is %zu", n * sizeof(T), block_bound);
   cudaError_t err = pool_malloc(reinterpret_cast<void**>(p), n * sizeof(T));
   if (err != cudaSuccess) {
     *p = nullptr;
@@ -192,6 +205,7 @@ struct gx_engine {
   gx::hvec<int64_t> off;
   gx::hvec<int32_t> outdeg;
   int64_t n_dangling = 0;            // vertices of out-degree 0
+  size_t block_bound = 0;            // GX_BOUND_BLOCK
   gx::UnitCaps caps{};               // tile and chunk sizes, heavy threshold (build_units)
   gx::hvec<int2> units;
   gx::hvec<int32_t> unit_shard;

@@ -312,6 +312,7 @@ extern "C" gx_status gx_ppr(gx_engine* e, int32_t k, const int32_t* sources, int
   for (int j = 0; j < k; ++j)
     if (sources[j] < 0 || sources[j] >= V) return fail(GX_ERR_INVALID, "gx_ppr: source %d outside [0, %d)", sources[j], V);
   GX_CUDA(cudaSetDevice(e->dev));
+  BlockBound bound(e->block_bound);
   cudaStream_t s = e->s_comp;
   const int W = k <= 8 ? 8 : k <= 16 ? 16 : k <= 32 ? 32 : 64;
   const size_t rows = static_cast<size_t>(V) * W;

@@ -431,6 +431,7 @@ extern "C" gx_status gx_triangle_count(gx_engine* e, uint64_t* total, gx_run_sta
   if (!e->all_resident)
     return fail(GX_ERR_STATE, "gx_triangle_count: needs every shard resident (no shard-cache budget)");
   GX_CUDA(cudaSetDevice(e->dev));
+  BlockBound bound(e->block_bound);
   const int32_t V = e->V;
   cudaStream_t s = e->s_comp;
   cudaEvent_t ev0, ev1, listed, big_done;

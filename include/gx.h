@@ -163,6 +163,14 @@ gx_status gx_destroy(gx_engine* e);
  * reference counterpart: the reference has no device-side waits. */
 gx_status gx_set_wait_limit(gx_engine* e, uint32_t polls);
 
+/* Bounds that only a graph near the device's size meets otherwise, lowered by
+ * tests to reach what lies behind them at small ones; 0 sets the default. */
+typedef enum gx_bound {
+  GX_BOUND_BLOCK = 0  /* bytes of the largest block of device memory the engine's calls get: for a
+                         larger one there is no room (default: what the device has) */
+} gx_bound;
+gx_status gx_set_bound(gx_engine* e, gx_bound which, int64_t value);
+
 /* Engines draw device memory from a per-device pool that keeps blocks after
  * gx_destroy, so the next engine's load maps no new memory.  This returns
  * the cached blocks of `device` to the driver.  No reference counterpart. */

@@ -1,0 +1,41 @@
+"""Calls that the device has no room for (a bound on the engine's blocks stands
+for a device that is nearly full): what they leave behind, and those that do
+with less.
+"""
+import numpy as np
+import pytest
+
+import graphee_gb300 as gx
+import gx_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def test_bounds_are_checked():
+    with gx.Engine() as e:
+        for which, value in ((gx.BOUND_BLOCK, -1), (99, 1)):
+            with pytest.raises(gx.GxError) as ei:
+                e.set_bound(which, value)
+            assert ei.value.status == gx.GX_ERR_INVALID
+
+
+@pytest.mark.parametrize("relabel", [0, 1])
+def test_out_edges_after_a_rebuild_that_failed(relabel):
+    """CC built the out-edge CSR; weighted SSSP replaces it by one with weights, and fails."""
+    g = gx.rmat_graph(12, 8, seed=5, P=4, weight_seed=6)
+    a = (g.V, g.P, g.bounds, g.off, g.col, g.outdeg)
+    labels = O.run(O.CC, *a, 1000)[0]
+    with gx.Engine(relabel=relabel, push_edge_fraction=1.0) as e:
+        e.load(g)
+        e.run(gx.APP_CC, 1000)
+        assert np.array_equal(e.values(), labels)
+        for room in (4 * g.E, 4 * g.V):
+            e.set_bound(gx.BOUND_BLOCK, room)
+            with pytest.raises(gx.GxError) as ei:
+                e.run(gx.APP_SSSP, 1000, source=1, weighted=True)
+            assert ei.value.status == gx.GX_ERR_OOM
+            e.set_bound(gx.BOUND_BLOCK, 0)
+            st = e.run(gx.APP_CC, 1000)
+            assert np.array_equal(e.values(), labels) and st["push_iterations"] > 0
+        e.run(gx.APP_SSSP, 1000, source=1, weighted=True)
+        assert np.array_equal(e.values(), O.run(O.SSSP, *a, 1000, weights=g.weights, source=1)[0])
