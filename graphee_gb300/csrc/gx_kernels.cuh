@@ -285,6 +285,18 @@ __device__ __forceinline__ bool apply_vertex(const ApplyCtx c, int v, typename A
   return act;
 }
 
+// A vertex of a shard that a selective step skips keeps its value, and with it
+// its part of the mass that standard PageRank takes from the sinks.
+template <int APP>
+__device__ __forceinline__ void carry_vertex(const ApplyCtx& c, int v, typename AppTraits<APP>::T old, int32_t od,
+                                             void* dst_val, const float* src_con, float* dst_con, LocalAcc& la) {
+  static_cast<typename AppTraits<APP>::T*>(dst_val)[v] = old;
+  if constexpr (is_pr<APP>()) dst_con[v] = src_con[v];
+  if constexpr (APP == K_PR_STD) {
+    if (od == 0) la.dangl += __double2ull_rn(static_cast<double>(old) * c.fx_scale);
+  }
+}
+
 __device__ __forceinline__ void bitmap_set_tile(uint32_t* bm, int vb, unsigned mask) {
   // Lanes are consecutive vertices vb..vb+31: at most two bitmap words.
   if (mask == 0) return;
@@ -698,10 +710,9 @@ __device__ __forceinline__ void pull_sweep(const PullArgs& a, const ApplyCtx& c,
         const int4 H = a.heavy[h];
         const int v = H.x;
         if (!on) {
-          if (wu.y == 0 && lane == 0) {
-            static_cast<T*>(dst_val)[v] = static_cast<const T*>(src_val)[v];
-            if constexpr (is_pr<APP>()) dst_con[v] = src_con[v];
-          }
+          if (wu.y == 0 && lane == 0)
+            carry_vertex<APP>(c, v, static_cast<const T*>(src_val)[v], APP == K_PR_STD ? a.outdeg[v] : 0, dst_val, src_con,
+                              dst_con, la);
           continue;
         }
         const int64_t vb = a.off[v], ve = a.off[v + 1];
@@ -765,10 +776,7 @@ __device__ __forceinline__ void pull_sweep(const PullArgs& a, const ApplyCtx& c,
       // Vertices above the heavy threshold are applied by their own units.
       const bool valid = lane < n && end - beg <= a.heavy_deg;
       if (!on) {
-        if (valid) {
-          static_cast<T*>(dst_val)[v] = old;
-          if constexpr (is_pr<APP>()) dst_con[v] = src_con[v];
-        }
+        if (valid) carry_vertex<APP>(c, v, old, od, dst_val, src_con, dst_con, la);
         continue;
       }
       T acc;
