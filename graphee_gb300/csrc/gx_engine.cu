@@ -1405,7 +1405,7 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
           GX_CUDA(cudaStreamWaitEvent(e->s_comp, e->slot_ready[slot], 0));
           sp.col = e->slot_col[slot] - lo;
           if (weighted) sp.w = e->slot_w[slot] - lo;
-          streamed += grp.last - grp.first;
+          for (int32_t i = p; i < grp.last; ++i) streamed += e->unit_begin[i + 1] > e->unit_begin[i];
         }
         const PullShape shape = pull_shape(sp.u_end - sp.u_begin, grid_pull_max, kThreads);
         sp.grab = shape.grab;
