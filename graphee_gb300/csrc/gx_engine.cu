@@ -711,17 +711,26 @@ gx_status plan_shards(gx_engine* e, const int32_t* src_col, bool col_on_device) 
     int64_t streamed_elems = 0;
     for (int32_t p = 0; p < P; ++p)
       if (!e->resident[p]) streamed_elems += hi[p] - lo[p];
-    e->slot_elems = std::max(max_stream, std::min(streamed_elems, kStreamGroup)) + 8;
-    for (auto ptr : e->slot_col) gx::pool_free(ptr);
-    for (auto ptr : e->slot_w) gx::pool_free(ptr);
     for (auto ptr : e->slot_blob) gx::pool_free(ptr);
     e->slot_blob.clear();
-    e->slot_col.assign(slots, nullptr);
-    e->slot_w.assign(slots, nullptr);
-    for (int i = 0; i < slots; ++i) {
-      GX_TRY(dev_alloc(&e->slot_col[i], e->slot_elems));
-      if (e->has_weights) GX_TRY(dev_alloc(&e->slot_w[i], e->slot_elems));
-    }
+    auto ring = [&](int64_t elems) -> gx_status {
+      for (auto ptr : e->slot_col) gx::pool_free(ptr);
+      for (auto ptr : e->slot_w) gx::pool_free(ptr);
+      e->slot_col.assign(slots, nullptr);
+      e->slot_w.assign(slots, nullptr);
+      e->slot_elems = elems;
+      for (int i = 0; i < slots; ++i) {
+        GX_TRY(dev_alloc(&e->slot_col[i], elems));
+        if (e->has_weights) GX_TRY(dev_alloc(&e->slot_w[i], elems));
+      }
+      return GX_OK;
+    };
+    // Without room for groups the slots hold the longest shard, and a group is
+    // what fits one.
+    const int64_t group = std::max(max_stream, std::min(streamed_elems, kStreamGroup)) + 8;
+    gx_status ring_st = ring(group);
+    if (ring_st == GX_ERR_OOM && group > max_stream + 8) ring_st = ring(max_stream + 8);
+    if (ring_st != GX_OK) return ring_st;
     e->n_slots = slots;
     GX_TRY(setup_slot_events(e, slots));
     // Streamed shards travel compressed when the weights (if any) fit bytes.

@@ -39,3 +39,22 @@ def test_out_edges_after_a_rebuild_that_failed(relabel):
             assert np.array_equal(e.values(), labels) and st["push_iterations"] > 0
         e.run(gx.APP_SSSP, 1000, source=1, weighted=True)
         assert np.array_equal(e.values(), O.run(O.SSSP, *a, 1000, weights=g.weights, source=1)[0])
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+def test_streaming_slots_of_one_shard(weighted):
+    """No room for slots that hold a group of shards (4 M edges): they hold the longest shard, as the others did."""
+    src, dst = gx.rmat_edges(16, 4 << 20, 8)
+    off, col = gx.build_csc(1 << 16, src, dst)
+    g = gx.Graph(1 << 16, off, col, None, 16)
+    a = (g.V, g.P, g.bounds, g.off, g.col, g.outdeg)
+    if weighted:
+        g.weights = gx.edge_weights(3, g)
+    room = 2 << 20
+    assert 4 * g.E > room > 4 * np.diff(g.off[g.bounds]).max() + 64
+    with gx.Engine(cache_budget_bytes=0, compress_cache=0) as e:
+        e.set_bound(gx.BOUND_BLOCK, room)
+        e.load(g)
+        st = e.run(gx.APP_SSSP, 1000, source=1, weighted=weighted)
+        assert np.array_equal(e.values(), O.run(O.SSSP, *a, 1000, weights=g.weights, source=1)[0])
+        assert st["pull_launches"] >= g.P // 2  # several groups a step
