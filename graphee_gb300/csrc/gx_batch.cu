@@ -38,7 +38,7 @@
 // per short list, else 4 consecutive edges per lane per round of 128 aligned
 // edges and an xor tree), so results do not depend on the layout.
 // 512 instances of scales 10 to 17 (290 M edges, 35 supersteps): 52.6 ms a
-// call swept as they lie, 26.8 rewritten (the rewriting's share 3.5 ms); long
+// call swept as they lie, 26.0 rewritten (the rewriting's share 2.4 ms); long
 // scoreboard stalls on the id loads lead now, at 0.29 of HBM's rate.
 // Threads per CTA, lane_max and CTAs per SM come from the autotuner
 // (gx_batch_autotune), which times candidate schedules on the batch and
@@ -62,9 +62,20 @@ using namespace gx;
 namespace {
 
 constexpr int kBatchSortThreads = 512;
-constexpr int kFillSplit = 8;       // CTAs that share an instance in batch_fill_kernel
+constexpr int kSortSmall = 64;       // where no instance has more than four times as many vertices
 constexpr int kBatchL1 = 64 * 1024;  // shared-memory bytes per SM left to the L1
-constexpr int kCheckSplit = 4;  // CTAs that share an instance in batch_check_kernel
+
+// CTAs that share an instance in the kernels that check and rewrite, which take
+// the instances in turn: as many as the longest has pieces of `piece` edges and
+// vertices, as far as `ctas` in all give every instance that many, but `least`
+// of them at any number (the longest instances of many end last).  (With one,
+// four and eight at any number, an instance of 2 M vertices and 30 M edges took
+// 6.8 ms to sort, 1.9 to check and 4.5 to write out, now 0.06, 0.03 and 0.09,
+// and 20000 instances of 8 vertices 0.17, 0.10 and 0.39, now 0.03, 0.03, 0.09.)
+int batch_split(int64_t longest, int64_t piece, int64_t ctas, int32_t n, int least) {
+  const int64_t most = std::max<int64_t>(least, ctas / n);
+  return static_cast<int>(std::max<int64_t>(1, std::min((longest + piece - 1) / piece, most)));
+}
 
 // A unit of an instance's sweep: `cnt` vertices from local (new) id `first`
 // on, its rounds from round `at` of the instance on.
@@ -104,8 +115,9 @@ struct BatchArgs {
   int32_t* od;              // out-degrees by new id
   BatchUnit* units;         // instance i's at units[vbeg[i]]
   int32_t* n_units;
-  unsigned long long* rounds;  // per instance: 256-byte blocks of its rounds
-  const unsigned long long* round_base;  // first block
+  unsigned long long* rounds;  // per instance
+  const unsigned long long* round_base;  // first block of its rounds
+  int* classes;             // split sorts, per instance: vertices of every class, and those placed
   uint2* ids;               // blocks of 32 x 4 16-bit ids; a round of 32-bit ids is two
   double damping;
 };
@@ -217,12 +229,12 @@ __device__ __forceinline__ void batch_tree(int from, float& f, int32_t& m) {
 // Barrier b of a team of `team` CTAs on instance state t[0..3]: adds this
 // CTA's change count to t[1 + b % 3] (member 0 first clears the slot barrier
 // b + 1 will use) and returns the team's total.  Every thread of the CTA
-// calls it.  Returns false when the wait timed out or another team aborted.
+// calls it, after a CTA barrier.  Returns false when the wait timed out or
+// another team aborted.
 __device__ bool team_barrier(const BatchArgs& a, unsigned int* t, int team, int member, int b, unsigned changed,
                              unsigned* total) {
   __shared__ unsigned s_tot;
   __shared__ int s_ok;
-  __syncthreads();
   if (threadIdx.x == 0) {
     int ok = 1;
     if (member == 0) atomicExch(t + 1 + (b + 1) % 3, 0u);
@@ -362,15 +374,15 @@ __global__ void __launch_bounds__(1024, 1) batch_kernel(const __grid_constant__ 
   extern __shared__ __align__(16) uint32_t s_tab[];
   __shared__ BatchStep s_st;
   __shared__ int s_slot;
-  __shared__ unsigned int s_changed;
+  __shared__ unsigned int s_changed[2];
   const int lane = threadIdx.x & 31;
   for (;;) {
-    if (threadIdx.x == 0) s_slot = static_cast<int>(atomicAdd(a.ctr, 1u));
+    if (threadIdx.x == 0)
+      s_slot = *reinterpret_cast<volatile unsigned*>(a.abort) ? a.n_slots : static_cast<int>(atomicAdd(a.ctr, 1u));
     __syncthreads();
     const int slot = s_slot;
     __syncthreads();
     if (slot >= a.n_slots) break;
-    if (*reinterpret_cast<volatile unsigned*>(a.abort)) break;
     const int2 sl = a.slots[slot];
     const int inst = sl.x, member = sl.y >> 16, team = sl.y & 0xffff;
     unsigned int* tstate = a.team + 4 * static_cast<int64_t>(inst);
@@ -383,20 +395,20 @@ __global__ void __launch_bounds__(1024, 1) batch_kernel(const __grid_constant__ 
     const bool dual = batch_dual(n, team, a.tab);
     const int tn = batch_table(n, a.tab);
     int bar = 0;
-    // The barrier that ends a phase: a CTA barrier, or the team's.
-    auto sync_count = [&](unsigned mine, unsigned* total) -> bool {
-      if (threadIdx.x == 0) s_changed = 0;
+    // The barrier that ends step `step` (or, -1, what comes before the first): a
+    // CTA barrier, or the team's; *total: the step's changes.  Steps count in two
+    // places in turn: the next sweep's set-up clears its own, which every thread
+    // has read before the barriers of the step between.  (Thousands of tiny
+    // instances are little but barriers: a superstep from the table has this one
+    // and the sweep's.  __syncthreads_or in place of the count, or two step
+    // records in turn to do without the sweep's, cost the sweep more in registers
+    // than they saved: 512 instances 26.1 -> 26.9 and 27.5 ms.)
+    auto sync_count = [&](int step, unsigned mine, unsigned* total) -> bool {
+      unsigned* at = s_changed + (step & 1);
+      if (lane == 0 && mine) atomicAdd(at, mine);
       __syncthreads();
-      if (threadIdx.x == 0) s_st.s_next = 0;
-      if (lane == 0 && mine) atomicAdd(&s_changed, mine);
-      __syncthreads();
-      const unsigned cta = s_changed;
-      if (team == 1) {
-        *total = cta;
-        __syncthreads();
-        return true;
-      }
-      return team_barrier(a, tstate, team, member, bar++, threadIdx.x == 0 ? cta : 0u, total);
+      *total = *reinterpret_cast<volatile unsigned*>(at);
+      return team == 1 || team_barrier(a, tstate, team, member, bar++, *total, total);
     };
     // The table's copy of the values a finished phase left in g (through L2:
     // other CTAs of the team wrote them).
@@ -415,9 +427,10 @@ __global__ void __launch_bounds__(1024, 1) batch_kernel(const __grid_constant__ 
       s_st.od = a.od + vb;
       s_st.damping = a.damping;
       s_st.inv_n = inv_n;
+      s_changed[0] = s_changed[1] = 0;
     }
     // Superstep `step` from buffer `cur` (x0, x1: ranks or labels; c0, c1:
-    // contributions); the changes of this warp.
+    // contributions), after a barrier; the changes of this warp.
     auto sweep = [&](auto pr, int step, int cur, void* x0, void* x1, float* c0, float* c1) -> unsigned {
       constexpr bool PR = decltype(pr)::value;
       if (threadIdx.x == 0) {
@@ -428,6 +441,8 @@ __global__ void __launch_bounds__(1024, 1) batch_kernel(const __grid_constant__ 
         s_st.g = static_cast<const uint32_t*>(PR ? (cur ? c1 : c0) : (cur ? x1 : x0));
         s_st.tab = dual && cur ? n + 1 : 0;
         s_st.next = cur ? 0 : n + 1;
+        s_st.s_next = 0;
+        s_changed[step & 1] = 0;
       }
       __syncthreads();
       const bool wide = n >= kBatchWide;
@@ -452,12 +467,12 @@ __global__ void __launch_bounds__(1024, 1) batch_kernel(const __grid_constant__ 
       if (dual) s_tab[k] = __float_as_uint(c);
       else a.con0[vb + k] = c;
     }
-    if (!sync_count(0, &tot)) return;
+    if (!sync_count(-1, 0, &tot)) return;
     if (!dual) fill(reinterpret_cast<const uint32_t*>(a.con0 + vb));
     int cur = 0, step = 0;
     for (step = 0; step < a.pr_iters; ++step) {
       const unsigned changed = sweep(std::true_type(), step, cur, a.pr0 + vb, a.pr1 + vb, a.con0 + vb, a.con1 + vb);
-      if (!sync_count(changed, &tot)) return;
+      if (!sync_count(step, changed, &tot)) return;
       cur ^= 1;
       if (tot == 0 && step > 1) {
         ++step;
@@ -475,12 +490,12 @@ __global__ void __launch_bounds__(1024, 1) batch_kernel(const __grid_constant__ 
       if (dual) s_tab[k] = static_cast<uint32_t>(label);
       else a.lab0[vb + k] = label;
     }
-    if (!sync_count(0, &tot)) return;
+    if (!sync_count(-1, 0, &tot)) return;
     if (!dual) fill(reinterpret_cast<const uint32_t*>(a.lab0 + vb));
     cur = 0;
     for (step = 0; step < a.cc_max; ++step) {
       const unsigned changed = sweep(std::false_type(), step, cur, a.lab0 + vb, a.lab1 + vb, nullptr, nullptr);
-      if (!sync_count(changed, &tot)) return;
+      if (!sync_count(step, changed, &tot)) return;
       cur ^= 1;
       if (tot == 0 && step > 1) {
         ++step;
@@ -496,16 +511,17 @@ __global__ void __launch_bounds__(1024, 1) batch_kernel(const __grid_constant__ 
   }
 }
 
-// CTAs take the instances in turn: every edge must stay inside its instance
-// (read end to end, four ids a thread: a thread per vertex, walking its list,
-// took 3.6 ms for 290 M edges).
+// `split` CTAs take the instances in turn: every edge must stay inside its
+// instance (read end to end, four ids a thread: a thread per vertex, walking
+// its list, took 3.6 ms for 290 M edges).
 __global__ void __launch_bounds__(512) batch_check_kernel(const int64_t* off, const int32_t* col, const int32_t* vbeg,
-                                                          int32_t n_inst, unsigned int* bad) {
+                                                          int32_t n_inst, int split, unsigned int* bad) {
   unsigned c = 0;
-  for (int i = blockIdx.x / kCheckSplit; i < n_inst; i += gridDim.x / kCheckSplit) {
+  const int64_t part = blockIdx.x % split, stride = 4ll * split * blockDim.x;
+  for (int i = blockIdx.x / split; i < n_inst; i += gridDim.x / split) {
     const int32_t vb = vbeg[i], ve = vbeg[i + 1];
-    const int64_t b = off[vb], e = off[ve], part = blockIdx.x % kCheckSplit;
-    for (int64_t q = (b & ~3ll) + 4 * (part * blockDim.x + threadIdx.x); q < e; q += 4 * kCheckSplit * blockDim.x) {
+    const int64_t b = off[vb], e = off[ve];
+    for (int64_t q = (b & ~3ll) + 4 * (part * blockDim.x + threadIdx.x); q < e; q += stride) {
       const int4 x = __ldcs(reinterpret_cast<const int4*>(col + q));
       const int32_t cs[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
@@ -533,48 +549,79 @@ __device__ __forceinline__ int batch_class(int64_t beg, int64_t len, int lane_ma
 // Lists across the warp of up to this many rounds share a unit, four to each.
 constexpr int kWarpShare = 4;
 
-// An instance per CTA (taken in turn): its vertices in order of their
-// classes, and its units.  Within a class the order is that of the atomics:
-// no result depends on it.
-__global__ void __launch_bounds__(kBatchSortThreads) batch_sort_kernel(const __grid_constant__ BatchArgs a) {
+// Instances (taken in turn) get their vertices in order of their classes, and
+// their units.  Within a class the order is that of the atomics, and so is the
+// units' place among the rounds: no result depends on them.  An instance per
+// CTA in one launch (kSortAll), or `split` CTAs to an instance in three that
+// count the classes, place the vertices and make the units.
+enum : int { kSortAll = 0, kSortCount = 1, kSortPlace = 2, kSortUnits = 3 };
+template <int PHASE>
+__global__ void __launch_bounds__(kBatchSortThreads) batch_sort_kernel(const __grid_constant__ BatchArgs a, int split) {
   __shared__ int s_at[kClasses + 1];
-  __shared__ int s_cur[kClasses];
+  __shared__ __align__(16) int s_cur[kClasses];
   __shared__ unsigned long long s_w[kBatchSortThreads / 32], s_run;
+  static_assert(kClasses == 128, "a lane scans four classes");
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int i = blockIdx.x; i < a.n_inst; i += gridDim.x) {
+  const int T = blockDim.x, part = blockIdx.x % split, stride = T * split;
+  for (int i = blockIdx.x / split; i < a.n_inst; i += gridDim.x / split) {
     const int32_t vb = a.vbeg[i], n = a.vbeg[i + 1] - vb;
-    for (int c = threadIdx.x; c < kClasses; c += kBatchSortThreads) s_cur[c] = 0;
-    __syncthreads();
-    for (int k = threadIdx.x; k < n; k += kBatchSortThreads) {
-      const int64_t beg = a.off[vb + k];
-      atomicAdd(&s_cur[batch_class(beg, a.off[vb + k + 1] - beg, a.lane_max)], 1);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int run = 0;
-      for (int c = 0; c < kClasses; ++c) {
-        s_at[c] = run;
-        run += s_cur[c];
-        s_cur[c] = s_at[c];
+    int* classes = PHASE == kSortAll ? nullptr : a.classes + 2 * kClasses * static_cast<int64_t>(i);  // counted; placed
+    if (PHASE != kSortUnits) {
+      for (int c = threadIdx.x; c < kClasses; c += T) s_cur[c] = 0;
+      __syncthreads();
+      for (int k = part * T + threadIdx.x; k < n; k += stride) {
+        const int64_t beg = a.off[vb + k];
+        atomicAdd(&s_cur[batch_class(beg, a.off[vb + k + 1] - beg, a.lane_max)], 1);
       }
-      s_at[kClasses] = run;
-      s_run = 0;
+      __syncthreads();
+    }
+    if (PHASE == kSortCount) {
+      for (int c = threadIdx.x; c < kClasses; c += T)
+        if (s_cur[c]) atomicAdd(classes + c, s_cur[c]);
+      __syncthreads();
+      continue;
+    }
+    if (wid == 0) {
+      const int4 x = *reinterpret_cast<const int4*>((PHASE == kSortAll ? s_cur : classes) + 4 * lane);
+      const int sum = x.x + x.y + x.z + x.w;
+      int incl = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      const int at = incl - sum;
+      s_at[4 * lane] = at;
+      s_at[4 * lane + 1] = at + x.x;
+      s_at[4 * lane + 2] = at + x.x + x.y;
+      s_at[4 * lane + 3] = at + x.x + x.y + x.z;
+      if (lane == 31) s_at[kClasses] = incl;
+      if (lane == 0) s_run = 0;
     }
     __syncthreads();
-    for (int k = threadIdx.x; k < n; k += kBatchSortThreads) {
-      const int64_t beg = a.off[vb + k];
-      const int p = atomicAdd(&s_cur[batch_class(beg, a.off[vb + k + 1] - beg, a.lane_max)], 1);
-      a.perm[vb + k] = p;
-      a.inv[vb + p] = vb + k;
-      a.od[vb + p] = a.outdeg[vb + k];
+    if (PHASE != kSortUnits) {
+      for (int c = threadIdx.x; c < kClasses; c += T) {
+        int at = s_at[c];
+        if (PHASE == kSortPlace && s_cur[c]) at += atomicAdd(classes + kClasses + c, s_cur[c]);
+        s_cur[c] = at;
+      }
+      __syncthreads();
+      for (int k = part * T + threadIdx.x; k < n; k += stride) {
+        const int64_t beg = a.off[vb + k];
+        const int p = atomicAdd(&s_cur[batch_class(beg, a.off[vb + k + 1] - beg, a.lane_max)], 1);
+        a.perm[vb + k] = p;
+        a.inv[vb + p] = vb + k;
+        a.od[vb + p] = a.outdeg[vb + k];
+      }
+      __syncthreads();
     }
-    __syncthreads();
+    if (PHASE == kSortPlace) continue;
     // Units: the warp lists of many rounds one each, the others four to a
     // unit, the half-warp lists eight to a unit, the lane lists 32.
     const int n_one = s_at[kClassCap - kWarpShare], n_warp = s_at[kClassHalf], n_wide = s_at[kClassLane];
     const int u_one = n_one, u_warp = u_one + (n_warp - n_one + 3) / 4, u_half = u_warp + (n_wide - n_warp + 7) / 8;
     const int u_all = u_half + (n - n_wide + 31) / 32;
-    for (int u0 = 0; u0 < u_all; u0 += kBatchSortThreads) {
+    for (int u0 = part * T; u0 < u_all; u0 += stride) {
       const int u = u0 + threadIdx.x;
       BatchUnit x{0, 0, 0, 0};
       unsigned long long total = 0;
@@ -614,37 +661,42 @@ __global__ void __launch_bounds__(kBatchSortThreads) batch_sort_kernel(const __g
       }
       if (lane == 31) s_w[wid] = incl;
       __syncthreads();
-      unsigned long long before = s_run, all = 0;
-      for (int w = 0; w < kBatchSortThreads / 32; ++w) {
+      unsigned long long before = 0, all = 0;
+      for (int w = 0; w < T / 32; ++w) {
         before += w < wid ? s_w[w] : 0;
         all += s_w[w];
       }
+      if (PHASE == kSortUnits) {  // the place of these T units among all CTAs'
+        if (threadIdx.x == 0) s_run = atomicAdd(a.rounds + i, all);
+        __syncthreads();
+      }
+      before += s_run;
       if (u < u_all) {
         x.at = static_cast<int32_t>(before + incl - total);
         a.units[vb + u] = x;
       }
       __syncthreads();
-      if (threadIdx.x == 0) s_run += all;
-      __syncthreads();
+      if (PHASE == kSortAll) {
+        if (threadIdx.x == 0) s_run += all;
+        __syncthreads();
+      }
     }
-    if (threadIdx.x == 0) {
-      a.n_units[i] = u_all;
-      a.rounds[i] = n >= kBatchWide ? 2 * s_run : s_run;
-    }
+    if (threadIdx.x == 0 && part == 0) a.n_units[i] = u_all;
+    if (PHASE == kSortAll && threadIdx.x == 0) a.rounds[i] = s_run;
     __syncthreads();
   }
 }
 
-// Writes the rounds: kFillSplit CTAs share an instance, a warp per unit.
-__global__ void __launch_bounds__(256) batch_fill_kernel(const __grid_constant__ BatchArgs a) {
+// Writes the rounds: `split` CTAs share an instance, a warp per unit.
+__global__ void __launch_bounds__(256) batch_fill_kernel(const __grid_constant__ BatchArgs a, int split) {
   const int lane = threadIdx.x & 31;
-  const int w0 = (blockIdx.x % kFillSplit) * 8 + (threadIdx.x >> 5);
-  for (int i = blockIdx.x / kFillSplit; i < a.n_inst; i += gridDim.x / kFillSplit) {
+  const int w0 = (blockIdx.x % split) * 8 + (threadIdx.x >> 5);
+  for (int i = blockIdx.x / split; i < a.n_inst; i += gridDim.x / split) {
     const int32_t vb = a.vbeg[i], n = a.vbeg[i + 1] - vb;
     const int tn = batch_table(n, a.tab);
     const bool wide = n >= kBatchWide;
     uint2* ids = a.ids + 32 * a.round_base[i];
-    for (int t = w0; t < a.n_units[i]; t += kFillSplit * 8) {
+    for (int t = w0; t < a.n_units[i]; t += split * 8) {
       const BatchUnit u = a.units[vb + t];
       const int kind = u.kind_cnt >> 8, cnt = u.kind_cnt & 255;
       // The vertex and the position of this lane's first place in each round.
@@ -691,44 +743,23 @@ __global__ void __launch_bounds__(256) batch_fill_kernel(const __grid_constant__
   }
 }
 
+// A call's device memory: one block for what depends on the vertices and
+// instances alone, the rounds, and the slots.
 struct BatchDev {
-  int32_t *vbeg = nullptr, *lab0 = nullptr, *lab1 = nullptr, *cc_out = nullptr;
-  int32_t *pr_steps = nullptr, *cc_steps = nullptr;
-  int32_t *inv = nullptr, *perm = nullptr, *od = nullptr, *n_units = nullptr;
-  BatchUnit* units = nullptr;
-  unsigned long long *rounds = nullptr, *round_base = nullptr;
+  unsigned char* block = nullptr;
   uint2* ids = nullptr;
-  float *pr0 = nullptr, *pr1 = nullptr, *con0 = nullptr, *con1 = nullptr, *pr_out = nullptr;
-  unsigned int* ctr = nullptr;
   int2* slots = nullptr;
-  unsigned int* team = nullptr;     // 4 per instance
-  unsigned int* abort = nullptr;
+  float* pr_out = nullptr;
+  int32_t *cc_out = nullptr, *pr_steps = nullptr, *cc_steps = nullptr;
+  unsigned long long *rounds = nullptr, *round_base = nullptr;
   std::vector<int32_t> order;       // instances, longest first
   std::vector<int64_t> work;        // per instance: edges + vertices
+  int32_t most_vertices = 0;        // of an instance
+  int sort_split = 1;               // CTAs that sort one
   ~BatchDev() {
-    dev_free(&vbeg);
+    dev_free(&block);
     dev_free(&slots);
-    dev_free(&team);
-    dev_free(&abort);
-    dev_free(&lab0);
-    dev_free(&lab1);
-    dev_free(&cc_out);
-    dev_free(&pr_steps);
-    dev_free(&cc_steps);
-    dev_free(&inv);
-    dev_free(&perm);
-    dev_free(&od);
-    dev_free(&n_units);
-    dev_free(&units);
-    dev_free(&rounds);
-    dev_free(&round_base);
     dev_free(&ids);
-    dev_free(&pr0);
-    dev_free(&pr1);
-    dev_free(&con0);
-    dev_free(&con1);
-    dev_free(&pr_out);
-    dev_free(&ctr);
   }
 };
 
@@ -744,63 +775,77 @@ gx_status batch_prepare(gx_engine* e, int32_t n, const int32_t* vbeg, BatchDev& 
     return e->off[vbeg[x + 1]] - e->off[vbeg[x]] > e->off[vbeg[y + 1]] - e->off[vbeg[y]];
   });
   d.work.resize(n);
-  for (int32_t i = 0; i < n; ++i) d.work[i] = (e->off[vbeg[i + 1]] - e->off[vbeg[i]]) + (vbeg[i + 1] - vbeg[i]);
-  GX_TRY(dev_alloc(&d.vbeg, static_cast<size_t>(n) + 1));
-  GX_TRY(dev_alloc(&d.team, 4 * static_cast<size_t>(n)));
-  GX_TRY(dev_alloc(&d.abort, 1));
-  GX_TRY(dev_alloc(&d.lab0, static_cast<size_t>(V)));
-  GX_TRY(dev_alloc(&d.lab1, static_cast<size_t>(V)));
-  GX_TRY(dev_alloc(&d.cc_out, static_cast<size_t>(V)));
-  GX_TRY(dev_alloc(&d.pr0, static_cast<size_t>(V)));
-  GX_TRY(dev_alloc(&d.pr1, static_cast<size_t>(V)));
-  GX_TRY(dev_alloc(&d.con0, static_cast<size_t>(V)));
-  GX_TRY(dev_alloc(&d.con1, static_cast<size_t>(V)));
-  GX_TRY(dev_alloc(&d.pr_out, static_cast<size_t>(V)));
-  GX_TRY(dev_alloc(&d.pr_steps, static_cast<size_t>(n)));
-  GX_TRY(dev_alloc(&d.cc_steps, static_cast<size_t>(n)));
-  GX_TRY(dev_alloc(&d.ctr, 1));
-  GX_TRY(dev_alloc(&d.inv, static_cast<size_t>(V)));
-  GX_TRY(dev_alloc(&d.perm, static_cast<size_t>(V)));
-  GX_TRY(dev_alloc(&d.od, static_cast<size_t>(V)));
-  GX_TRY(dev_alloc(&d.units, static_cast<size_t>(V)));
-  GX_TRY(dev_alloc(&d.n_units, static_cast<size_t>(n)));
-  GX_TRY(dev_alloc(&d.rounds, static_cast<size_t>(n)));
-  GX_TRY(dev_alloc(&d.round_base, static_cast<size_t>(n)));
-  GX_CUDA(cudaMemcpy(d.vbeg, vbeg, sizeof(int32_t) * (n + 1), cudaMemcpyHostToDevice));
-  // Every edge must stay inside its instance (a block-diagonal CSC).
-  GX_CUDA(cudaMemset(d.ctr, 0, sizeof(unsigned int)));
-  batch_check_kernel<<<e->n_sm * 4, 512, 0, e->s_comp>>>(e->d_off, e->d_col, d.vbeg, n, d.ctr);
-  unsigned int bad = 0;
-  GX_CUDA(cudaMemcpyAsync(&bad, d.ctr, sizeof(bad), cudaMemcpyDeviceToHost, e->s_comp));
-  GX_CUDA(cudaStreamSynchronize(e->s_comp));
-  if (bad) return fail(GX_ERR_INVALID, "gx_batch: %u edges cross instance boundaries", bad);
+  for (int32_t i = 0; i < n; ++i) {
+    d.work[i] = (e->off[vbeg[i + 1]] - e->off[vbeg[i]]) + (vbeg[i + 1] - vbeg[i]);
+    d.most_vertices = std::max(d.most_vertices, vbeg[i + 1] - vbeg[i]);
+  }
+  size_t at = 0;
+  auto place = [&](size_t count, size_t bytes) {
+    const size_t x = at;
+    at += (count * bytes + 255) & ~size_t(255);
+    return x;
+  };
+  const size_t v = static_cast<size_t>(V), m = static_cast<size_t>(n);
+  const size_t o_vbeg = place(m + 1, 4), o_team = place(4 * m, 4), o_abort = place(1, 4), o_ctr = place(1, 4);
+  const size_t o_lab0 = place(v, 4), o_lab1 = place(v, 4), o_cc = place(v, 4), o_pr0 = place(v, 4), o_pr1 = place(v, 4),
+               o_con0 = place(v, 4), o_con1 = place(v, 4), o_pr = place(v, 4);
+  const size_t o_prs = place(m, 4), o_ccs = place(m, 4);
+  const size_t o_inv = place(v, 4), o_perm = place(v, 4), o_od = place(v, 4), o_units = place(v, sizeof(BatchUnit));
+  const size_t o_nu = place(m, 4), o_rounds = place(m, 8), o_base = place(m, 8);
+  // Several CTAs sort an instance where there are few instances, or one that
+  // would keep a single CTA long after the others (unless the counts of all
+  // of them, 1 KB each, were many).
+  if (n < 65536 && d.most_vertices > (n < e->n_sm ? 4 : 64) * kBatchSortThreads)
+    d.sort_split = batch_split(d.most_vertices, 4 * kBatchSortThreads, e->n_sm * 4, n, 8);
+  const size_t o_classes = place(d.sort_split > 1 ? 2 * kClasses * m : 0, 4);
+  GX_TRY(dev_alloc(&d.block, at));
   a = BatchArgs{};
-  a.off = e->d_off;
-  a.col = e->d_col;
-  a.outdeg = e->d_outdeg;
-  a.vbeg = d.vbeg;
-  a.n_inst = n;
-  a.ctr = d.ctr;
-  a.team = d.team;
-  a.abort = d.abort;
-  a.spin_limit = e->cfg.wait_limit;  // polls of at least 64 ns each
-  a.pr0 = d.pr0;
-  a.pr1 = d.pr1;
-  a.con0 = d.con0;
-  a.con1 = d.con1;
-  a.lab0 = d.lab0;
-  a.lab1 = d.lab1;
+  auto as = [&](size_t o, auto*& p) { p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(d.block + o); };
+  int32_t* d_vbeg = nullptr;
+  as(o_vbeg, d_vbeg);
+  as(o_team, a.team);
+  as(o_abort, a.abort);
+  as(o_ctr, a.ctr);
+  as(o_lab0, a.lab0);
+  as(o_lab1, a.lab1);
+  as(o_pr0, a.pr0);
+  as(o_pr1, a.pr1);
+  as(o_con0, a.con0);
+  as(o_con1, a.con1);
+  as(o_inv, a.inv);
+  as(o_perm, a.perm);
+  as(o_od, a.od);
+  as(o_units, a.units);
+  as(o_nu, a.n_units);
+  as(o_pr, d.pr_out);
+  as(o_cc, d.cc_out);
+  as(o_prs, d.pr_steps);
+  as(o_ccs, d.cc_steps);
+  as(o_rounds, d.rounds);
+  as(o_base, d.round_base);
+  as(o_classes, a.classes);
+  a.vbeg = d_vbeg;
   a.pr_out = d.pr_out;
   a.cc_out = d.cc_out;
   a.pr_steps = d.pr_steps;
   a.cc_steps = d.cc_steps;
-  a.inv = d.inv;
-  a.perm = d.perm;
-  a.od = d.od;
-  a.units = d.units;
-  a.n_units = d.n_units;
   a.rounds = d.rounds;
   a.round_base = d.round_base;
+  a.off = e->d_off;
+  a.col = e->d_col;
+  a.outdeg = e->d_outdeg;
+  a.n_inst = n;
+  a.spin_limit = e->cfg.wait_limit;  // polls of at least 64 ns each
+  GX_CUDA(cudaMemcpyAsync(d_vbeg, vbeg, sizeof(int32_t) * (m + 1), cudaMemcpyHostToDevice, e->s_comp));
+  // Every edge must stay inside its instance (a block-diagonal CSC).
+  GX_CUDA(cudaMemsetAsync(a.ctr, 0, sizeof(unsigned int), e->s_comp));
+  const int ctas = e->n_sm * 4, split = batch_split(d.work[order[0]], 8192, ctas, n, 4);
+  batch_check_kernel<<<split * std::min(n, ctas / split), 512, 0, e->s_comp>>>(e->d_off, e->d_col, d_vbeg, n, split, a.ctr);
+  GX_CUDA(cudaGetLastError());
+  unsigned int bad = 0;
+  GX_CUDA(cudaMemcpyAsync(&bad, a.ctr, sizeof(bad), cudaMemcpyDeviceToHost, e->s_comp));
+  GX_CUDA(cudaStreamSynchronize(e->s_comp));
+  if (bad) return fail(GX_ERR_INVALID, "gx_batch: %u edges cross instance boundaries", bad);
   return GX_OK;
 }
 
@@ -823,7 +868,11 @@ gx_status batch_table_bytes(gx_engine* e, const gx_batch_tuning& t, int* bytes) 
 // threads per SM, or one of 1024 with twice the table where most of the work
 // is in instances that the default's table does not hold whole (512 R-MAT
 // instances of scales 10 to 17: 32.6 -> 26.8 ms a call; 2000 of scales 6 to
-// 12, which it does hold: 2.2 ms against 2.6).
+// 12, which it does hold: 2.2 ms against 2.6).  Instances of at most kTinyMost
+// vertices are a warp or two of work between barriers: where there are waves of
+// them, CTAs of 64 threads, 16 to an SM, keep eight times as many going (20000
+// of 8 vertices: a call of 5.0 -> 2.1 ms).
+constexpr int kTinyMost = 256;
 gx_status batch_default_schedule(gx_engine* e, int32_t n, const int32_t* vbeg, const BatchDev& d, gx_batch_tuning* t) {
   gx_batch_tuning_default(t);
   int smem = 0;
@@ -833,13 +882,16 @@ gx_status batch_default_schedule(gx_engine* e, int32_t n, const int32_t* vbeg, c
   if (out > in) {
     t->threads = 1024;
     t->ctas_per_sm = 1;
+  } else if (d.most_vertices <= kTinyMost && n >= 8 * e->n_sm) {
+    t->threads = 64;
+    t->ctas_per_sm = 16;
   }
   return GX_OK;
 }
 
 // One persistent launch (plus its cursor and team-state resets), captured as
 // a CUDA graph.  The grid holds no more CTAs than are resident at once.
-gx_status batch_launch(gx_engine* e, BatchDev& d, BatchArgs& a, const gx_batch_tuning& t, float* ms) {
+gx_status batch_launch(gx_engine* e, const int32_t* vbeg, BatchDev& d, BatchArgs& a, const gx_batch_tuning& t, float* ms) {
   cudaStream_t s = e->s_comp;
   int per_sm = 0;
   int smem = 0;
@@ -871,20 +923,33 @@ gx_status batch_launch(gx_engine* e, BatchDev& d, BatchArgs& a, const gx_batch_t
   std::unique_ptr<CUevent_st, cudaError_t (*)(cudaEvent_t)> e0_g(e0, cudaEventDestroy), e1_g(e1, cudaEventDestroy);
   cudaEventRecord(e0, s);
   // The instances rewritten for this schedule.
-  batch_sort_kernel<<<std::min(a.n_inst, e->n_sm * 4), kBatchSortThreads, 0, s>>>(a);
+  const int32_t n = a.n_inst;
+  const int64_t longest = d.work[d.order[0]];
+  if (d.sort_split == 1) {
+    const int threads = d.most_vertices <= 4 * kSortSmall ? kSortSmall : kBatchSortThreads;
+    batch_sort_kernel<kSortAll><<<std::min(n, e->n_sm * (2048 / threads)), threads, 0, s>>>(a, 1);
+  } else {
+    const int split = d.sort_split, grid = split * std::min(n, std::max(1, e->n_sm * 4 / split));
+    GX_CUDA(cudaMemsetAsync(a.classes, 0, sizeof(int) * 2 * kClasses * n, s));
+    GX_CUDA(cudaMemsetAsync(a.rounds, 0, sizeof(unsigned long long) * n, s));
+    batch_sort_kernel<kSortCount><<<grid, kBatchSortThreads, 0, s>>>(a, split);
+    batch_sort_kernel<kSortPlace><<<grid, kBatchSortThreads, 0, s>>>(a, split);
+    batch_sort_kernel<kSortUnits><<<grid, kBatchSortThreads, 0, s>>>(a, split);
+  }
   GX_CUDA(cudaGetLastError());
-  std::vector<unsigned long long> blocks_of(static_cast<size_t>(a.n_inst)), base(static_cast<size_t>(a.n_inst));
-  GX_CUDA(cudaMemcpyAsync(blocks_of.data(), d.rounds, sizeof(unsigned long long) * a.n_inst, cudaMemcpyDeviceToHost, s));
+  std::vector<unsigned long long> rounds_of(static_cast<size_t>(a.n_inst)), base(static_cast<size_t>(a.n_inst));
+  GX_CUDA(cudaMemcpyAsync(rounds_of.data(), d.rounds, sizeof(unsigned long long) * a.n_inst, cudaMemcpyDeviceToHost, s));
   GX_CUDA(cudaStreamSynchronize(s));
   unsigned long long n_blocks = 0;
   for (int32_t i = 0; i < a.n_inst; ++i) {
     base[i] = n_blocks;
-    n_blocks += blocks_of[i];
+    n_blocks += vbeg[i + 1] - vbeg[i] >= kBatchWide ? 2 * rounds_of[i] : rounds_of[i];
   }
   GX_TRY(dev_alloc(&d.ids, static_cast<size_t>(n_blocks) * 32));
   a.ids = d.ids;
   GX_CUDA(cudaMemcpyAsync(d.round_base, base.data(), sizeof(unsigned long long) * a.n_inst, cudaMemcpyHostToDevice, s));
-  batch_fill_kernel<<<std::min(a.n_inst, e->n_sm) * kFillSplit, 256, 0, s>>>(a);
+  const int ctas = e->n_sm * 8, split = batch_split(longest, 4096, ctas, n, 8);
+  batch_fill_kernel<<<split * std::min(n, ctas / split), 256, 0, s>>>(a, split);
   GX_CUDA(cudaGetLastError());
   // Every status counts: a graph that lacks the kernel would end well, with
   // the results as the memory happened to be.
@@ -963,7 +1028,7 @@ gx_status gx_batch_run(gx_engine* e, int32_t n_inst, const int32_t* inst_vbegin,
   a.lane_max = t.lane_max;
   a.damping = damping;
   float ms = 0;
-  GX_TRY(batch_launch(e, d, a, t, &ms));
+  GX_TRY(batch_launch(e, inst_vbegin, d, a, t, &ms));
   const int32_t V = e->V;
   if (pr_out) GX_TRY(copy_to_host(e, pr_out, d.pr_out, sizeof(float) * static_cast<size_t>(V)));
   if (cc_out) GX_TRY(copy_to_host(e, cc_out, d.cc_out, sizeof(int32_t) * static_cast<size_t>(V)));
@@ -1013,8 +1078,8 @@ gx_status gx_batch_autotune(gx_engine* e, int32_t n_inst, const int32_t* inst_vb
         gx_batch_tuning t{th, lm, cp};
         a.lane_max = lm;
         float ms = 0, ms2 = 0;
-        GX_TRY(batch_launch(e, d, a, t, &ms));   // warm
-        GX_TRY(batch_launch(e, d, a, t, &ms2));
+        GX_TRY(batch_launch(e, inst_vbegin, d, a, t, &ms));   // warm
+        GX_TRY(batch_launch(e, inst_vbegin, d, a, t, &ms2));
         ms = std::min(ms, ms2);
         char buf[160];
         snprintf(buf, sizeof(buf), "{\"threads\": %d, \"lane_max\": %d, \"ctas_per_sm\": %d, \"ms\": %.4f}", th, lm, cp,
