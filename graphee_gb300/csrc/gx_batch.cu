@@ -763,11 +763,27 @@ struct BatchDev {
   }
 };
 
-gx_status batch_prepare(gx_engine* e, int32_t n, const int32_t* vbeg, BatchDev& d, BatchArgs& a) {
-  const int32_t V = e->V;
-  if (vbeg[0] != 0 || vbeg[n] != V) return fail(GX_ERR_INVALID, "gx_batch: instance ranges must cover [0, V)");
-  for (int32_t i = 0; i < n; ++i)
-    if (vbeg[i + 1] <= vbeg[i]) return fail(GX_ERR_INVALID, "gx_batch: instance %d is empty or out of order", i);
+// Every edge must stay inside its instance (a block-diagonal CSC).  d_vbeg:
+// room for the n + 1 bounds, copied there first; ctr: a word.
+gx_status batch_check(gx_engine* e, int32_t n, const int32_t* vbeg, int32_t* d_vbeg, unsigned int* ctr) {
+  int64_t longest = 0;
+  for (int32_t i = 0; i < n; ++i) longest = std::max(longest, e->off[vbeg[i + 1]] - e->off[vbeg[i]]);
+  GX_CUDA(cudaMemcpyAsync(d_vbeg, vbeg, sizeof(int32_t) * (static_cast<size_t>(n) + 1), cudaMemcpyHostToDevice, e->s_comp));
+  GX_CUDA(cudaMemsetAsync(ctr, 0, sizeof(unsigned int), e->s_comp));
+  const int ctas = e->n_sm * 4, split = batch_split(longest, 8192, ctas, n, 4);
+  batch_check_kernel<<<split * std::min(n, ctas / split), 512, 0, e->s_comp>>>(e->d_off, e->d_col, d_vbeg, n, split, ctr);
+  GX_CUDA(cudaGetLastError());
+  unsigned int bad = 0;
+  GX_CUDA(cudaMemcpyAsync(&bad, ctr, sizeof(bad), cudaMemcpyDeviceToHost, e->s_comp));
+  GX_CUDA(cudaStreamSynchronize(e->s_comp));
+  if (bad) return fail(GX_ERR_INVALID, "gx_batch: %u edges cross instance boundaries", bad);
+  return GX_OK;
+}
+
+// Device memory and arguments for instances [0, n) of vbeg, whose first vertex
+// need not be the graph's.
+gx_status batch_prepare(gx_engine* e, int32_t n, const int32_t* vbeg, bool check, BatchDev& d, BatchArgs& a) {
+  const int32_t V = vbeg[n] - vbeg[0];
   std::vector<int32_t>& order = d.order;
   order.resize(n);
   std::iota(order.begin(), order.end(), 0);
@@ -836,16 +852,12 @@ gx_status batch_prepare(gx_engine* e, int32_t n, const int32_t* vbeg, BatchDev& 
   a.outdeg = e->d_outdeg;
   a.n_inst = n;
   a.spin_limit = e->cfg.wait_limit;  // polls of at least 64 ns each
+  // Indexed by the graph's vertices, of which they hold these instances'.
+  for (float** x : {&a.pr0, &a.pr1, &a.con0, &a.con1, &a.pr_out}) *x -= vbeg[0];
+  for (int32_t** x : {&a.lab0, &a.lab1, &a.cc_out, &a.inv, &a.perm, &a.od}) *x -= vbeg[0];
+  a.units -= vbeg[0];
+  if (check) return batch_check(e, n, vbeg, d_vbeg, a.ctr);
   GX_CUDA(cudaMemcpyAsync(d_vbeg, vbeg, sizeof(int32_t) * (m + 1), cudaMemcpyHostToDevice, e->s_comp));
-  // Every edge must stay inside its instance (a block-diagonal CSC).
-  GX_CUDA(cudaMemsetAsync(a.ctr, 0, sizeof(unsigned int), e->s_comp));
-  const int ctas = e->n_sm * 4, split = batch_split(d.work[order[0]], 8192, ctas, n, 4);
-  batch_check_kernel<<<split * std::min(n, ctas / split), 512, 0, e->s_comp>>>(e->d_off, e->d_col, d_vbeg, n, split, a.ctr);
-  GX_CUDA(cudaGetLastError());
-  unsigned int bad = 0;
-  GX_CUDA(cudaMemcpyAsync(&bad, a.ctr, sizeof(bad), cudaMemcpyDeviceToHost, e->s_comp));
-  GX_CUDA(cudaStreamSynchronize(e->s_comp));
-  if (bad) return fail(GX_ERR_INVALID, "gx_batch: %u edges cross instance boundaries", bad);
   return GX_OK;
 }
 
@@ -873,16 +885,21 @@ gx_status batch_table_bytes(gx_engine* e, const gx_batch_tuning& t, int* bytes) 
 // them, CTAs of 64 threads, 16 to an SM, keep eight times as many going (20000
 // of 8 vertices: a call of 5.0 -> 2.1 ms).
 constexpr int kTinyMost = 256;
-gx_status batch_default_schedule(gx_engine* e, int32_t n, const int32_t* vbeg, const BatchDev& d, gx_batch_tuning* t) {
+gx_status batch_default_schedule(gx_engine* e, int32_t n, const int32_t* vbeg, gx_batch_tuning* t) {
   gx_batch_tuning_default(t);
   int smem = 0;
   GX_TRY(batch_table_bytes(e, *t, &smem));
   int64_t in = 0, out = 0;
-  for (int32_t i = 0; i < n; ++i) (vbeg[i + 1] - vbeg[i] < smem / 4 ? in : out) += d.work[i];
+  int32_t most = 0;
+  for (int32_t i = 0; i < n; ++i) {
+    const int32_t v = vbeg[i + 1] - vbeg[i];
+    (v < smem / 4 ? in : out) += e->off[vbeg[i + 1]] - e->off[vbeg[i]] + v;
+    most = std::max(most, v);
+  }
   if (out > in) {
     t->threads = 1024;
     t->ctas_per_sm = 1;
-  } else if (d.most_vertices <= kTinyMost && n >= 8 * e->n_sm) {
+  } else if (most <= kTinyMost && n >= 8 * e->n_sm) {
     t->threads = 64;
     t->ctas_per_sm = 16;
   }
@@ -994,6 +1011,70 @@ gx_status check_tuning(const gx_batch_tuning& t) {
   return GX_OK;
 }
 
+// One call, or one schedule of the autotuner.
+struct BatchCall {
+  const int32_t* vbeg;
+  int32_t n, pr_iters, cc_max;
+  double damping;
+  gx_batch_tuning tuning;
+  float* pr_out = nullptr;         // nullable, as are the others
+  int32_t *cc_out = nullptr, *pr_steps = nullptr, *cc_steps = nullptr;
+  bool checked = false;            // batch_check
+  float ms = 0;
+  int32_t launches = 0;
+};
+
+gx_status batch_ranges(const gx_engine* e, int32_t n, const int32_t* vbeg) {
+  if (vbeg[0] != 0 || vbeg[n] != e->V) return fail(GX_ERR_INVALID, "gx_batch: instance ranges must cover [0, V)");
+  for (int32_t i = 0; i < n; ++i)
+    if (vbeg[i + 1] <= vbeg[i]) return fail(GX_ERR_INVALID, "gx_batch: instance %d is empty or out of order", i);
+  return GX_OK;
+}
+
+// Instances [i0, i1) at once, or, where the device has no room for that (the
+// rewritten lists take some 4 bytes an edge, the arrays 60 a vertex), one half
+// of the work after the other.
+gx_status batch_range(gx_engine* e, BatchCall& c, int32_t i0, int32_t i1) {
+  const int32_t n = i1 - i0, v0 = c.vbeg[i0], v1 = c.vbeg[i1];
+  const int32_t* vbeg = c.vbeg + i0;
+  auto run = [&]() -> gx_status {
+    BatchDev d;
+    BatchArgs a;
+    GX_TRY(batch_prepare(e, n, vbeg, !c.checked, d, a));
+    c.checked = true;
+    a.pr_iters = c.pr_iters;
+    a.cc_max = c.cc_max;
+    a.lane_max = c.tuning.lane_max;
+    a.damping = c.damping;
+    float ms = 0;
+    GX_TRY(batch_launch(e, vbeg, d, a, c.tuning, &ms));
+    c.ms += ms;
+    ++c.launches;
+    const size_t v = static_cast<size_t>(v1 - v0), m = static_cast<size_t>(n);
+    if (c.pr_out) GX_TRY(copy_to_host(e, c.pr_out + v0, d.pr_out, sizeof(float) * v));
+    if (c.cc_out) GX_TRY(copy_to_host(e, c.cc_out + v0, d.cc_out, sizeof(int32_t) * v));
+    if (c.pr_steps) GX_CUDA(cudaMemcpy(c.pr_steps + i0, d.pr_steps, sizeof(int32_t) * m, cudaMemcpyDeviceToHost));
+    if (c.cc_steps) GX_CUDA(cudaMemcpy(c.cc_steps + i0, d.cc_steps, sizeof(int32_t) * m, cudaMemcpyDeviceToHost));
+    return GX_OK;
+  };
+  const gx_status st = run();
+  if (st != GX_ERR_OOM || n == 1) return st;
+  if (!c.checked) {  // all instances, before any results are written
+    struct Words {
+      int32_t* p = nullptr;
+      ~Words() { dev_free(&p); }
+    } w;
+    GX_TRY(dev_alloc(&w.p, static_cast<size_t>(c.n) + 2));
+    GX_TRY(batch_check(e, c.n, c.vbeg, w.p, reinterpret_cast<unsigned int*>(w.p + c.n + 1)));
+    c.checked = true;
+  }
+  const int64_t half = (e->off[v0] + e->off[v1] + v0 + v1) / 2;
+  int32_t mid = i0 + 1;
+  while (mid < i1 - 1 && e->off[c.vbeg[mid]] + c.vbeg[mid] < half) ++mid;
+  GX_TRY(batch_range(e, c, i0, mid));
+  return batch_range(e, c, mid, i1);
+}
+
 }  // namespace
 
 extern "C" {
@@ -1019,22 +1100,15 @@ gx_status gx_batch_run(gx_engine* e, int32_t n_inst, const int32_t* inst_vbegin,
   GX_TRY(check_tuning(t));
   GX_CUDA(cudaSetDevice(e->dev));
   BlockBound bound(e->block_bound);
-  BatchDev d;
-  BatchArgs a;
-  GX_TRY(batch_prepare(e, n_inst, inst_vbegin, d, a));
-  if (!tuning) GX_TRY(batch_default_schedule(e, n_inst, inst_vbegin, d, &t));
-  a.pr_iters = pr_iters;
-  a.cc_max = cc_max_iter;
-  a.lane_max = t.lane_max;
-  a.damping = damping;
-  float ms = 0;
-  GX_TRY(batch_launch(e, inst_vbegin, d, a, t, &ms));
-  const int32_t V = e->V;
-  if (pr_out) GX_TRY(copy_to_host(e, pr_out, d.pr_out, sizeof(float) * static_cast<size_t>(V)));
-  if (cc_out) GX_TRY(copy_to_host(e, cc_out, d.cc_out, sizeof(int32_t) * static_cast<size_t>(V)));
+  GX_TRY(batch_ranges(e, n_inst, inst_vbegin));
+  if (!tuning) GX_TRY(batch_default_schedule(e, n_inst, inst_vbegin, &t));
   std::vector<int32_t> ps(n_inst), cs(n_inst);
-  GX_CUDA(cudaMemcpy(ps.data(), d.pr_steps, sizeof(int32_t) * n_inst, cudaMemcpyDeviceToHost));
-  GX_CUDA(cudaMemcpy(cs.data(), d.cc_steps, sizeof(int32_t) * n_inst, cudaMemcpyDeviceToHost));
+  BatchCall c{inst_vbegin, n_inst, pr_iters, cc_max_iter, damping, t};
+  c.pr_out = pr_out;
+  c.cc_out = cc_out;
+  c.pr_steps = ps.data();
+  c.cc_steps = cs.data();
+  GX_TRY(batch_range(e, c, 0, n_inst));
   if (pr_steps) memcpy(pr_steps, ps.data(), sizeof(int32_t) * n_inst);
   if (cc_steps) memcpy(cc_steps, cs.data(), sizeof(int32_t) * n_inst);
   if (stats) {
@@ -1044,9 +1118,9 @@ gx_status gx_batch_run(gx_engine* e, int32_t n_inst, const int32_t* inst_vbegin,
       edges += (e->off[inst_vbegin[i + 1]] - e->off[inst_vbegin[i]]) * static_cast<int64_t>(ps[i] + cs[i]);
     stats->iterations = *std::max_element(ps.begin(), ps.end()) + *std::max_element(cs.begin(), cs.end());
     stats->edges_scanned = edges;
-    stats->ms_total = ms;
-    stats->ms_compute = ms;
-    stats->kernel_launches = 1;  // the supersteps; the call's preparation (check, sort, fill) is not counted
+    stats->ms_total = c.ms;
+    stats->ms_compute = c.ms;
+    stats->kernel_launches = c.launches;  // the supersteps; the preparation (check, sort, fill) is not counted
   }
   return GX_OK;
 }
@@ -1059,12 +1133,8 @@ gx_status gx_batch_autotune(gx_engine* e, int32_t n_inst, const int32_t* inst_vb
   if (e->relabeled) return fail(GX_ERR_STATE, "gx_batch_autotune: the engine renumbered the vertices (config.relabel)");
   GX_CUDA(cudaSetDevice(e->dev));
   BlockBound bound(e->block_bound);
-  BatchDev d;
-  BatchArgs a;
-  GX_TRY(batch_prepare(e, n_inst, inst_vbegin, d, a));
-  a.pr_iters = pr_iters;
-  a.cc_max = cc_max_iter;
-  a.damping = 0.85;
+  GX_TRY(batch_ranges(e, n_inst, inst_vbegin));
+  bool checked = false;
   const int threads_c[] = {256, 512, 1024};
   const int lane_c[] = {16, 32, 64};
   const int cps_c[] = {1, 2, 4};
@@ -1076,11 +1146,14 @@ gx_status gx_batch_autotune(gx_engine* e, int32_t n_inst, const int32_t* inst_vb
       for (int cp : cps_c) {
         if (th * cp > 2048) continue;
         gx_batch_tuning t{th, lm, cp};
-        a.lane_max = lm;
-        float ms = 0, ms2 = 0;
-        GX_TRY(batch_launch(e, inst_vbegin, d, a, t, &ms));   // warm
-        GX_TRY(batch_launch(e, inst_vbegin, d, a, t, &ms2));
-        ms = std::min(ms, ms2);
+        float ms = 0;
+        for (int warm = 1; warm >= 0; --warm) {
+          BatchCall c{inst_vbegin, n_inst, pr_iters, cc_max_iter, 0.85, t};
+          c.checked = checked;
+          GX_TRY(batch_range(e, c, 0, n_inst));
+          checked = true;
+          ms = warm ? c.ms : std::min(ms, c.ms);
+        }
         char buf[160];
         snprintf(buf, sizeof(buf), "{\"threads\": %d, \"lane_max\": %d, \"ctas_per_sm\": %d, \"ms\": %.4f}", th, lm, cp,
                  ms);

@@ -270,7 +270,11 @@ void gx_batch_tuning_default(gx_batch_tuning* t);
  * changes (at most cc_max_iter), each with GraphPS::run's stop rule
  * (GraphPS.h:383) per instance.  pr_out float[V], cc_out int32[V]
  * (instance-local labels), pr_steps / cc_steps int32[n_inst]; all
- * nullable.  No reference counterpart for the batching itself. */
+ * nullable.  The call holds a rewritten copy of the lists (about 2 to 5
+ * bytes an edge and 60 a vertex); without room for all of it, the instances
+ * are run in parts, a launch each, down to one instance (GX_ERR_OOM when
+ * the device has no room for that one).  No reference counterpart for the
+ * batching itself. */
 gx_status gx_batch_run(gx_engine* e, int32_t n_inst, const int32_t* inst_vbegin, int32_t pr_iters,
                        int32_t cc_max_iter, double damping, const gx_batch_tuning* tuning,
                        float* pr_out, int32_t* cc_out, int32_t* pr_steps, int32_t* cc_steps,

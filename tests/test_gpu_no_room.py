@@ -58,3 +58,38 @@ def test_streaming_slots_of_one_shard(weighted):
         st = e.run(gx.APP_SSSP, 1000, source=1, weighted=weighted)
         assert np.array_equal(e.values(), O.run(O.SSSP, *a, 1000, weights=g.weights, source=1)[0])
         assert st["pull_launches"] >= g.P // 2  # several groups a step
+
+
+@pytest.mark.parametrize("parts", [2, 7])
+def test_batch_in_parts(parts):
+    """No room for all instances' lists at once: part of them after part, the same results; none for one: an error."""
+    g, vb = gx.batch_graph(48, scales=(6, 13), edge_factors=(8, 16), seed=5)
+    with gx.Engine() as e:
+        e.load(g)
+        want = e.batch_run(vb, 20, 1000)
+        assert want[4]["kernel_launches"] == 1
+        e.set_bound(gx.BOUND_BLOCK, 64 * g.V // parts + 100000)
+        got = e.batch_run(vb, 20, 1000, tuning={"threads": 256})
+        assert got[4]["kernel_launches"] >= parts
+        for x, y in zip(got[:4], want[:4]):
+            assert np.array_equal(x, y)
+        best, ms = e.batch_autotune(vb, 2, 5)
+        assert ms > 0
+        e.set_bound(gx.BOUND_BLOCK, 60 * 64)
+        with pytest.raises(gx.GxError) as ei:
+            e.batch_run(vb, 20, 1000)
+        assert ei.value.status == gx.GX_ERR_OOM
+
+
+def test_batch_in_parts_checks_all_first():
+    """An edge that leaves the last instance: an error before the first part's results are written."""
+    g, vb = gx.batch_graph(16, scales=(10, 10), edge_factors=(8, 8), seed=2)
+    wrong = vb.copy()
+    wrong[-2] += 100
+    with gx.Engine() as e:
+        e.load(g)
+        for room in (0, 30 * g.V):
+            e.set_bound(gx.BOUND_BLOCK, room)
+            pr = np.full(g.V, 7, np.float32)
+            st = gx.lib().gx_batch_run(e._h, 16, gx._ptr(wrong), 5, 5, 0.85, None, gx._ptr(pr), None, None, None, None)
+            assert st == gx.GX_ERR_INVALID and (pr == 7).all()
