@@ -8,6 +8,8 @@
 //     as out-neighbour;
 //  2. write N+(v) in the room its CSC list leaves (no order is needed below,
 //     so no count pass or scan comes first), padded to whole 16-byte pieces;
+//     where the device has no room for that, the lists are counted first and
+//     laid end to end, in half of it;
 //  3. count sum over edges {x, y} of |N+(x) n N+(y)|: the end with the longer
 //     N+ (x) is staged, the shorter list is scanned (half the probes of
 //     scanning N+(v) for every u -> v on R-MAT).  A vertex with much to scan
@@ -109,12 +111,21 @@ __device__ __forceinline__ int32_t tc_mixed(const TcArgs& a, int32_t y) {
 // Where N+(v) begins: at least as much room as its list, whole 16-byte pieces.
 __device__ __forceinline__ int64_t tc_start(int64_t off, int32_t v) { return (off + 4 * static_cast<int64_t>(v) + 3) & ~3ll; }
 
+// How N+ is laid out: in the room of the CSC's lists, or end to end from
+// info[v].start; or only counted, for the latter.
+enum : int { kTcSpaced, kTcPacked, kTcCount };
+template <int MODE>
+__device__ __forceinline__ int64_t tc_place(const TcArgs& a, int32_t v) {
+  return MODE == kTcSpaced ? tc_start(a.off[v], v) : MODE == kTcPacked ? a.info[v].start : 0;
+}
+
 // The engine's units (tiles of at most 32 vertices, chunks of heavy ones), a
 // warp each: the unit's entries 128 at a time, every stage's loads in flight
 // together; an entry's vertex is found among the lanes' offsets, and the
 // entries kept for one vertex reserve their places with one atomic.
 // (A warp per vertex, with R-MAT's hubs, took 0.83 + 0.95 ms to count and fill
 // at symmetric scale 20.)
+template <int MODE>
 __global__ void __launch_bounds__(kTcThreads) tc_fill_kernel(const __grid_constant__ TcArgs a) {
   const int lane = threadIdx.x & 31;
   for (;;) {
@@ -147,7 +158,7 @@ __global__ void __launch_bounds__(kTcThreads) tc_fill_kernel(const __grid_consta
     const int total = __shfl_sync(0xffffffffu, pre, 31);
     pre -= len;
     const int32_t dv = len > 0 ? (a.rank ? a.rank[v] : a.deg[v]) : 0;
-    const int64_t to = tc_start(a.off[v], v);
+    const int64_t to = tc_place<MODE>(a, v);
     for (int k0 = 0; k0 < total; k0 += 128) {
       int l[4], lo[4];
       int32_t y[4], dy[4];
@@ -179,6 +190,7 @@ __global__ void __launch_bounds__(kTcThreads) tc_fill_kernel(const __grid_consta
         const unsigned m = __ballot_sync(0xffffffffu, keep) & mine;
         int at = 0;
         if (k < total && lane == first && m) at = atomicAdd(a.n + x, __popc(m));
+        if (MODE == kTcCount) continue;
         at = __shfl_sync(0xffffffffu, at, first < 32 ? first : 0);
         if (keep) a.dcol[tx + at + __popc(m & ((1u << lane) - 1u))] = a.rank ? dy[j] : tc_mixed(a, y[j]);
       }
@@ -186,14 +198,27 @@ __global__ void __launch_bounds__(kTcThreads) tc_fill_kernel(const __grid_consta
   }
 }
 
+// Packed lists: their lengths in whole 16-byte pieces, and where they begin.
+__global__ void tc_pieces_kernel(const __grid_constant__ TcArgs a, uint32_t* pieces) {
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < a.V; v += gridDim.x * blockDim.x)
+    pieces[v] = (static_cast<uint32_t>(a.n[v]) + 3u) >> 2;
+}
+__global__ void tc_starts_kernel(const __grid_constant__ TcArgs a, const unsigned long long* at) {
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < a.V; v += gridDim.x * blockDim.x) {
+    a.info[v].start = 4 * static_cast<int64_t>(at[v]);
+    a.n[v] = 0;  // counted again as the lists are written
+  }
+}
+
 // Padding, scan descriptors and the vertices to count from.
+template <int MODE>
 __global__ void tc_list_kernel(const __grid_constant__ TcArgs a) {
   const int lane = threadIdx.x & 31;
   for (int v0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); v0 < a.V; v0 += gridDim.x * blockDim.x) {
     const int v = v0 + lane;
     bool big = false, small = false;
     if (v < a.V) {
-      TcInfo x{tc_start(a.off[v], v), a.n[v], 0};
+      TcInfo x{tc_place<MODE>(a, v), a.n[v], 0};
       a.info[v] = x;
       for (int k = x.n; k & 3; ++k) a.dcol[x.start + k] = kTcNone;
       const bool in = !a.rank || a.rank[v] >= a.base;
@@ -447,8 +472,9 @@ extern "C" gx_status gx_triangle_count(gx_engine* e, uint64_t* total, gx_run_sta
   const bool ranked = V > tc_bits(V);
   int vb = 1;
   while (vb < 31 && (int64_t(1) << vb) < V) ++vb;
-  // One block for all arrays.
-  TcBlock block;
+  // One block for all arrays; or, without room for it, one for those of a
+  // vertex, one that the sort gives back, and the packed lists' own.
+  TcBlock block, sort_block, list_block;
   size_t at = 0;
   auto place = [&](size_t bytes) {
     const size_t x = at;
@@ -461,12 +487,20 @@ extern "C" gx_status gx_triangle_count(gx_engine* e, uint64_t* total, gx_run_sta
   const size_t o_deg = place(4 * nv), o_n = place(4 * nv), o_info = place(sizeof(TcInfo) * nv);
   const size_t o_big = place(4 * nv), o_small = place(4 * nv), o_ctr = place(8 * sizeof(unsigned int)),
                o_out = place(2 * sizeof(unsigned long long));
-  const size_t o_dcol = place(sizeof(int32_t) * (static_cast<size_t>(e->E) + 4 * nv + 8));
-  const size_t o_rank = place(ranked ? 4 * nv : 0), o_keys = place(ranked ? 16 * nv : 0),
-               o_hist = place(ranked ? 4 * static_cast<size_t>(hist_n) : 0),
+  const size_t o_rank = place(ranked ? 4 * nv : 0), o_sort = at;
+  const size_t o_keys = place(ranked ? 16 * nv : 0), o_hist = place(ranked ? 4 * static_cast<size_t>(hist_n) : 0),
                o_offs = place(ranked ? 8 * static_cast<size_t>(hist_n) : 0),
-               o_part = place(ranked ? 8 * static_cast<size_t>(part_n) : 0);
-  GX_TRY(dev_alloc(&block.p, at));
+               o_part = place(ranked ? 8 * static_cast<size_t>(part_n) : 0), o_dcol = at;
+  place(sizeof(int32_t) * (static_cast<size_t>(e->E) + 4 * nv + 8));
+  gx_status room = dev_alloc(&block.p, at);
+  const bool packed = room == GX_ERR_OOM;
+  unsigned char* sort_at = block.p + o_sort;
+  if (packed) {
+    room = dev_alloc(&block.p, o_sort);
+    if (room == GX_OK && ranked) room = dev_alloc(&sort_block.p, o_dcol - o_sort);
+    sort_at = sort_block.p;
+  }
+  if (room != GX_OK) return room;
   TcArgs a{};
   a.off = e->d_off;
   a.col = e->d_col;
@@ -484,7 +518,7 @@ extern "C" gx_status gx_triangle_count(gx_engine* e, uint64_t* total, gx_run_sta
   a.small = reinterpret_cast<int32_t*>(block.p + o_small);
   a.ctr = reinterpret_cast<unsigned int*>(block.p + o_ctr);
   a.out = reinterpret_cast<unsigned long long*>(block.p + o_out);
-  a.dcol = reinterpret_cast<int32_t*>(block.p + o_dcol);
+  a.dcol = packed ? nullptr : reinterpret_cast<int32_t*>(block.p + o_dcol);
   a.bits = static_cast<int32_t>(tc_bits(V));
   a.base = V - a.bits;
   a.mask = vb >= 32 ? 0xffffffffu : (1u << vb) - 1u;
@@ -492,23 +526,46 @@ extern "C" gx_status gx_triangle_count(gx_engine* e, uint64_t* total, gx_run_sta
   GX_CUDA(cudaMemsetAsync(a.ctr, 0, 8 * sizeof(unsigned int), s));
   GX_CUDA(cudaMemsetAsync(a.out, 0, 2 * sizeof(unsigned long long), s));
   const int grid_v = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(e->n_sm * 8, (V + 255) / 256)));
-  unsigned long long* keys = reinterpret_cast<unsigned long long*>(block.p + o_keys);
+  unsigned long long* keys = reinterpret_cast<unsigned long long*>(sort_at);
   tc_degree_kernel<<<grid_v, 256, 0, s>>>(e->d_off, V, deg, a.n, ranked ? keys : nullptr, vb);
   if (ranked) {
     unsigned long long* sorted = nullptr;
-    GX_TRY(radix_sort_bits(keys, keys + nv, V, vb, 2 * vb, reinterpret_cast<uint32_t*>(block.p + o_hist),
-                           reinterpret_cast<unsigned long long*>(block.p + o_offs),
-                           reinterpret_cast<unsigned long long*>(block.p + o_part), s, &sorted));
+    GX_TRY(radix_sort_bits(keys, keys + nv, V, vb, 2 * vb, reinterpret_cast<uint32_t*>(sort_at + (o_hist - o_keys)),
+                           reinterpret_cast<unsigned long long*>(sort_at + (o_offs - o_keys)),
+                           reinterpret_cast<unsigned long long*>(sort_at + (o_part - o_keys)), s, &sorted));
     int32_t* rank = reinterpret_cast<int32_t*>(block.p + o_rank);
     tc_rank_kernel<<<grid_v, 256, 0, s>>>(sorted, (1ull << vb) - 1, V, rank);
     a.rank = rank;
   }
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tc_fill_kernel, kTcThreads, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tc_fill_kernel<kTcSpaced>, kTcThreads, 0);
   const int64_t grid_u = (static_cast<int64_t>(a.n_units) + kTcWarps - 1) / kTcWarps;
-  tc_fill_kernel<<<static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(std::max(1, per_sm) * e->n_sm, grid_u))),
-                   kTcThreads, 0, s>>>(a);
-  tc_list_kernel<<<grid_v, 256, 0, s>>>(a);
+  const int grid_fill = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(std::max(1, per_sm) * e->n_sm, grid_u)));
+  if (packed) {
+    dev_free(&sort_block.p);
+    tc_fill_kernel<kTcCount><<<grid_fill, kTcThreads, 0, s>>>(a);
+    // The lists' pieces end to end, in a block that the lists' then replaces.
+    uint32_t* pieces = reinterpret_cast<uint32_t*>(a.small);
+    GX_TRY(dev_alloc(&sort_block.p, 8 * (nv + static_cast<size_t>(part_n))));
+    unsigned long long* starts = reinterpret_cast<unsigned long long*>(sort_block.p);
+    tc_pieces_kernel<<<grid_v, 256, 0, s>>>(a, pieces);
+    GX_TRY(scan_u32(pieces, V, starts, starts + nv, s));
+    unsigned long long last = 0;
+    uint32_t last_n = 0;
+    GX_CUDA(cudaMemcpyAsync(&last, starts + nv - 1, sizeof(last), cudaMemcpyDeviceToHost, s));
+    GX_CUDA(cudaMemcpyAsync(&last_n, pieces + nv - 1, sizeof(last_n), cudaMemcpyDeviceToHost, s));
+    tc_starts_kernel<<<grid_v, 256, 0, s>>>(a, starts);
+    GX_CUDA(cudaMemsetAsync(a.ctr, 0, sizeof(unsigned int), s));  // the units' cursor
+    GX_CUDA(cudaStreamSynchronize(s));
+    dev_free(&sort_block.p);
+    GX_TRY(dev_alloc(&list_block.p, 16 * static_cast<size_t>(last + last_n)));
+    a.dcol = reinterpret_cast<int32_t*>(list_block.p);
+    tc_fill_kernel<kTcPacked><<<grid_fill, kTcThreads, 0, s>>>(a);
+    tc_list_kernel<kTcPacked><<<grid_v, 256, 0, s>>>(a);
+  } else {
+    tc_fill_kernel<kTcSpaced><<<grid_fill, kTcThreads, 0, s>>>(a);
+    tc_list_kernel<kTcSpaced><<<grid_v, 256, 0, s>>>(a);
+  }
   GX_CUDA(cudaGetLastError());
   // The CTAs' vertices on the copy stream, the warps' beside them.
   GX_CUDA(cudaEventRecord(listed, s));
@@ -542,7 +599,7 @@ extern "C" gx_status gx_triangle_count(gx_engine* e, uint64_t* total, gx_run_sta
     stats->edges_scanned = static_cast<int64_t>(res[1]);
     stats->ms_total = ms;
     stats->ms_compute = ms;
-    stats->kernel_launches = ranked ? 6 : 5;  // the sort's passes not counted
+    stats->kernel_launches = (ranked ? 6 : 5) + (packed ? 3 : 0);  // the sort's and scan's passes not counted
   }
   return GX_OK;
 }

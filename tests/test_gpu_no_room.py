@@ -93,3 +93,30 @@ def test_batch_in_parts_checks_all_first():
             pr = np.full(g.V, 7, np.float32)
             st = gx.lib().gx_batch_run(e._h, 16, gx._ptr(wrong), 5, 5, 0.85, None, gx._ptr(pr), None, None, None, None)
             assert st == gx.GX_ERR_INVALID and (pr == 7).all()
+
+
+@pytest.mark.parametrize("relabel", [0, 1])
+@pytest.mark.parametrize("V", [1, 5, 4096, (1 << 18) + 5])
+def test_triangles_packed(V, relabel):
+    """No room for N+ in the CSC's spacing: counted, packed and the same triangles; unranked and ranked ids."""
+    m = 12 * V if V < 1 << 18 else V // 2
+    src, dst = gx.rmat_edges(max(1, int(np.ceil(np.log2(V)))), max(m, 1), V)
+    hub = np.arange(V)
+    src = np.concatenate([src % V, np.zeros(V, np.int64), hub])
+    dst = np.concatenate([dst % V, hub, (hub + 1) % V])
+    off, col = gx.build_csc(V, src, dst, gx.BUILD_DROP_SELF | gx.BUILD_DEDUP | gx.BUILD_SYMMETRIZE)
+    g = gx.Graph(V, off, col, None, 3)
+    with gx.Engine(relabel=relabel) as e:
+        e.load(g)
+        want, st = e.triangle_count()
+        if V > 5:
+            assert want > V // 2
+            # 32 bytes a vertex (36, and the sort's 17, where ranked) and 4 an entry of N+ have room, one by one.
+            e.set_bound(gx.BOUND_BLOCK, 80 * V)
+            got, packed = e.triangle_count()
+            assert got == want and packed["edges_scanned"] == st["edges_scanned"]
+            assert packed["kernel_launches"] == st["kernel_launches"] + 3
+        e.set_bound(gx.BOUND_BLOCK, 200)
+        with pytest.raises(gx.GxError) as ei:
+            e.triangle_count()
+        assert ei.value.status == gx.GX_ERR_OOM
