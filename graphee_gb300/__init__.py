@@ -24,7 +24,7 @@ GX_OK, GX_ERR_INVALID, GX_ERR_IO, GX_ERR_FORMAT, GX_ERR_OOM, GX_ERR_CUDA, GX_ERR
 STATUS_NAMES = ["OK", "INVALID", "IO", "FORMAT", "OOM", "CUDA", "TIMEOUT", "NODEVICE", "STATE"]
 
 APP_PAGERANK_REF, APP_PAGERANK_STD, APP_SSSP, APP_CC, APP_INDEGREE = range(5)
-BOUND_BLOCK = 0
+BOUND_BLOCK, BOUND_STREAM_GROUP, BOUND_RUN_POLLS = range(3)
 BUILD_DROP_SELF, BUILD_DEDUP, BUILD_SYMMETRIZE = 1, 2, 4
 GPS_INF = 10000          # GraphMP/system/Global.h:50
 INF_WEIGHTED = 0xFFFFFFFF

@@ -642,14 +642,6 @@ gx_status encode_streamed(gx_engine* e, const int32_t* col) {
   return GX_OK;
 }
 
-// Streamed shards side by side travel and are swept together up to this many
-// edges, resident ones up to twice as many: a launch of one small shard lasts
-// some 30 us, whatever it holds, and a copy of 2 MB half as long as its calls.
-// Scale 24 in 256 shards, half of them streamed, a superstep: a shard at a time
-// 7.5 ms, groups of 1 M edges 6.0, 2 M 4.6, 4 M 3.5, 8 M 3.0, 16 M 3.0, of
-// which the link takes 2.6.
-constexpr int64_t kStreamGroup = int64_t(8) << 20;
-
 // Decides which shards stay in HBM under the budget (in shard order, like the
 // reference's insert-until-full edge cache, Global.h:170-244), uploads them,
 // and sets up the streaming ring for the rest.  When the plain shards exceed
@@ -727,7 +719,7 @@ gx_status plan_shards(gx_engine* e, const int32_t* src_col, bool col_on_device) 
     };
     // Without room for groups the slots hold the longest shard, and a group is
     // what fits one.
-    const int64_t group = std::max(max_stream, std::min(streamed_elems, kStreamGroup)) + 8;
+    const int64_t group = std::max(max_stream, std::min(streamed_elems, e->stream_group)) + 8;
     gx_status ring_st = ring(group);
     if (ring_st == GX_ERR_OOM && group > max_stream + 8) ring_st = ring(max_stream + 8);
     if (ring_st != GX_OK) return ring_st;
@@ -1154,7 +1146,7 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
         ra.run = e->d_run;
         // A step's own limit, well above any step's length: gx_run has no
         // other device-side wait, so a short config.wait_limit is not for it.
-        ra.wait_limit = std::max(e->cfg.wait_limit, 1u << 24);
+        ra.wait_limit = e->run_polls ? e->run_polls : std::max(e->cfg.wait_limit, 1u << 24);
         void (*fn)(RunArgs) = run_kernel<APP>;
         const PullShape shape = pull_shape(pa.u_end, occupancy_grid<APP>(e, reinterpret_cast<const void*>(fn)), kThreads);
         ra.pull.grab = shape.grab;
@@ -1303,7 +1295,7 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
       order.clear();
       for (int32_t p = 0; p < e->P;) {
         const bool resident = e->resident[p] != 0, active = on[p] != 0;
-        const int64_t most = resident ? 2 * kStreamGroup : e->slot_elems - 8;
+        const int64_t most = resident ? 2 * e->stream_group : e->slot_elems - 8;
         const bool alone = active && travels_compressed(p);
         int32_t q = p + 1;
         while (!alone && q < e->P && (e->resident[q] != 0) == resident && (on[q] != 0) == active &&
@@ -1596,8 +1588,13 @@ gx_status gx_set_bound(gx_engine* e, gx_bound which, int64_t value) {
   if (!e || value < 0) return fail(GX_ERR_INVALID, "gx_set_bound: engine NULL or value negative");
   switch (which) {
     case GX_BOUND_BLOCK: e->block_bound = static_cast<size_t>(value); return GX_OK;
+    case GX_BOUND_STREAM_GROUP: e->stream_group = value ? value : kStreamGroup; return GX_OK;
+    case GX_BOUND_RUN_POLLS:
+      if (value > UINT32_MAX) break;
+      e->run_polls = static_cast<uint32_t>(value);
+      return GX_OK;
   }
-  return fail(GX_ERR_INVALID, "gx_set_bound: unknown bound %d", static_cast<int>(which));
+  return fail(GX_ERR_INVALID, "gx_set_bound: bound %d to %lld", static_cast<int>(which), static_cast<long long>(value));
 }
 
 gx_status gx_release_cached_memory(int32_t device) {

@@ -185,6 +185,14 @@ inline int app_kind(const gx_run_params& p) {
   return -1;
 }
 
+// Streamed shards side by side travel and are swept together up to this many
+// edges, resident ones up to twice as many: a launch of one small shard lasts
+// some 30 us, whatever it holds, and a copy of 2 MB half as long as its calls.
+// Scale 24 in 256 shards, half of them streamed, a superstep: a shard at a time
+// 7.5 ms, groups of 1 M edges 6.0, 2 M 4.6, 4 M 3.5, 8 M 3.0, 16 M 3.0, of
+// which the link takes 2.6.
+constexpr int64_t kStreamGroup = int64_t(8) << 20;
+
 constexpr size_t kStageBytes = size_t(8) << 20, kStageSlots = 3, kStageFrom = size_t(128) << 20;
 
 }  // namespace gx
@@ -206,6 +214,8 @@ struct gx_engine {
   gx::hvec<int32_t> outdeg;
   int64_t n_dangling = 0;            // vertices of out-degree 0
   size_t block_bound = 0;            // GX_BOUND_BLOCK
+  int64_t stream_group = gx::kStreamGroup;  // GX_BOUND_STREAM_GROUP
+  uint32_t run_polls = 0;            // GX_BOUND_RUN_POLLS
   gx::UnitCaps caps{};               // tile and chunk sizes, heavy threshold (build_units)
   gx::hvec<int2> units;
   gx::hvec<int32_t> unit_shard;

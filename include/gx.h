@@ -166,8 +166,12 @@ gx_status gx_set_wait_limit(gx_engine* e, uint32_t polls);
 /* Bounds that only a graph near the device's size meets otherwise, lowered by
  * tests to reach what lies behind them at small ones; 0 sets the default. */
 typedef enum gx_bound {
-  GX_BOUND_BLOCK = 0  /* bytes of the largest block of device memory the engine's calls get: for a
+  GX_BOUND_BLOCK = 0, /* bytes of the largest block of device memory the engine's calls get: for a
                          larger one there is no room (default: what the device has) */
+  GX_BOUND_STREAM_GROUP = 1, /* edges that travel and are swept together when shards are streamed, from the
+                         next load on (default 8 M; resident shards: twice as many) */
+  GX_BOUND_RUN_POLLS = 2 /* polls of gx_run's grid barrier (PageRank) before GX_ERR_TIMEOUT (default: the
+                         larger of config.wait_limit and 1<<24) */
 } gx_bound;
 gx_status gx_set_bound(gx_engine* e, gx_bound which, int64_t value);
 
