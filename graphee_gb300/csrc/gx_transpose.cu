@@ -195,7 +195,7 @@ bool transpose_by_buckets(gx_engine* e, bool weighted, gx_status* status) {
   struct Block {
     unsigned char* p = nullptr;
     ~Block() { dev_free(&p); }
-  } block, sblock;
+  } block;
   size_t at = 0;
   auto place = [&](size_t bytes) {
     const size_t x = at;
@@ -206,6 +206,7 @@ bool transpose_by_buckets(gx_engine* e, bool weighted, gx_status* status) {
   const size_t o_src = place(2 * n), o_dst = place(4 * n), o_wt = place(weighted ? 4 * n : 0);
   const size_t o_bucket = place(8 * (static_cast<size_t>(nb) + 1)), o_source = place(8 * static_cast<size_t>(V)),
                o_ctr = place(8);
+  const size_t o_slices = place(sizeof(TrSlice) * (n / kTrSlice + static_cast<size_t>(nb)));
   if (dev_alloc(&block.p, at) != GX_OK) return false;  // no room: the caller's one-pass kernel
   auto run = [&]() -> gx_status {
     TrArgs a{};
@@ -257,9 +258,8 @@ bool transpose_by_buckets(gx_engine* e, bool weighted, gx_status* status) {
                                  static_cast<int32_t>(static_cast<uint32_t>(b) | (only ? 0x80000000u : 0u))});
     }
     if (slices.empty()) return GX_OK;
-    GX_TRY(dev_alloc(&sblock.p, slices.size() * sizeof(TrSlice)));
-    GX_CUDA(cudaMemcpyAsync(sblock.p, slices.data(), slices.size() * sizeof(TrSlice), cudaMemcpyHostToDevice, s));
-    a.slices = reinterpret_cast<const TrSlice*>(sblock.p);
+    GX_CUDA(cudaMemcpyAsync(block.p + o_slices, slices.data(), slices.size() * sizeof(TrSlice), cudaMemcpyHostToDevice, s));
+    a.slices = reinterpret_cast<const TrSlice*>(block.p + o_slices);
     tr_place_kernel<<<static_cast<unsigned>(slices.size()), kTrThreads, smem_p, s>>>(a);
     GX_CUDA(cudaGetLastError());
     // Every bucket has as many edges as its sources' out-degrees say, so a

@@ -120,3 +120,21 @@ def test_triangles_packed(V, relabel):
         with pytest.raises(gx.GxError) as ei:
             e.triangle_count()
         assert ei.value.status == gx.GX_ERR_OOM
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+def test_out_edges_without_room_for_buckets(weighted):
+    """Room for the out-edge CSR, not for the buckets' copy of its edges: built in one pass."""
+    src, dst = gx.rmat_edges(17, 6 << 20, 8)
+    off, col = gx.build_csc(1 << 17, src, dst)
+    g = gx.Graph(1 << 17, off, col, None, 16)
+    assert g.E >= 4 << 20
+    g.weights = gx.edge_weights(3, g)
+    a = (g.V, g.P, g.bounds, g.off, g.col, g.outdeg)
+    with gx.Engine(push_edge_fraction=1.0) as e:
+        e.load(g)
+        e.set_bound(gx.BOUND_BLOCK, 5 * g.E)
+        st = e.run(gx.APP_SSSP, 1000, source=1, weighted=weighted)
+        assert st["push_iterations"] == st["iterations"]
+        ref = O.run(O.SSSP, *a, 1000, weights=g.weights if weighted else None, source=1)[0]
+        assert np.array_equal(e.values(), ref)
