@@ -98,7 +98,7 @@ struct BatchArgs {
   unsigned int* ctr;
   unsigned int* team;       // per instance: arrivals, change counts [3]
   unsigned int* abort;      // set when a team barrier times out
-  unsigned int spin_limit;
+  unsigned int spin_limit;  // polls of a team barrier, each a load and a pause of some 64 ns
   float *pr0, *pr1;         // working values, indexed vbeg[i] + new local id
   float *con0, *con1;
   int32_t *lab0, *lab1;
@@ -851,7 +851,7 @@ gx_status batch_prepare(gx_engine* e, int32_t n, const int32_t* vbeg, bool check
   a.col = e->d_col;
   a.outdeg = e->d_outdeg;
   a.n_inst = n;
-  a.spin_limit = e->cfg.wait_limit;  // polls of at least 64 ns each
+  a.spin_limit = e->cfg.wait_limit;
   // Indexed by the graph's vertices, of which they hold these instances'.
   for (float** x : {&a.pr0, &a.pr1, &a.con0, &a.con1, &a.pr_out}) *x -= vbeg[0];
   for (int32_t** x : {&a.lab0, &a.lab1, &a.cc_out, &a.inv, &a.perm, &a.od}) *x -= vbeg[0];

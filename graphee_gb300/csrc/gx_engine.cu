@@ -1136,7 +1136,10 @@ gx_status run_app(gx_engine* e, const gx_run_params& prm, gx_run_stats* out) {
       // the dense supersteps in run_kernel, at every size (a superstep against
       // the replayed launches': 1000 vertices 7.8 for 14.6 us, 1 M 7 us less,
       // 7 M 3, 67 M 20).  SSSP and CC keep the launches: with pull, push and
-      // finalize in one such kernel they took 3 to 17 % longer.
+      // finalize in one such kernel they took 3 to 17 % longer.  So does PageRank
+      // once the engine holds the out-edge CSR (a run of SSSP or CC, or a
+      // selective step of PageRank itself built it): its steps then mark the
+      // shards of the next one, which this kernel does not.
       if (e->cfg.use_graph && !prof && !every && !e->cfg.exact_order && pa.hot_n == 0 && c.mark_mode == MARK_NONE &&
           run_scratch(e)) {
         RunArgs ra;

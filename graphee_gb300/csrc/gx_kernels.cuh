@@ -339,11 +339,10 @@ constexpr int kMinChunk = 256;     // shortest: one round of warp_reduce_range
 #define GX_LANE_MAX 16
 #endif
 constexpr int kLaneMaxDegree = GX_LANE_MAX;  // longest list a lane walks alone
-// Units a warp claims per atomic, when it has swept the last: a claim issued
-// ahead holds units that others could sweep (7 M vertices, a run of standard
-// PageRank: 7.98 ms with it, 7.67 without).  Claims of 1, 2, 3 and 4: 7 M
-// vertices 8.25, 7.70, 7.64 and 7.74 ms, 67 M (20 supersteps) 84.2, 80.0, 79.4
-// and 79.0, 1 M 1.61, 1.55, 1.55 and 1.60.
+// Units a warp claims per atomic, when it has swept the last: fewer wait for
+// the atomics, more, or a claim issued ahead, hold units that others could
+// sweep (standard PageRank, 7 M vertices: 8.25 ms a run with claims of one,
+// 7.64 of three, 7.98 issued ahead).
 constexpr int kGrab = 3;
 // PageRank loads a tile's offsets, old values and out-degrees a unit ahead
 // (17 M vertices, 20 supersteps: 19.50 -> 19.31 ms); the min apps, a register
@@ -351,10 +350,8 @@ constexpr int kGrab = 3;
 template <int APP> constexpr bool tile_prefetch() { return is_pr<APP>(); }
 // Work-unit cursors per launch, at most 32.  Neighbouring vertices share
 // sources, so the fewer places the graph is swept at, the more gathers meet in
-// L1 and L2, until the claims wait for each other: 64, 16, 8, 6 and 4 cursors,
-// 20 supersteps at 1 M vertices 1.81, 1.70, 1.62, 1.61 and 1.65 ms, 7 M
-// (standard) 7.94, 7.95, 7.73, 7.67 and 7.73, 17 M 20.1, 19.9, 19.5, 19.5 and
-// 19.6.  (A cursor per SM or CTA instead: +8 to 13 %, -1 to +2 %.)
+// L1 and L2, until the claims wait for each other (20 supersteps at 1 M
+// vertices: 1.81 ms with 64 cursors, 1.61 with 6, 1.65 with 4).
 constexpr int kQueues = 6;
 // A cursor to a 128-byte line: atomics on one line are served one after the
 // other.  (64 cursors in two lines, one unit to a claim: 16 M edges took 0.139
@@ -365,16 +362,11 @@ constexpr int kQueueStride = 32;
 // unit is a serial chain of loads, and a launch is never shorter than its
 // longest unit: the caps shrink until every warp has about three units, down
 // to one round of a warp's loads, and reach their full size (2048-edge tiles
-// at 30 M edges, chunks of 4096 at 60 M).  20 supersteps with 2, 3,
-// 4, 6 and 8 units a warp: 1 M vertices (16 M edges) 1.62, 1.57, 1.62, 1.77 and
-// 1.83 ms; 0.5 M 0.99, 0.99 and 1.09 with 2, 3 and 4; 2 M 2.62, 2.62 and 2.59.
-// Chunks of 2048, 4096 and 8192 at most: 7 M vertices (standard) 7.66, 7.58 and
-// 7.86 ms, 17 M relabelled 17.8, 17.3 and 17.7, 67 M relabelled 79.4, 77.8 and
-// 77.7, weighted SSSP at 17 M 5.59, 5.59 and 5.78: a chunk starts with loads
-// that nothing overlaps, and a launch ends with the last one.  Tiles of 1024
-// instead of 2048 edges: 8.03 (7 M), 20.4 (17 M), 87.0 (67 M).
-// With the full-size caps 1 M vertices took 2.8 ms and 1000 vertices 34
-// instead of 14 us a superstep.
+// at 30 M edges, chunks of 4096 at 60 M).  A chunk starts with loads that
+// nothing overlaps, and a launch ends with the last one, so neither small nor
+// large ones are best: 17 M vertices relabelled 17.8 ms with chunks of 2048,
+// 17.3 of 4096, 17.7 of 8192.  With the full-size caps 1 M vertices took 2.8
+// instead of 1.6 ms, and 1000 vertices 34 instead of 14 us a superstep.
 // A heavy_degree above the default is the caller's own and holds at every size;
 // the default, and less, shrinks with the chunks.
 constexpr int32_t kHeavyDegree = 4096;
@@ -1261,7 +1253,7 @@ struct RunArgs {
   PullArgs pull;
   StepStats* stats;
   RunScratch* run;
-  unsigned int wait_limit;  // polls (of at least 32 ns) of a barrier
+  unsigned int wait_limit;  // polls of a barrier, each a load and a pause of some 32 ns
 };
 
 template <int APP>

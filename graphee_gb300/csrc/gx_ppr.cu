@@ -52,7 +52,7 @@ struct PprArgs {
   unsigned int* ctr;        // kQueues work cursors per step
   unsigned int* arrive;     // grid-barrier arrival count per step
   unsigned int* abort;      // set when a grid barrier gives up
-  unsigned int wait_limit;  // polls (of at least 64 ns) before it does
+  unsigned int wait_limit;  // polls before it does, each a load and a pause of some 64 ns
   float* partial;           // [n_chunks][W]
   unsigned int* ticket;     // per chunked vertex, indexed by partial base
   const int32_t* src;       // [W] source vertex of each column (-1 past k)

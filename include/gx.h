@@ -76,10 +76,11 @@ typedef struct gx_config {
                                   vertices above heavy_degree (default 0) */
   int32_t push_sparse;         /* SSSP/CC: push over out-edges when selective (default 1) */
   int32_t use_graph;           /* replay the iteration loop as a CUDA graph (default 1) */
-  uint32_t wait_limit;         /* polls (each of at least 64 ns) a device-side wait makes before it gives
-                                  up and the call returns GX_ERR_TIMEOUT; bounds the CTA-team barrier
-                                  of gx_batch_run and the grid barrier of gx_ppr (default 1<<24, over
-                                  a second); gx_run's grid barrier (PageRank) makes at least 1<<24 */
+  uint32_t wait_limit;         /* polls (each a load and a pause of some 64 ns) a device-side wait makes
+                                  before it gives up and the call returns GX_ERR_TIMEOUT; bounds the
+                                  CTA-team barrier of gx_batch_run and the grid barrier of gx_ppr
+                                  (default 1<<24, seconds); gx_run's grid barrier (PageRank) makes at
+                                  least 1<<24 (GX_BOUND_RUN_POLLS) */
   int32_t verbose;             /* per-iteration log lines on stderr (default 0) */
   int32_t profile;             /* time every pull launch with CUDA events (default 0) */
   int32_t compress_cache;      /* with a budget the plain shards exceed: keep every shard compressed
@@ -201,7 +202,10 @@ gx_status gx_set_weights(gx_engine* e, const uint32_t* w);
  * the init_vertex() override (GraphPS.h:60). Used when params.use_init. */
 gx_status gx_set_init(gx_engine* e, const void* host_vals);
 
-/* Superstep loop of GraphPS<T>::run (GraphPS.h:256-386). */
+/* Superstep loop of GraphPS<T>::run (GraphPS.h:256-386).  PageRank's dense
+ * supersteps are one launch for up to 64 of them while the engine has no
+ * out-edge CSR; once a run of SSSP or CC, or a selective step, has built it,
+ * they are launched one by one (same results), until the next load. */
 gx_status gx_run(gx_engine* e, const gx_run_params* params, gx_run_stats* stats);
 
 /* Copies the final _VertexMsg (T[V]) to host memory. */
@@ -241,7 +245,10 @@ gx_status gx_get_iter_stats(gx_engine* e, int32_t step, gx_iter_stats* out);
 
 /* Triangles of the loaded graph taken as undirected (load the CSC of a
  * symmetrised, deduplicated edge list).  Orients u->v iff (deg u, u) <
- * (deg v, v) and intersects sorted out-lists.  No reference counterpart:
+ * (deg v, v) and looks the shorter out-list of every edge's ends up in the
+ * longer one's bitmap or hash table.  Holds up to 4 bytes an entry and 65 a
+ * vertex beside the graph; without room for that, 2 to 3 an entry and 55 a
+ * vertex, in parts.  No reference counterpart:
  * GraphH/list/system/GraphPS.h:15-95 ("tc") counts reciprocal edges, not
  * triangles.  *total receives the exact count. */
 gx_status gx_triangle_count(gx_engine* e, uint64_t* total, gx_run_stats* stats);
