@@ -835,19 +835,17 @@ gx_status build_out_edges(gx_engine* e, bool weighted) {
   if (!transpose_by_buckets(e, weighted, &st)) {
     // Few edges, too many for its tables, or no room for its copy.
     GX_TRY(dev_alloc(&cursor.p, static_cast<size_t>(V) + 1));
-    unsigned int* bad = reinterpret_cast<unsigned int*>(cursor.p + V);
     GX_CUDA(cudaMemcpyAsync(cursor.p, e->d_ooff, sizeof(int64_t) * V, cudaMemcpyDeviceToDevice, e->s_comp));
-    GX_CUDA(cudaMemsetAsync(bad, 0, sizeof(*bad), e->s_comp));
+    e->h_ctl->error = 0;  // in pinned memory: the check's word, with no copy of its own
     transpose_kernel<<<e->n_sm * 8, 256, 0, e->s_comp>>>(e->d_off, e->d_col, weighted ? e->d_w : nullptr, V, cursor.p,
                                                           e->d_ocol, weighted ? e->d_ow : nullptr,
                                                           static_cast<unsigned long long>(e->E));
-    transpose_check_kernel<<<e->n_sm * 4, 256, 0, e->s_comp>>>(cursor.p, e->d_ooff, V, bad);
-    GX_CUDA(cudaGetLastError());
-    unsigned int h_bad = 0;
-    cudaError_t err = cudaMemcpyAsync(&h_bad, bad, sizeof(h_bad), cudaMemcpyDeviceToHost, e->s_comp);
+    transpose_check_kernel<<<std::max(1, std::min(e->n_sm * 4, (V + 255) / 256)), 256, 0, e->s_comp>>>(
+        cursor.p, e->d_ooff, V, &e->h_ctl->error);
+    cudaError_t err = cudaGetLastError();
     if (err == cudaSuccess) err = cudaStreamSynchronize(e->s_comp);
     if (err != cudaSuccess) return fail(GX_ERR_CUDA, "transpose: %s", cudaGetErrorString(err));
-    if (h_bad) return out_degrees_wrong();
+    if (*static_cast<volatile int*>(&e->h_ctl->error)) return out_degrees_wrong();
   }
   if (st != GX_OK) return st;
   e->out_built = true;

@@ -1572,7 +1572,7 @@ static __global__ void transpose_kernel(const int64_t* off, const int32_t* col, 
 
 // Whether every source's last place is where the next one's places begin.
 static __global__ void transpose_check_kernel(const unsigned long long* cursor, const int64_t* ooff, int n,
-                                              unsigned int* bad) {
+                                              int* bad) {
   for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
     if (cursor[v] != static_cast<unsigned long long>(ooff[v + 1])) *bad = 1;
 }
