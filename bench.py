@@ -512,7 +512,10 @@ def run_gx(args, rank, local_rank, world):
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                              "frac": achieved / peak, "traffic": traffic, "peak_source": peak_kind,
                              "kernel": "pull_kernel<PAGERANK_REF>", "kernel_ms": pull_ms,
-                             "algorithmic_bytes_per_launch": alg_bytes},
+                             "algorithmic_bytes_per_launch": alg_bytes,
+                             # What the timed region launches: the same sweep, run_kernel's, many supersteps to a launch.
+                             "timed_kernel": "run_kernel<PAGERANK_REF>", "timed_ms_per_superstep": ms_step / args.iters,
+                             "timed_frac": alg_bytes / (ms_step / args.iters / 1000) / 1e9 / peak},
                 "cpu_baseline": cpu, "clocks": clocks, "wall_s_timed": wall, "sssp": sssp,
                 "rmat24": rmat24, "layout": args.layout, other_name: other,
                 "iterations_per_step": iters_done / args.steps}
