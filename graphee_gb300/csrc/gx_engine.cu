@@ -804,10 +804,12 @@ gx_status build_out_edges(gx_engine* e, bool weighted) {
   e->out_built = false;  // its arrays are replaced: a failure below leaves none
   int64_t total = 0;
   int negative = 0;
-#pragma omp parallel for reduction(+ : total) reduction(| : negative)
+  int32_t most = 0;
+#pragma omp parallel for reduction(+ : total) reduction(| : negative) reduction(max : most)
   for (int32_t v = 0; v < V; ++v) {
     total += e->outdeg[v];
     negative |= e->outdeg[v] < 0;
+    most = std::max(most, e->outdeg[v]);
   }
   if (negative) return fail(GX_ERR_FORMAT, "vertexout.npy holds a negative out-degree");
   if (total != e->E)
@@ -832,8 +834,8 @@ gx_status build_out_edges(gx_engine* e, bool weighted) {
                   part.p, e->s_comp));
   store_i64_kernel<<<1, 1, 0, e->s_comp>>>(e->d_ooff + V, e->E);
   gx_status st = GX_OK;
-  if (!transpose_by_buckets(e, weighted, &st)) {
-    // Few edges, too many for its tables, or no room for its copy.
+  if (!transpose_by_buckets(e, weighted, most, &st)) {
+    // Few or evenly spread edges, too many for its tables, or no room for its copy.
     GX_TRY(dev_alloc(&cursor.p, static_cast<size_t>(V) + 1));
     GX_CUDA(cudaMemcpyAsync(cursor.p, e->d_ooff, sizeof(int64_t) * V, cudaMemcpyDeviceToDevice, e->s_comp));
     e->h_ctl->error = 0;  // in pinned memory: the check's word, with no copy of its own

@@ -443,8 +443,8 @@ inline gx_status out_degrees_wrong() {
 
 // Fills e->d_ocol (and d_ow) from the CSC by way of buckets of sources
 // (gx_transpose.cu), with e->d_ooff in place; the work is done on return.
-// False, with nothing written, where its tables do not reach or its scratch
-// has no room.
-bool transpose_by_buckets(gx_engine* e, bool weighted, gx_status* status);
+// `most`: the largest out-degree.  False, with nothing written, where its
+// tables do not reach, its scratch has no room or one pass takes less.
+bool transpose_by_buckets(gx_engine* e, bool weighted, int32_t most, gx_status* status);
 
 }  // namespace gx

@@ -34,9 +34,15 @@ constexpr int kBucket = 1 << kBucketBits;
 constexpr int kMostBuckets = 8192;                // V up to 2^27: 96 KB of a CTA's counters and places
 constexpr int kTrThreads = 512;
 constexpr int64_t kTrSlice = 128 * 1024;          // edges of a slice
-// Below this one pass of transpose_kernel takes less than the two passes'
-// allocations and wait (281 K edges: a first run of 0.60 ms, 1.07 this way).
+// One pass of transpose_kernel takes less than the two passes' allocations and
+// wait (some 0.25 ms) where there are few edges (281 K: a first run of 0.60 ms,
+// 1.07 this way), and also with more as long as L2 holds what it scatters and no
+// source draws thousands of its atomics, some 16 ns each (uniform, 12 M edges:
+// 0.27 ms, 0.54 this way; 18 M of 2 M vertices 1.56 and 0.88; 11 M with a source
+// of 100 K out-edges 1.90 and 0.55).
 constexpr int64_t kTrLeast = int64_t(4) << 20;
+constexpr int64_t kTrBytes = int64_t(64) << 20;  // of destinations, weights and places
+constexpr int32_t kTrDegree = 16384;             // of a source
 
 struct TrSlice {
   int64_t begin;   // in the bucketed arrays
@@ -185,11 +191,12 @@ __global__ void tr_bucket_starts_kernel(const int64_t* ooff, int32_t V, int32_t 
 
 namespace gx {
 
-bool transpose_by_buckets(gx_engine* e, bool weighted, gx_status* status) {
+bool transpose_by_buckets(gx_engine* e, bool weighted, int32_t most, gx_status* status) {
   const int32_t V = e->V;
   const int64_t E = e->E;
   const int64_t nb64 = (static_cast<int64_t>(V) + kBucket - 1) / kBucket;
   if (nb64 > kMostBuckets || E > static_cast<int64_t>(UINT32_MAX) || E < kTrLeast) return false;
+  if ((weighted ? 8 : 4) * E + 8 * static_cast<int64_t>(V) < kTrBytes && most < kTrDegree) return false;
   const int32_t nb = static_cast<int32_t>(nb64);
   cudaStream_t s = e->s_comp;
   struct Block {

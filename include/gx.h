@@ -246,9 +246,9 @@ gx_status gx_get_iter_stats(gx_engine* e, int32_t step, gx_iter_stats* out);
 /* Triangles of the loaded graph taken as undirected (load the CSC of a
  * symmetrised, deduplicated edge list).  Orients u->v iff (deg u, u) <
  * (deg v, v) and looks the shorter out-list of every edge's ends up in the
- * longer one's bitmap or hash table.  Holds up to 4 bytes an entry and 65 a
- * vertex beside the graph; without room for that, 2 to 3 an entry and 55 a
- * vertex, in parts.  No reference counterpart:
+ * longer one's bitmap or hash table.  Holds 4 bytes an entry and 48 to 70 a
+ * vertex beside the graph; without room for that, 2 an entry and 45 to 55 a
+ * vertex, in several blocks.  No reference counterpart:
  * GraphH/list/system/GraphPS.h:15-95 ("tc") counts reciprocal edges, not
  * triangles.  *total receives the exact count. */
 gx_status gx_triangle_count(gx_engine* e, uint64_t* total, gx_run_stats* stats);
